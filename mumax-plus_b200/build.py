@@ -1,27 +1,29 @@
 """Build libmpx.so (the sm_100a engine behind include/mpx.h) in-tree with nvcc.
 
-The library is one translation unit (csrc/engine.cu includes the kernel
-headers) compiled for sm_100a only.  The resulting shared object sits next to
-this file so that it travels with the source tree.  A second build of the same
-sources with -DMPX_BOUNDS_CHECK, libmpx_checked.so, verifies the index of every
-per-cell field access (mpx_bounds_check reads the record); the two compile in
-parallel.
+The kernel families compile in one file each (csrc/*.cu, see csrc/launch.h), in
+parallel, into _build/ and link into one library next to this file, so that it
+travels with the source tree; a file is compiled again when one of the headers
+it includes has changed.  A second build of the same sources in one translation
+unit (csrc/checked.cu) with -DMPX_BOUNDS_CHECK, libmpx_checked.so, verifies the
+index of every per-cell field access (mpx_bounds_check reads the record).
 """
+import concurrent.futures
 import os
 import subprocess
 import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
-SRC = os.path.join(HERE, "csrc", "engine.cu")
-HEADERS = sorted(os.path.join(HERE, "csrc", f) for f in os.listdir(os.path.join(HERE, "csrc")) if f.endswith(".cuh"))
+CSRC = os.path.join(HERE, "csrc")
+OBJ = os.path.join(HERE, "_build")
+UNITS = ["engine", "xpass", "yz", "yzwarp", "yzlong", "thick", "pairs"]
 OUT = os.path.join(HERE, "libmpx.so")
 OUT_CHECKED = os.path.join(HERE, "libmpx_checked.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC",
     "--expt-relaxed-constexpr",
 ]
 
@@ -33,42 +35,76 @@ def nvcc_path():
     return "nvcc"
 
 
+def _obj(unit):
+    return os.path.join(OBJ, unit + ".o")
+
+
+def _deps(unit):
+    """Files the unit was compiled from (the compiler's dependency file), or None."""
+    try:
+        with open(os.path.join(OBJ, unit + ".d")) as f:
+            words = f.read().replace("\\\n", " ").split()
+    except OSError:
+        return None
+    return [w for w in words[1:] if w.startswith(ROOT)]
+
+
+def _stale(unit):
+    deps = _deps(unit)
+    if deps is None or not os.path.exists(_obj(unit)):
+        return True
+    t = os.path.getmtime(_obj(unit))
+    return any(not os.path.exists(d) or os.path.getmtime(d) > t for d in deps + [os.path.abspath(__file__)])
+
+
 def up_to_date(out=OUT):
-    if not os.path.exists(out):
+    units = ["checked"] if out == OUT_CHECKED else UNITS
+    if not os.path.exists(out) or any(_stale(u) for u in units):
         return False
-    t = os.path.getmtime(out)
-    deps = [SRC, os.path.join(ROOT, "include", "mpx.h"), __file__] + HEADERS
-    return all(os.path.getmtime(d) <= t for d in deps if os.path.exists(d))
+    return all(os.path.getmtime(_obj(u)) <= os.path.getmtime(out) for u in units)
 
 
-def _command(out, extra):
-    defs = ["-DMPX_BOUNDS_CHECK"] if out == OUT_CHECKED else []
-    return [nvcc_path()] + NVCC_FLAGS + defs + list(extra) + ["-I", os.path.join(ROOT, "include"), SRC, "-o", out]
+def _run(cmd, verbose):
+    if verbose:
+        print(" ".join(cmd), file=sys.stderr)
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("nvcc failed:\n" + r.stdout)
+    if verbose and r.stdout:
+        print(r.stdout, file=sys.stderr)
+
+
+def _command(out, extra=(), unit="engine"):
+    """The nvcc command of `unit` into `out`; the checked library's adds the check."""
+    defs = ["-DMPX_BOUNDS_CHECK"] if out in (OUT_CHECKED, _obj("checked")) else []
+    return ([nvcc_path()] + NVCC_FLAGS + defs + list(extra) + ["-I", os.path.join(ROOT, "include")]
+            + [os.path.join(CSRC, unit + ".cu"), "-o", out])
+
+
+def _compile(unit, extra, verbose):
+    extra = list(extra) + ["-c", "-MMD", "-MF", os.path.join(OBJ, unit + ".d")]
+    if unit == "checked":  # one large file: its kernels are optimised in parallel
+        extra.append("--split-compile=0")
+    _run(_command(_obj(unit), extra, unit), verbose)
 
 
 def build(force=False, verbose=False, extra=(), checked=True):
     """Compile libmpx.so (and libmpx_checked.so when `checked`) for sm_100a;
     returns the path of libmpx.so."""
+    os.makedirs(OBJ, exist_ok=True)
     outs = [o for o in ([OUT, OUT_CHECKED] if checked else [OUT]) if force or not up_to_date(o)]
-    procs = []
+    units = [u for o in outs for u in (["checked"] if o == OUT_CHECKED else UNITS) if force or _stale(u)]
+    units.sort(key=lambda u: u != "checked")  # the longest first
+    with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, os.cpu_count() or 1)) as pool:
+        for f in [pool.submit(_compile, u, extra, verbose) for u in units]:
+            f.result()
     for out in outs:
-        cmd = _command(out, extra)
-        if verbose:
-            print(" ".join(cmd), file=sys.stderr)
-        procs.append(subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.PIPE, text=True))
-    errors = []
-    for proc in procs:
-        so, se = proc.communicate()
-        if proc.returncode != 0:
-            errors.append(so + se)
-        elif verbose and (so or se):
-            print(so + se, file=sys.stderr)
-    if errors:
-        raise RuntimeError("nvcc failed:\n" + "\n".join(errors))
+        objs = [_obj(u) for u in (["checked"] if out == OUT_CHECKED else UNITS)]
+        _run([nvcc_path(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", out] + objs, verbose)
     return OUT
 
 
 if __name__ == "__main__":
     force = "--force" in sys.argv
     extra = ["-Xptxas", "-v"] if "--ptxas" in sys.argv else []
-    print(build(force=force or bool(extra), verbose=True, extra=extra))
+    print(build(force=force or bool(extra), verbose=True, extra=extra, checked="--unchecked" not in sys.argv))

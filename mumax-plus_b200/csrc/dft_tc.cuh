@@ -36,7 +36,7 @@
 
 namespace mpx {
 
-__device__ unsigned int g_tc_timeouts = 0;  // mbarrier waits that gave up (read by mpx_tc_status)
+static __device__ unsigned int g_tc_timeouts = 0;  // mbarrier waits that gave up (read by mpx_tc_status)
 
 namespace tc {
 
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(128, TC_BLOCKS_PER_SM)
 // on the barrier, so its bounded wait (`polls` polls) runs out.  The block then
 // counts the timeout, waits once more (bounded), releases its tensor memory and
 // returns; the context stays usable.
-__global__ void __launch_bounds__(128, 1) k_tc_timeout_probe(int polls) {
+static __global__ void __launch_bounds__(128, 1) k_tc_timeout_probe(int polls) {
   __shared__ __align__(8) unsigned long long mbar;
   __shared__ uint32_t tbase;
   const int tid = threadIdx.x, warp = tid >> 5;

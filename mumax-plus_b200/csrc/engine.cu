@@ -22,10 +22,10 @@
 
 #include "../../include/mpx.h"
 #include "kernels.cuh"
+#include "launch.h"
+#include "reduce.cuh"
 #include "newell.cuh"
 #include "stray.cuh"
-#include "pairfft.cuh"
-#include "yzsplit.cuh"
 #include "dft_tc.cuh"
 
 using namespace mpx;
@@ -73,7 +73,6 @@ constexpr int MAX_FFT = 4096;
 constexpr int SMEM_MAX = 227 * 1024;
 // dynamic shared memory left next to the static descriptor copies of a block
 constexpr int SMEM_DYN_MAX = SMEM_MAX - 2048;
-constexpr int YZ_CLASSES = 24;  // k_yz / k_yzw / k_yzw32 / k_yzw64 launch classes (yz_class)
 
 // ------------------------------------------------------------ tableaus
 // core/butchertableau.cpp: Heun, Bogacki-Shampine, Cash-Karp, Fehlberg, Dormand-Prince
@@ -532,6 +531,11 @@ int yz_class(const Magnet* m) {
   return ilog2(m->P[2]) + (m->P[1] > 2048 ? 5 : 0);
 }
 constexpr int YZ_THREADS = 384;
+// threads per block of a y/z launch class
+int yz_threads(int cls) {
+  if (cls >= 20) return YZP_THREADS;
+  return cls >= 10 ? yzw_threads_of(1 << ((cls - 10) % 5)) : YZ_THREADS;
+}
 
 // Tile shapes.  Row tiles: about 4096 points of the padded x transform per
 // tile (4 rows above Px = 1024; up to TY_MAX rows of short transforms), 8 rows
@@ -574,21 +578,21 @@ mpx_status launch_split(mpx_engine* e, const Work* ycw, int nyc, const Work* zmw
   }
   if (nyc > 0) {
     if (ry)
-      k_ycols<-1, 3><<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
+      ycols_fn(-1, 3)<<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
     else
-      k_ycols<-1, 4><<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
+      ycols_fn(-1, 4)<<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
     e->launches++;
   }
   if (rz)
-    k_zmul<3><<<nzm, YZ_THREADS, smem_z, e->stream>>>(e->d_mags, e->d_groups, zmw, stage, gate, e->d_tw);
+    zmul_fn(3)<<<nzm, YZ_THREADS, smem_z, e->stream>>>(e->d_mags, e->d_groups, zmw, stage, gate, e->d_tw);
   else
-    k_zmul<4><<<nzm, YZ_THREADS, smem_z, e->stream>>>(e->d_mags, e->d_groups, zmw, stage, gate, e->d_tw);
+    zmul_fn(4)<<<nzm, YZ_THREADS, smem_z, e->stream>>>(e->d_mags, e->d_groups, zmw, stage, gate, e->d_tw);
   e->launches++;
   if (nyc > 0) {
     if (ry)
-      k_ycols<1, 3><<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
+      ycols_fn(1, 3)<<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
     else
-      k_ycols<1, 4><<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
+      ycols_fn(1, 4)<<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
     e->launches++;
   }
   if (ntc > 0) {
@@ -621,58 +625,14 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, int smem, 
 // radix-16 form otherwise (k_yz)
 mpx_status launch_yz(mpx_engine* e, int cls, const Work* work, int n, int smem, int stage, int gate) {
   if (n <= 0) return MPX_OK;
-#define MPX_YZ(PZ, LR) \
-  CUDA_TRY(launch_pdl(k_yz<PZ, LR>, n, YZ_THREADS, smem, e->stream, e->d_mags, e->d_groups, work, stage, gate, e->d_tw))
-#define MPX_YZW(PZ) \
-  CUDA_TRY(launch_pdl(k_yzw<PZ>, n, yzw_threads<PZ>(), smem, e->stream, e->d_mags, e->d_groups, work, stage, gate, \
-                      e->d_tw))
-#define MPX_YZW32(PZ) \
-  CUDA_TRY(launch_pdl(k_yzw32<PZ>, n, yzw_threads<PZ>(), smem, e->stream, e->d_mags, e->d_groups, work, stage, gate, \
-                      e->d_tw))
-#define MPX_YZW64(PZ) \
-  CUDA_TRY(launch_pdl(k_yzw64<PZ>, n, YZP_THREADS, smem, e->stream, e->d_mags, e->d_groups, work, stage, gate, e->d_tw))
-  switch (cls) {
-    case 0: MPX_YZ(1, 3); break;
-    case 1: MPX_YZ(2, 3); break;
-    case 2: MPX_YZ(4, 3); break;
-    case 3: MPX_YZ(8, 3); break;
-    case 5: MPX_YZ(1, 4); break;
-    case 6: MPX_YZ(2, 4); break;
-    case 7: MPX_YZ(4, 4); break;
-    case 8: MPX_YZ(8, 4); break;
-    case 10: MPX_YZW(1); break;
-    case 11: MPX_YZW(2); break;
-    case 12: MPX_YZW(4); break;
-    case 13: MPX_YZW(8); break;
-    case 14: MPX_YZW(16); break;
-    case 15: MPX_YZW32(1); break;
-    case 16: MPX_YZW32(2); break;
-    case 17: MPX_YZW32(4); break;
-    case 18: MPX_YZW32(8); break;
-    case 19: MPX_YZW32(16); break;
-    case 20: MPX_YZW64(1); break;
-    case 21: MPX_YZW64(2); break;
-    case 22: MPX_YZW64(4); break;
-    case 23: MPX_YZW64(8); break;
-    default: MPX_YZ(16, 4); break;  // 4 and 9 (z length 16)
-  }
-#undef MPX_YZ
-#undef MPX_YZW
-#undef MPX_YZW32
-#undef MPX_YZW64
+  const YzFn fn = cls >= 15 ? yz_long_fn(cls) : cls >= 10 ? yz_warp_fn(cls) : yz_block_fn(cls);
+  CUDA_TRY(launch_pdl(fn, n, yz_threads(cls), smem, e->stream, e->d_mags, e->d_groups, work, stage, gate, e->d_tw));
   e->launches++;
   return MPX_OK;
 }
 // The x-pass kernels of a launch: the PAIR forms (2048-point warp-pair rows
 // compiled in) when one of its magnets has 2048-point x rows, else the forms
 // without them (the shorter lengths keep their registers and code).
-using XfwdFn = void (*)(const MagnetDev*, const GroupDev*, const Work*, int, int, const float*, const float2*);
-using XinvFn = void (*)(const MagnetDev*, GroupDev*, const Work*, EpiArgs, const float2*);
-XfwdFn xfwd_fn(bool combine, bool pair) {
-  if (combine) return pair ? k_xfwd<true, true> : k_xfwd<true, false>;
-  return pair ? k_xfwd<false, true> : k_xfwd<false, false>;
-}
-XinvFn xinv_fn(bool pair) { return pair ? k_xinv<true> : k_xinv<false>; }
 bool x_pair_of(const Magnet* m) { return m->P[0] == 2048; }
 
 int x_threads(const Magnet* m) {
@@ -1026,11 +986,11 @@ mpx_status build_pair_fft(mpx_engine* e, const Magnet* A, const int nB[3], const
   for (int a = 0; a < 3; ++a) kp.pf.nin[a] = kp.pf.nout[a] = K[a];
   kp.pf.win[0] = kp.pf.win[1] = kp.pf.win[2] = 0;
   pair_shapes(kp, 6);
-  k_pair_xfwd<true><<<kp.g_xf, PF_THREADS, kp.s_xf, e->stream>>>(e->d_mags, e->d_groups, -1, 0, 0, tab, kp.pf, 6,
+  pair_xfwd_fn(true)<<<kp.g_xf, PF_THREADS, kp.s_xf, e->stream>>>(e->d_mags, e->d_groups, -1, 0, 0, tab, kp.pf, 6,
                                                                   kp.ry_f, e->d_tw);
-  k_pair_yfft<-1><<<kp.g_yf, PF_THREADS, kp.s_yf, e->stream>>>(e->d_mags, e->d_groups, -1, 0, 0, kp.pf, 6, kp.zc_f,
+  pair_yfft_fn(-1)<<<kp.g_yf, PF_THREADS, kp.s_yf, e->stream>>>(e->d_mags, e->d_groups, -1, 0, 0, kp.pf, 6, kp.zc_f,
                                                                 e->d_tw);
-  k_pair_zmul<false><<<kp.g_z, PF_THREADS, kp.s_z, e->stream>>>(e->d_mags, e->d_groups, -1, 0, 0, kp.pf, 6, kp.tky,
+  pair_zmul_fn(false)<<<kp.g_z, PF_THREADS, kp.s_z, e->stream>>>(e->d_mags, e->d_groups, -1, 0, 0, kp.pf, 6, kp.tky,
                                                                  e->d_tw);
   e->launches += 3;
   pfree(e, tab);
@@ -1094,25 +1054,21 @@ mpx_status cached_pair_plan(mpx_engine* e, const Magnet* A, const Magnet* B, con
 // into out (3 x N of `dst`, added with `add`); `gate` as the stage kernels.
 void launch_pair_fft(mpx_engine* e, const PairPlan& pl, int src, int dst, int stage, int gate, int add, float* out) {
   const PairFft& pf = pl.pf;
-  k_pair_xfwd<false><<<pl.g_xf, PF_THREADS, pl.s_xf, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, nullptr,
+  pair_xfwd_fn(false)<<<pl.g_xf, PF_THREADS, pl.s_xf, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, nullptr,
                                                                    pf, 3, pl.ry_f, e->d_tw);
   if (pl.s_yz > 0) {
     const int Hx = (1 << pf.logP[0]) / 2 + 1;
-    switch (pf.logP[2]) {
-      case 0: k_pair_yz<1><<<Hx, PF_THREADS, pl.s_yz, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, e->d_tw); break;
-      case 1: k_pair_yz<2><<<Hx, PF_THREADS, pl.s_yz, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, e->d_tw); break;
-      case 2: k_pair_yz<4><<<Hx, PF_THREADS, pl.s_yz, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, e->d_tw); break;
-      default: k_pair_yz<8><<<Hx, PF_THREADS, pl.s_yz, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, e->d_tw); break;
-    }
+    pair_yz_fn(pf.logP[2])<<<Hx, PF_THREADS, pl.s_yz, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf,
+                                                                   e->d_tw);
   } else {
-    k_pair_yfft<-1><<<pl.g_yf, PF_THREADS, pl.s_yf, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, 3,
+    pair_yfft_fn(-1)<<<pl.g_yf, PF_THREADS, pl.s_yf, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, 3,
                                                                   pl.zc_f, e->d_tw);
-    k_pair_zmul<true><<<pl.g_z, PF_THREADS, pl.s_z, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, 3,
+    pair_zmul_fn(true)<<<pl.g_z, PF_THREADS, pl.s_z, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, 3,
                                                                   pl.tky, e->d_tw);
-    k_pair_yfft<1><<<pl.g_yi, PF_THREADS, pl.s_yi, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, 3,
+    pair_yfft_fn(1)<<<pl.g_yi, PF_THREADS, pl.s_yi, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, 3,
                                                                  pl.zc_i, e->d_tw);
   }
-  k_pair_xinv<<<pl.g_xi, PF_THREADS, pl.s_xi, e->stream>>>(e->d_mags, e->d_groups, dst, stage, gate, pf, pl.ry_i, add,
+  pair_xinv_fn()<<<pl.g_xi, PF_THREADS, pl.s_xi, e->stream>>>(e->d_mags, e->d_groups, dst, stage, gate, pf, pl.ry_i, add,
                                                            out, e->d_tw);
   e->launches += pl.launches();
 }
@@ -1616,7 +1572,7 @@ mpx_status setup_magnet(mpx_engine* e, Magnet* m, const mpx_magnet_desc* d, bool
 // every run so that engines with different methods never see a stale one.
 mpx_status upload_tableau(mpx_engine* e, int method) {
   TableauDev t = make_tableau(method);
-  CUDA_TRY(cudaMemcpyToSymbolAsync(c_tab, &t, sizeof(t), 0, cudaMemcpyHostToDevice, e->stream));
+  CUDA_TRY(upload_tableau_symbol(t, e->stream));
   e->tab_method = method;
   return MPX_OK;
 }
@@ -1669,7 +1625,7 @@ mpx_status eval_into(mpx_engine* e, Magnet* m, int q, float* out) {
                         e->d_tw));
     e->launches += 2;
   } else {
-    k_local<<<ntile, 256, 0, e->stream>>>(e->d_mags, e->d_groups, m->d_tiles, ea);
+    local_fn()<<<ntile, 256, 0, e->stream>>>(e->d_mags, e->d_groups, m->d_tiles, ea);
     e->launches += 1;
   }
   return check_launch(e, "eval");
@@ -1703,7 +1659,7 @@ mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
       e->launches++;
     }
     if (e->n_t_local > 0 && s > 0) {
-      k_combine<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, s, 0);
+      combine_fn()<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, s, 0);
       e->launches++;
     }
     // stray fields of the stage states of the other magnets
@@ -1718,22 +1674,22 @@ mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
       e->launches++;
     }
     if (e->n_t_local > 0) {
-      k_local<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, ea);
+      local_fn()<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, ea);
       e->launches++;
     }
   }
   if (!T.fsal) {
     if (e->n_t_demag > 0) {
-      k_combine<<<e->n_t_demag, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_demag, S, 1);
+      combine_fn()<<<e->n_t_demag, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_demag, S, 1);
       e->launches++;
     }
     if (e->n_t_local > 0) {
-      k_combine<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, S, 1);
+      combine_fn()<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, S, 1);
       e->launches++;
     }
   }
   const int ng = (int)e->groups.size();
-  k_controller<<<(ng + 127) / 128, 128, 0, e->stream>>>(e->d_groups, ng);
+  controller_fn()<<<(ng + 127) / 128, 128, 0, e->stream>>>(e->d_groups, ng);
   e->launches++;
   // sampled run: <m> of the group's magnets into the rows the controller marked due
   if (e->sampling_group >= 0) {
@@ -1968,24 +1924,24 @@ mpx_status mpx_engine_create(int device, mpx_engine** out) {
   CUDA_TRY(cudaMalloc(&e->d_red, sizeof(double) * 3 * 1024));
   CUDA_TRY(cudaMalloc(&e->d_redout, sizeof(double) * 4));  // 3 reduction results, or the 4 of k_min_final
   // large dynamic shared memory and the max-shared carveout for the FFT kernels
-  const void* fft_kernels[] = {(const void*)k_xfwd<false, false>, (const void*)k_xfwd<true, false>,
-                               (const void*)k_xinv<false>, (const void*)k_xfwd<false, true>,
-                               (const void*)k_xfwd<true, true>, (const void*)k_xinv<true>,
-                               (const void*)k_yz<1, 4>, (const void*)k_yz<2, 4>, (const void*)k_yz<4, 4>,
-                               (const void*)k_yz<8, 4>, (const void*)k_yz<16, 4>, (const void*)k_yz<1, 3>,
-                               (const void*)k_yz<2, 3>, (const void*)k_yz<4, 3>, (const void*)k_yz<8, 3>,
-                               (const void*)k_ycols<-1, 3>, (const void*)k_ycols<-1, 4>, (const void*)k_ycols<1, 3>,
-                               (const void*)k_ycols<1, 4>, (const void*)k_zmul<3>, (const void*)k_zmul<4>,
-                               (const void*)k_yzw<1>, (const void*)k_yzw<2>, (const void*)k_yzw<4>,
-                               (const void*)k_yzw<8>, (const void*)k_yzw<16>, (const void*)k_yzw32<1>,
-                               (const void*)k_yzw32<2>, (const void*)k_yzw32<4>, (const void*)k_yzw32<8>,
-                               (const void*)k_yzw32<16>, (const void*)k_yzw64<1>, (const void*)k_yzw64<2>,
-                               (const void*)k_yzw64<4>, (const void*)k_yzw64<8>, (const void*)k_pair_xfwd<true>,
-                               (const void*)k_pair_xfwd<false>, (const void*)k_pair_yfft<-1>,
-                               (const void*)k_pair_yfft<1>, (const void*)k_pair_zmul<true>,
-                               (const void*)k_pair_zmul<false>, (const void*)k_pair_xinv,
-                               (const void*)k_pair_yz<1>, (const void*)k_pair_yz<2>, (const void*)k_pair_yz<4>,
-                               (const void*)k_pair_yz<8>};
+  std::vector<const void*> fft_kernels;
+  for (int pair = 0; pair < 2; ++pair) {
+    fft_kernels.push_back((const void*)xfwd_fn(false, pair));
+    fft_kernels.push_back((const void*)xfwd_fn(true, pair));
+    fft_kernels.push_back((const void*)xinv_fn(pair));
+    fft_kernels.push_back((const void*)pair_xfwd_fn(pair));
+    fft_kernels.push_back((const void*)pair_zmul_fn(pair));
+    fft_kernels.push_back((const void*)pair_yfft_fn(pair ? 1 : -1));
+  }
+  fft_kernels.push_back((const void*)pair_xinv_fn());
+  for (int l = 0; l < 4; ++l) fft_kernels.push_back((const void*)pair_yz_fn(l));
+  for (int c = 0; c < YZ_CLASSES; ++c)
+    fft_kernels.push_back((const void*)(c >= 15 ? yz_long_fn(c) : c >= 10 ? yz_warp_fn(c) : yz_block_fn(c)));
+  for (int lr = 3; lr <= 4; ++lr) {
+    fft_kernels.push_back((const void*)ycols_fn(-1, lr));
+    fft_kernels.push_back((const void*)ycols_fn(1, lr));
+    fft_kernels.push_back((const void*)zmul_fn(lr));
+  }
   // the DFT32 matrix of the tensor-core y transforms in its real 64 x 64 form
   // B[2 k + r][2 n + s] (output k, part r; input n, part s; forward, angle
   // 2 pi k n / 32): re <- cos re + sin im, im <- -sin re + cos im; split into
@@ -2693,7 +2649,7 @@ mpx_status mpx_profile_attempt(mpx_engine* e, int method, int reps, double ms[4]
       xfwd_fn(true, e->x_pair)<<<e->n_t_demag, e->nt_x, e->smem_x, e->stream>>>(e->d_mags, e->d_groups, e->d_t_demag, s, 1,
                                                                     nullptr, e->d_tw);
     if (e->n_t_local > 0)
-      k_combine<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, s, 0);
+      combine_fn()<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, s, 0);
     CUDA_TRY(cudaEventRecord(ev[1], e->stream));
     MPX_TRY(launch_pairs(e, -1, s, 1));
     CUDA_TRY(cudaEventRecord(ev[2], e->stream));
@@ -2707,7 +2663,7 @@ mpx_status mpx_profile_attempt(mpx_engine* e, int method, int reps, double ms[4]
     if (e->n_t_demag > 0)
       CUDA_TRY(launch_pdl(xinv_fn(e->x_pair), e->n_t_demag, e->nt_x, e->smem_x, e->stream, e->d_mags, e->d_groups, e->d_t_demag, ea,
                           e->d_tw));
-    if (e->n_t_local > 0) k_local<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, ea);
+    if (e->n_t_local > 0) local_fn()<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, ea);
     CUDA_TRY(cudaEventRecord(ev[4], e->stream));
     CUDA_TRY(cudaEventSynchronize(ev[4]));
     MPX_TRY(check_launch(e, "profile attempt"));
@@ -2797,7 +2753,7 @@ mpx_status mpx_profile_eval(mpx_engine* e, int magnet, int reps, double ms[4]) {
       for (int k = 0; k < 3; ++k) CUDA_TRY(cudaEventElapsedTime(&t[k], ev[k], ev[k + 1]));
     } else {
       CUDA_TRY(cudaEventRecord(ev[3], e->stream));
-      k_local<<<ntile, 256, 0, e->stream>>>(e->d_mags, e->d_groups, m->d_tiles, ea);
+      local_fn()<<<ntile, 256, 0, e->stream>>>(e->d_mags, e->d_groups, m->d_tiles, ea);
       CUDA_TRY(cudaEventRecord(ev[4], e->stream));
       e->launches += 1;
       CUDA_TRY(cudaEventSynchronize(ev[4]));

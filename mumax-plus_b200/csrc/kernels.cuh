@@ -33,7 +33,7 @@ struct TableauDev {
   double a[7][7];
   double b1[7], b2[7];
 };
-__constant__ TableauDev c_tab;
+static __constant__ TableauDev c_tab;
 
 // Block size bounds: the x passes hold 8 FFT values per thread, so a block of
 // X_THREADS_MAX threads covers transforms of up to 8*X_THREADS_MAX points; the
@@ -1762,358 +1762,6 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __re
     tn = fmax(tn, b);
   }
   if (ea.fsal_err) block_max2(en, tn, &groups[M.group].err_bits, &groups[M.group].tmax_bits);
-}
-
-// Local terms only (no demag): same tiles, no dynamic shared memory.
-__global__ void __launch_bounds__(256) k_local(const MagnetDev* __restrict__ mags, GroupDev* __restrict__ groups,
-                                               const Work* __restrict__ work, EpiArgs ea) {
-  __shared__ MagnetDev M;
-  __shared__ GroupDev G;
-  const Work wk = work[blockIdx.x];
-  if (!load_descs(M, G, mags, groups, wk.mag, ea.gate, ea.stage)) return;
-  const int nx = M.n[0], ny = M.n[1];
-  const float* m = ea.msrc ? ea.msrc : stage_m(M, G, ea.stage);
-  double en = 0.0, tn = 0.0;
-  const int rowbase = nx * (wk.y0 + ny * wk.z);
-  const float rn = 1.0f / (float)nx;
-  for (int e = threadIdx.x; e < wk.ty * nx; e += blockDim.x) {
-    const int yl = tile_row(e, nx, rn), x = e - yl * nx;
-    double a = 0.0, b = 0.0;
-    epilogue_cell(M, G, ea, m, x, wk.y0 + yl, wk.z, rowbase + e, f3(0, 0, 0), a, b);
-    en = (a > en || a != a) ? a : en;
-    tn = fmax(tn, b);
-  }
-  if (ea.fsal_err) block_max2(en, tn, &groups[M.group].err_bits, &groups[M.group].tmax_bits);
-}
-
-// Stage combination without a demag pass (writes the stage state xs), or the
-// final combination of a non-FSAL method with its error estimate
-// (core/rungekutta.cpp:123-151).
-__global__ void __launch_bounds__(256) k_combine(const MagnetDev* __restrict__ mags, GroupDev* __restrict__ groups,
-                                                 const Work* __restrict__ work, int stage, int final_b1) {
-  __shared__ MagnetDev M;
-  __shared__ GroupDev G;
-  const Work wk = work[blockIdx.x];
-  if (!load_descs(M, G, mags, groups, wk.mag, 1, 1)) return;
-  const int nx = M.n[0], ny = M.n[1], N = M.N;
-  float* xs = M.buf[G.map[1]];
-  const float* x0 = M.buf[G.map[0]];
-  double en = 0.0;
-  const int rowbase = nx * (wk.y0 + ny * wk.z);
-  for (int e = threadIdx.x; e < wk.ty * nx; e += blockDim.x) {
-    const int i = rowbase + e;
-    if (!in_geom(M, i)) {
-      store3(xs, N, i, load3(x0, N, i));
-      continue;
-    }
-    store3(xs, N, i, combine_cell(M, G, stage, i, final_b1 != 0));
-    if (final_b1 && G.adaptive) {
-      float3 ev = f3(0, 0, 0);
-      for (int j = 0; j < c_tab.S; ++j) {
-        const float cf = (float)(G.dt * (c_tab.b1[j] - c_tab.b2[j]));
-        const float3 kj = load3(M.buf[G.map[2 + j]], N, i);
-        ev = f3(ev.x + cf * kj.x, ev.y + cf * kj.y, ev.z + cf * kj.z);
-      }
-      const double a = sqrt((double)ev.x * ev.x + (double)ev.y * ev.y + (double)ev.z * ev.z);
-      en = (a > en || a != a) ? a : en;
-    }
-  }
-  if (final_b1) block_max2(en, 0.0, &groups[M.group].err_bits, &groups[M.group].tmax_bits);
-}
-
-// --------------------------------------------------------------- controller
-// core/rungekutta.cpp:60-82 and core/timesolver.cpp:60-111, one thread per group,
-// in FP64.  Also runs the run()/steps() state machine on the device.
-// Sampled run: time point samp_k has been reached.  Its row (and the rows of
-// the next points that need no step, as run(t_k - t) with t_k <= t takes none)
-// become due with the time; the next point that needs steps is armed as run()
-// arms its end (core/timesolver.cpp:100-109).  Returns false when no point is
-// left.
-__device__ __forceinline__ bool sample_advance(GroupDev& G) {
-  G.samp_lo = G.samp_k;
-  do {
-    G.samp_out[(size_t)G.samp_k * G.samp_row] = G.t;
-    ++G.samp_k;
-  } while (G.samp_k < G.samp_n && !(G.samp_t[G.samp_k] - G.t > 0.0));
-  G.samp_hi = G.samp_k;
-  if (G.samp_k >= G.samp_n) return false;
-  G.phase = 0;
-  G.t_stop = G.t + (G.samp_t[G.samp_k] - G.t);
-  if (!(G.t < G.t_stop - G.dt)) {
-    G.phase = 1;
-    G.dt_saved = G.dt;
-    G.dt = G.t_stop - G.t;
-  }
-  return true;
-}
-
-__global__ void k_controller(GroupDev* __restrict__ groups, int ngroups) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= ngroups) return;
-  GroupDev& G = groups[g];
-  if (G.status != GS_RUNNING) return;
-  G.samp_lo = G.samp_hi;  // the rows of the previous attempt have been written
-  const double err = __longlong_as_double((long long)G.err_bits);
-  const double tmax = __longlong_as_double((long long)G.tmax_bits);
-  G.err_bits = 0ull;
-  G.tmax_bits = 0ull;
-  G.attempts++;
-  const double dt = G.dt;
-  bool success = true;
-  if (G.adaptive) {
-    success = err < G.max_error;
-    double corr = success ? pow(G.max_error / err, 1.0 / (c_tab.order2 + 1))
-                          : pow(G.max_error / err, 1.0 / (c_tab.order1 + 1));
-    if (isnan(corr)) corr = 1.0;
-    corr *= G.headroom;
-    corr = corr > G.upper ? G.upper : corr;
-    corr = corr < G.lower ? G.lower : corr;
-    G.dt = dt * corr;
-    if (isnan(err)) {  // the reference would retry forever; fail the solve instead
-      G.status = GS_FAILED;
-      G.finished_flag = 1;
-      return;
-    }
-  }
-  if (!success) {
-    G.rejected++;
-    G.k0_valid = G.thermal ? 0 : 1;  // with noise k0 depends on dt (noise / sqrt(dt))
-    return;
-  }
-  // accept: t = t0 + dt; x0 <- x_new; FSAL: k0 <- k_{S-1}
-  G.t += dt;
-  G.steps++;
-  const int t0 = G.map[0];
-  G.map[0] = G.map[1];
-  G.map[1] = t0;
-  if (c_tab.fsal) {
-    const int k0 = G.map[2];
-    G.map[2] = G.map[2 + c_tab.S - 1];
-    G.map[2 + c_tab.S - 1] = k0;
-    G.k0_valid = G.thermal ? 0 : 1;  // a new step draws new noise
-  } else {
-    G.k0_valid = 0;
-  }
-  bool done = false;
-  if (G.phase == 1) {
-    done = true;
-    if (!G.adaptive) G.dt = G.dt_saved;
-    if (G.mode == 2) done = !sample_advance(G);
-  } else if (G.mode == 1) {
-    if (--G.steps_left <= 0) done = true;
-  } else {
-    if (G.torque_stop > 0.0 && c_tab.fsal && tmax / (double)GAMMA_LL < G.torque_stop) {
-      done = true;
-    } else if (!(G.t < G.t_stop - G.dt)) {
-      G.phase = 1;
-      G.dt_saved = G.dt;
-      G.dt = G.t_stop - G.t;
-    }
-  }
-  if (done) {
-    G.status = GS_FINISHED;
-    G.finished_flag = 1;
-    G.phase = 0;
-  }
-}
-
-// ---------------------------------------------------------------- reductions
-// Deterministic two-level reductions over the geometry: block partials in a
-// fixed order, then one block.  op 0: per-component sum, op 1: max |v|.
-__global__ void k_reduce_partial(const float* __restrict__ a, int N, int ncomp,
-                                 const unsigned char* __restrict__ geom, int op, double* partial) {
-  __shared__ double sh[3][256];
-  double acc[3] = {0, 0, 0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    if (geom && !geom[i]) continue;
-    if (op == 0) {
-      for (int c = 0; c < ncomp; ++c) acc[c] += (double)a[(size_t)c * N + i];
-    } else if (op == 2) {  // sum of squared norms (dotSum(a, a), core/reduce.cu)
-      for (int c = 0; c < ncomp; ++c) {
-        const double v = a[(size_t)c * N + i];
-        acc[0] += v * v;
-      }
-    } else {
-      double s = 0;
-      for (int c = 0; c < ncomp; ++c) {
-        const double v = a[(size_t)c * N + i];
-        s += v * v;
-      }
-      s = sqrt(s);
-      acc[0] = (s > acc[0] || s != s) ? s : acc[0];
-    }
-  }
-  for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] = acc[c];
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s)
-      for (int c = 0; c < 3; ++c) {
-        if (op != 1) sh[c][threadIdx.x] += sh[c][threadIdx.x + s];
-        else {
-          const double o = sh[c][threadIdx.x + s];
-          if (o > sh[c][threadIdx.x] || o != o) sh[c][threadIdx.x] = o;
-        }
-      }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0)
-    for (int c = 0; c < 3; ++c) partial[blockIdx.x * 3 + c] = sh[c][0];
-}
-
-__global__ void k_reduce_final(const double* __restrict__ partial, int nblocks, int op, double* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double r[3] = {0, 0, 0};
-  for (int b = 0; b < nblocks; ++b)
-    for (int c = 0; c < 3; ++c) {
-      const double v = partial[b * 3 + c];
-      if (op != 1) r[c] += v;
-      else if (v > r[c] || v != v) r[c] = v;
-    }
-  for (int c = 0; c < 3; ++c) out[c] = r[c];
-}
-
-// Sampled run: <m> of one magnet into the due rows of its group's table, with
-// the arithmetic of mpx_average (k_reduce_partial / k_reduce_final over the
-// same 256 x 256 grid), so the values equal a host-side average of the state.
-// Both kernels do nothing unless rows are due.
-__global__ void __launch_bounds__(256) k_sample_partial(const MagnetDev* __restrict__ mags,
-                                                        const GroupDev* __restrict__ groups, int slot,
-                                                        double* partial) {
-  __shared__ double sh[3][256];
-  const MagnetDev& M = mags[slot];
-  const GroupDev& G = groups[M.group];
-  if (G.samp_hi <= G.samp_lo) return;
-  const int N = M.N;
-  const float* __restrict__ a = M.buf[G.map[0]];
-  const unsigned char* __restrict__ geom = M.geom;
-  double acc[3] = {0, 0, 0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    if (geom && !geom[i]) continue;
-    for (int c = 0; c < 3; ++c) acc[c] += (double)a[(size_t)c * N + i];
-  }
-  for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] = acc[c];
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s)
-      for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] += sh[c][threadIdx.x + s];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0)
-    for (int c = 0; c < 3; ++c) partial[blockIdx.x * 3 + c] = sh[c][0];
-}
-
-__global__ void k_sample_final(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, int slot,
-                               const double* __restrict__ partial, int nblocks, long long ngeo, int col) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const GroupDev& G = groups[mags[slot].group];
-  if (G.samp_hi <= G.samp_lo) return;
-  double r[3] = {0, 0, 0};
-  for (int b = 0; b < nblocks; ++b)
-    for (int c = 0; c < 3; ++c) r[c] += partial[b * 3 + c];
-  for (int row = G.samp_lo; row < G.samp_hi; ++row)
-    for (int c = 0; c < 3; ++c) G.samp_out[(size_t)row * G.samp_row + col + c] = ngeo > 0 ? r[c] / ngeo : 0.0;
-}
-
-// Set m: normalise per cell inside the geometry (core/variable.cpp:76-87).
-__global__ void k_normalize_into(float* dst, const float* __restrict__ src, int N,
-                                 const unsigned char* __restrict__ geom) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  float x = src[i], y = src[N + i], z = src[2 * N + i];
-  if (!geom || geom[i]) {
-    const float inv = rsqrtf(x * x + y * y + z * z);
-    x *= inv;
-    y *= inv;
-    z *= inv;
-  }
-  dst[i] = x;
-  dst[N + i] = y;
-  dst[2 * N + i] = z;
-}
-
-// n normal(0,1) numbers for the initial magnetisation of a new magnet: the
-// splitmix64 finaliser of (seed, index) (Steele, Lea and Flood, OOPSLA 2014)
-// gives two 24-bit uniforms, turned into one normal by Box-Muller.
-__global__ void k_random_normal(float* __restrict__ out, int n, unsigned long long seed) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    unsigned long long z = seed + 0x9E3779B97F4A7C15ull * (unsigned long long)(i + 1);
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    z ^= z >> 31;
-    const float u1 = (float)((unsigned)(z >> 40) + 1u) * (1.0f / 16777216.0f);  // (0, 1]
-    const float u2 = (float)(unsigned)(z & 0xFFFFFFull) * (1.0f / 16777216.0f);  // [0, 1)
-    out[i] = sqrtf(-2.0f * logf(u1)) * cospif(2.0f * u2);
-  }
-}
-
-// ------------------------------------------------------------- minimizer
-// One steepest-descent step of physics/minimizer.cu (k_step): from the state m0
-// and its damping torque t0, m1 = ((4 - dt^2 t0^2) m0 + 4 dt t0) / (4 + dt^2 t0^2)
-// over every cell of the grid; m0 and the unnormalised m1 are kept for the
-// Barzilai-Borwein step size, the state becomes m1 normalised inside the
-// geometry (the reference's magnetization()->set(m1)).
-__global__ void k_min_step(float* __restrict__ state, float* __restrict__ m0_out, float* __restrict__ m1_out,
-                           const float* __restrict__ t0, int N, float dt, const unsigned char* __restrict__ geom) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    const float3 m0 = load3(state, N, i), t = load3(t0, N, i);
-    const float t2 = dt * dt * dot3(t, t);
-    const float inv = 1.0f / (4.0f + t2);
-    const float3 m1 = f3(((4.0f - t2) * m0.x + 4.0f * dt * t.x) * inv, ((4.0f - t2) * m0.y + 4.0f * dt * t.y) * inv,
-                         ((4.0f - t2) * m0.z + 4.0f * dt * t.z) * inv);
-    store3(m0_out, N, i, m0);
-    store3(m1_out, N, i, m1);
-    float3 n = m1;
-    if (!geom || geom[i]) {
-      const float r = rsqrtf(dot3(m1, m1));
-      n = f3(m1.x * r, m1.y * r, m1.z * r);
-    }
-    store3(state, N, i, n);
-  }
-}
-
-// Block partials (FP64) of dm.dm, dm.dt, dt.dt and max|dm| with dm = m1 - m0 and
-// dt = t0 - t1 (physics/minimizer.cu: BarzilianBorweinStepSize, maxVecNorm(dm)).
-__global__ void k_min_partial(const float* __restrict__ m0, const float* __restrict__ m1, const float* __restrict__ t0,
-                              const float* __restrict__ t1, int N, double* __restrict__ partial) {
-  __shared__ double sh[4][256];
-  double a = 0, b = 0, c = 0, mx = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    const float3 p = load3(m0, N, i), q = load3(m1, N, i), u = load3(t0, N, i), v = load3(t1, N, i);
-    const float3 dm = f3(q.x - p.x, q.y - p.y, q.z - p.z);
-    const float3 dt = f3(u.x - v.x, u.y - v.y, u.z - v.z);
-    const double mm = (double)dm.x * dm.x + (double)dm.y * dm.y + (double)dm.z * dm.z;
-    a += mm;
-    b += (double)dm.x * dt.x + (double)dm.y * dt.y + (double)dm.z * dt.z;
-    c += (double)dt.x * dt.x + (double)dt.y * dt.y + (double)dt.z * dt.z;
-    const double n = sqrt(mm);
-    mx = (n > mx || n != n) ? n : mx;
-  }
-  sh[0][threadIdx.x] = a;
-  sh[1][threadIdx.x] = b;
-  sh[2][threadIdx.x] = c;
-  sh[3][threadIdx.x] = mx;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      for (int k = 0; k < 3; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + s];
-      const double o = sh[3][threadIdx.x + s];
-      if (o > sh[3][threadIdx.x] || o != o) sh[3][threadIdx.x] = o;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 4; ++k) partial[blockIdx.x * 4 + k] = sh[k][0];
-}
-
-__global__ void k_min_final(const double* __restrict__ partial, int nblocks, double* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double r[4] = {0, 0, 0, 0};
-  for (int b = 0; b < nblocks; ++b) {
-    for (int k = 0; k < 3; ++k) r[k] += partial[b * 4 + k];
-    const double v = partial[b * 4 + 3];
-    if (v > r[3] || v != v) r[3] = v;
-  }
-  for (int k = 0; k < 4; ++k) out[k] = r[k];
 }
 
 }  // namespace mpx

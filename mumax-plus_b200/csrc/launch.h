@@ -1,0 +1,68 @@
+// launch.h -- the kernels of the demag passes and of the Runge-Kutta stages, as
+// the engine launches them.  The instantiations are compiled in one file per
+// family (xpass.cu, yz.cu, yzwarp.cu, yzlong.cu, thick.cu, pairs.cu), so that a change of
+// one kernel compiles that family only and the families compile in parallel;
+// engine.cu reaches them through these functions.  The index-checked build
+// (-DMPX_BOUNDS_CHECK) keeps everything in one translation unit (checked.cu):
+// its record of the first bad index is one device variable.
+#pragma once
+#include "../../include/mpx.h"
+#include "kernels.cuh"
+
+namespace mpx {
+
+// ---- the pair grid of stray fields (pairfft.cuh)
+constexpr int PF_THREADS = 512;
+constexpr int PF_LR = 3;                              // log2 of the largest radix
+constexpr int PF_POINTS = (1 << PF_LR) * PF_THREADS;  // points of one transform group
+
+struct PairFft {
+  float2* t;         // work spectrum (or, while it is made, the kernel spectrum)
+  const float2* ks;  // kernel spectrum
+  int logP[3];
+  int nin[3];   // rows of the input per axis (source grid, or the table K)
+  int win[3];   // first row of the output window per axis (n_A - 1)
+  int nout[3];  // rows of the output window per axis (n_B)
+  float scale;  // -mu0 / (Px Py Pz)
+};
+
+using XfwdFn = void (*)(const MagnetDev*, const GroupDev*, const Work*, int, int, const float*, const float2*);
+using XinvFn = void (*)(const MagnetDev*, GroupDev*, const Work*, EpiArgs, const float2*);
+using LocalFn = void (*)(const MagnetDev*, GroupDev*, const Work*, EpiArgs);
+using CombineFn = void (*)(const MagnetDev*, GroupDev*, const Work*, int, int);
+using ControllerFn = void (*)(GroupDev*, int);
+using YzFn = void (*)(const MagnetDev*, const GroupDev*, const Work*, int, int, const float2*);
+
+// xpass.cu: everything that reads the Butcher tableau
+XfwdFn xfwd_fn(bool combine, bool pair);
+XinvFn xinv_fn(bool pair);
+LocalFn local_fn();
+CombineFn combine_fn();
+ControllerFn controller_fn();
+cudaError_t upload_tableau_symbol(const TableauDev& t, cudaStream_t stream);
+
+// Launch classes of the y/z pass (yz_class of engine.cu): 0 .. 9 the block-wide
+// passes (yz.cu), 10 .. 14 the warp columns of y lengths 64 .. 512 (yzwarp.cu),
+// 15 .. 23 y lengths 1024 and 2048 (yzlong.cu).
+constexpr int YZ_CLASSES = 24;
+YzFn yz_block_fn(int cls);
+YzFn yz_warp_fn(int cls);
+YzFn yz_long_fn(int cls);
+
+// thick.cu: the split y/z path
+YzFn ycols_fn(int dir, int maxlr);
+YzFn zmul_fn(int maxlr);
+
+// pairs.cu: stray fields on the pair grid
+using PairXfwdFn = void (*)(const MagnetDev*, const GroupDev*, int, int, int, const float*, PairFft, int, int,
+                            const float2*);
+using PairYfftFn = void (*)(const MagnetDev*, const GroupDev*, int, int, int, PairFft, int, int, const float2*);
+using PairYzFn = void (*)(const MagnetDev*, const GroupDev*, int, int, int, PairFft, const float2*);
+using PairXinvFn = void (*)(const MagnetDev*, const GroupDev*, int, int, int, PairFft, int, int, float*, const float2*);
+PairXfwdFn pair_xfwd_fn(bool table);
+PairYfftFn pair_yfft_fn(int dir);
+PairYfftFn pair_zmul_fn(bool mul);
+PairYzFn pair_yz_fn(int logPz);
+PairXinvFn pair_xinv_fn();
+
+}  // namespace mpx

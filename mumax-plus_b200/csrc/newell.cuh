@@ -47,7 +47,7 @@ __device__ __forceinline__ int newell_w(int dx, int dy, int dz) {
   return s == 0 ? 8 : s == 1 ? -4 : s == 2 ? 2 : -1;
 }
 
-__device__ double newell_nxx(int ix, int iy, int iz, double cx, double cy, double cz) {
+static __device__ double newell_nxx(int ix, int iy, int iz, double cx, double cy, double cz) {
   double r = 0;
   for (int dx = -1; dx <= 1; ++dx)
     for (int dy = -1; dy <= 1; ++dy)
@@ -56,7 +56,7 @@ __device__ double newell_nxx(int ix, int iy, int iz, double cx, double cy, doubl
   return r / (4 * M_PI * cx * cy * cz);
 }
 
-__device__ double newell_nxy(int ix, int iy, int iz, double cx, double cy, double cz) {
+static __device__ double newell_nxy(int ix, int iy, int iz, double cx, double cy, double cz) {
   if (ix == 0 || iy == 0) return 0;
   double r = 0;
   for (int dx = -1; dx <= 1; ++dx)
@@ -67,7 +67,7 @@ __device__ double newell_nxy(int ix, int iy, int iz, double cx, double cy, doubl
 }
 
 // component c (xx, yy, zz, xy, xz, yz) at displacement (x, y, z) cells
-__device__ double newell_comp(int c, int x, int y, int z, double cx, double cy, double cz) {
+static __device__ double newell_comp(int c, int x, int y, int z, double cx, double cy, double cz) {
   switch (c) {
     case 0: return newell_nxx(x, y, z, cx, cy, cz);
     case 1: return newell_nxx(y, z, x, cy, cz, cx);
@@ -87,7 +87,7 @@ struct KernelGeom {
 
 // Octant values N_c(|rx|, |ry|, |rz|) for |r_a| < n_a, all 6 components, FP64.
 // out layout: [c][rz][ry][rx]
-__global__ void k_newell_octant(double* __restrict__ out, KernelGeom g) {
+static __global__ void k_newell_octant(double* __restrict__ out, KernelGeom g) {
   const long long total = (long long)g.n[0] * g.n[1] * g.n[2];
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -108,7 +108,7 @@ __global__ void k_newell_octant(double* __restrict__ out, KernelGeom g) {
 
 // Reference-layout real-space kernel (physics/strayfieldkernel.cu:80-99):
 // grid K with origin O (cells), 6 comps, cast to float.
-__global__ void k_newell_reflayout(float* __restrict__ out, KernelGeom g, int K0, int K1, int K2, int O0, int O1,
+static __global__ void k_newell_reflayout(float* __restrict__ out, KernelGeom g, int K0, int K1, int K2, int O0, int O1,
                                    int O2) {
   const long long total = (long long)K0 * K1 * K2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
@@ -133,7 +133,7 @@ __global__ void k_newell_reflayout(float* __restrict__ out, KernelGeom g, int K0
 // component, xy odd in x and y, xz in x and z, yz in y and z, also after the sum
 // over periodic images (their repetitions run over -p .. p), so each output is
 // an input entry times the signs of its odd components.
-__global__ void k_newell_expand_abs(float* __restrict__ out, const float* __restrict__ abs_tab, int K0, int K1,
+static __global__ void k_newell_expand_abs(float* __restrict__ out, const float* __restrict__ abs_tab, int K0, int K1,
                                     int K2, int O0, int O1, int O2, int A0, int A1, int A2, int L0, int L1, int L2) {
   const long long total = (long long)K0 * K1 * K2, ltot = (long long)L0 * L1 * L2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
@@ -154,7 +154,7 @@ __global__ void k_newell_expand_abs(float* __restrict__ out, const float* __rest
 
 // Expand component c of the octant table to the circular P-grid (imag = 0).
 // Parity: xy odd in x,y; xz odd in x,z; yz odd in y,z; diagonal even.
-__global__ void k_kernel_expand(double2* __restrict__ full, const double* __restrict__ oct, int c, KernelGeom g,
+static __global__ void k_kernel_expand(double2* __restrict__ full, const double* __restrict__ oct, int c, KernelGeom g,
                                 int P0, int P1, int P2) {
   const long long total = (long long)P0 * P1 * P2;
   const long long noct = (long long)g.n[0] * g.n[1] * g.n[2];
@@ -180,7 +180,7 @@ __global__ void k_kernel_expand(double2* __restrict__ full, const double* __rest
 // Consecutive threads take consecutive butterflies of a line along x and
 // consecutive lines (adjacent x) along y and z, so that every load and store
 // of a warp is contiguous.
-__global__ void k_fft64_pass(const double2* __restrict__ in, double2* __restrict__ out, int P0, int P1, int P2,
+static __global__ void k_fft64_pass(const double2* __restrict__ in, double2* __restrict__ out, int P0, int P1, int P2,
                              int axis, int Ns) {
   const int L = axis == 0 ? P0 : axis == 1 ? P1 : P2;
   const long long stride = axis == 0 ? 1 : axis == 1 ? P0 : (long long)P0 * P1;
@@ -208,7 +208,7 @@ __global__ void k_fft64_pass(const double2* __restrict__ in, double2* __restrict
 
 // Store the real, symmetry-reduced spectrum of component c (slot kc of kcomp)
 // in the layout read by k_yz: [kx][kz'][kcomp][ky'].
-__global__ void k_kernel_extract(float* __restrict__ kspec, const double2* __restrict__ full, int kc, int kcomp,
+static __global__ void k_kernel_extract(float* __restrict__ kspec, const double2* __restrict__ full, int kc, int kcomp,
                                  int P0, int P1, int P2, double pref) {
   const int Fh = P0 / 2 + 1, hy = P1 / 2 + 1, hz = P2 / 2 + 1;
   const long long total = (long long)Fh * hy * hz;

@@ -35,23 +35,9 @@
 // per group) and at most 64 registers, so that two blocks share an SM (the
 // radix-16 form needed ~150 registers: one 8-warp block per SM).
 #pragma once
-#include "stray.cuh"
+#include "launch.h"
 
 namespace mpx {
-
-constexpr int PF_THREADS = 512;
-constexpr int PF_LR = 3;                              // log2 of the largest radix
-constexpr int PF_POINTS = (1 << PF_LR) * PF_THREADS;  // points of one transform group
-
-struct PairFft {
-  float2* t;         // work spectrum (or, while it is made, the kernel spectrum)
-  const float2* ks;  // kernel spectrum
-  int logP[3];
-  int nin[3];   // rows of the input per axis (source grid, or the table K)
-  int win[3];   // first row of the output window per axis (n_A - 1)
-  int nout[3];  // rows of the output window per axis (n_B)
-  float scale;  // -mu0 / (Px Py Pz)
-};
 
 // Forward x transforms.  TABLE: input the tabulated tensor [q][z][y][x] of
 // `ncomp` = 6 components; else Ms m of the source magnet's state for `stage`
@@ -299,7 +285,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) k_pair_yz(const MagnetDev* __re
 // rest by Hermitian symmetry, inverse FFT; x of the window, scaled, into
 // `out` (3 x N_B, component-major; added with `add`), zero outside the
 // destination's geometry.  Block: rows y0 .. y0 + ry - 1 of (c, z).
-__global__ void __launch_bounds__(PF_THREADS, 2) k_pair_xinv(const MagnetDev* __restrict__ mags,
+static __global__ void __launch_bounds__(PF_THREADS, 2) k_pair_xinv(const MagnetDev* __restrict__ mags,
                                                           const GroupDev* __restrict__ groups, int dst, int stage,
                                                           int gate, PairFft pf, int ry, int add,
                                                           float* __restrict__ out, const float2* __restrict__ tw) {

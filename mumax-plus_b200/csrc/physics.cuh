@@ -143,7 +143,7 @@ __device__ __forceinline__ bool in_geom(const MagnetDev& M, int i) { return !M.g
 // access is recorded (bit 63 set, N in bits 32..62, i in the low word) and
 // skipped -- a load gives 0 -- so the kernel runs to its end and the host reads
 // the record with mpx_bounds_check.  Nothing traps.
-__device__ unsigned long long g_bounds_first_bad;
+static __device__ unsigned long long g_bounds_first_bad;
 __device__ __forceinline__ bool cell_ok(int N, int i) {
   if ((unsigned)i < (unsigned)N) return true;
   atomicCAS(&g_bounds_first_bad, 0ull, (1ull << 63) | ((unsigned long long)(unsigned)N << 32) | (unsigned)i);
@@ -456,7 +456,7 @@ __device__ __forceinline__ float3 llg_torque(float3 m, float3 h, float a) {
 // differences of m along the current, neighbours in the grid with msat != 0,
 // mastergrid wrap) or Slonczewski (current along z through a free layer).
 constexpr float MUB_F = 9.274009152e-24f, QE_F = 1.60217646e-19f, HBAR_F = 1.054571817e-34f;
-__device__ __noinline__ float3 stt_torque(const MagnetDev& M, const float* __restrict__ m, int x, int y, int z, int i,
+static __device__ __noinline__ float3 stt_torque(const MagnetDev& M, const float* __restrict__ m, int x, int y, int z, int i,
                                           float3 mc) {
   const int N = M.N;
   const float ms = M.msat.at(i), alpha = M.alpha.at(i);
@@ -523,7 +523,7 @@ __device__ __forceinline__ float thermal_normal(unsigned long long seed, long lo
 
 // physics/thermalnoise.cu:20-43: the thermal field of the step times 1/sqrt(dt)
 // (added to every stage, core/rungekutta.cpp:100-106)
-__device__ __noinline__ float3 thermal_term(const MagnetDev& M, int i, long long step, double dt) {
+static __device__ __noinline__ float3 thermal_term(const MagnetDev& M, int i, long long step, double dt) {
   const float ms = M.msat.at(i), T = M.temp.at(i), a = M.alpha.at(i);
   if (ms == 0.f || T == 0.f) return f3(0.f, 0.f, 0.f);
   const float s = sqrtf(M.noise_pref * a * T / ((1 + a * a) * ms)) * (float)(1.0 / sqrt(dt));

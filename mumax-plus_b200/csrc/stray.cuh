@@ -27,7 +27,7 @@ struct StrayTable {
 // outside its geometry get no stray field.  The source state is A's state for
 // `stage` (x0 for stage 0, the stage state otherwise); `gate` skips groups that
 // are not running, as the other stage kernels.
-__global__ void __launch_bounds__(256) k_stray_pair(const MagnetDev* __restrict__ mags,
+static __global__ void __launch_bounds__(256) k_stray_pair(const MagnetDev* __restrict__ mags,
                                                     const GroupDev* __restrict__ groups, int src, int dst,
                                                     StrayTable tab, int stage, int gate, int add,
                                                     float* __restrict__ out) {

@@ -1,0 +1,13 @@
+// thick.cu -- the split y/z path of thick magnets (yzsplit.cuh).
+#include "launch.h"
+#include "yzsplit.cuh"
+
+namespace mpx {
+
+YzFn ycols_fn(int dir, int maxlr) {
+  if (dir < 0) return maxlr == 3 ? k_ycols<-1, 3> : k_ycols<-1, 4>;
+  return maxlr == 3 ? k_ycols<1, 3> : k_ycols<1, 4>;
+}
+YzFn zmul_fn(int maxlr) { return maxlr == 3 ? k_zmul<3> : k_zmul<4>; }
+
+}  // namespace mpx

@@ -1,0 +1,16 @@
+// yzwarp.cu -- the warp-column y/z pass k_yzw of y lengths 64 .. 512.
+#include "launch.h"
+
+namespace mpx {
+
+YzFn yz_warp_fn(int cls) {
+  switch (cls) {
+    case 10: return k_yzw<1>;
+    case 11: return k_yzw<2>;
+    case 12: return k_yzw<4>;
+    case 13: return k_yzw<8>;
+    default: return k_yzw<16>;
+  }
+}
+
+}  // namespace mpx
