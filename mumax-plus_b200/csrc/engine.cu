@@ -861,14 +861,61 @@ mpx_status rebuild_tables(mpx_engine* e) {
 // the FP32 table of the Newell tensor (built in FP64, PBC images included) of
 // their displacements; B gets a stray-field buffer and FLAG_STRAY.
 mpx_status setup_magnet(mpx_engine* e, Magnet* m, const mpx_magnet_desc* d, bool keep_fields);
+mpx_status check_launch(mpx_engine* e, const char* what);
 void release_all(mpx_engine* e, Magnet* m);
 
 // Pairs whose direct sum would take at least this many cell interactions use
 // the FFT form on the pair's kernel grid (periodic images included).
 constexpr long long STRAY_FFT_MIN_INTERACTIONS = 1LL << 22;
 
+// The lattice of the integrals that a table of displacements O + j, j < K per
+// axis, with the images of g, meets (newell.cuh), and how many of its `ncomp`
+// components are held at once: all where they take at most NEWELL_LATTICE_MAX,
+// one at a time where one does, none (the point-by-point sum) beyond.
+constexpr int64_t NEWELL_LATTICE_MAX = 1LL << 30;
+int newell_lattice(const KernelGeom& g, const int K[3], const int O[3], int ncomp, NewellLattice* L) {
+  int64_t n = 8;
+  for (int a = 0; a < 3; ++a) {
+    const int64_t reach = (int64_t)g.pbc[a] * g.mg[a] + 1, lo = O[a] - reach, hi = O[a] + K[a] - 1 + reach;
+    const int64_t a0 = lo <= 0 && hi >= 0 ? 0 : std::min(std::abs(lo), std::abs(hi));
+    const int64_t len = std::max(std::abs(lo), std::abs(hi)) - a0 + 1;
+    if (len > (1 << 24)) return 0;
+    L->a0[a] = (int)a0;
+    L->len[a] = (int)len;
+    n *= len;
+    if (n > NEWELL_LATTICE_MAX) return 0;
+  }
+  return n * ncomp <= NEWELL_LATTICE_MAX ? ncomp : 1;
+}
+
+// Components 0 .. ncomp - 1 of the Newell tensor, with the periodic images of g, at
+// the displacements O + j, j < K per axis, into out (layout [c][z][y][x]).
+template <typename T>
+mpx_status newell_table(mpx_engine* e, const KernelGeom& g, const int K[3], const int O[3], int ncomp, T* out) {
+  const int grid = 148 * 8;
+  NewellLattice L;
+  const int nc = newell_lattice(g, K, O, ncomp, &L);
+  double* lat = nullptr;
+  if (nc > 0) {
+    const size_t lt = (size_t)L.len[0] * L.len[1] * L.len[2];
+    if (palloc(e, (void**)&lat, sizeof(double) * nc * lt) != MPX_OK) lat = nullptr;  // no room: point by point
+  }
+  if (lat) {
+    for (int c0 = 0; c0 < ncomp; c0 += nc) {
+      k_newell_lattice<<<grid, 128, 0, e->stream>>>(lat, g, L, c0, nc);
+      k_newell_from_lattice<<<grid, 256, 0, e->stream>>>(out, lat, g, L, c0, nc, K[0], K[1], K[2], O[0], O[1], O[2]);
+      e->launches += 2;
+    }
+    pfree(e, lat);
+  } else {
+    k_newell_direct<<<grid, 128, 0, e->stream>>>(out, g, K[0], K[1], K[2], O[0], O[1], O[2], ncomp);
+    e->launches++;
+  }
+  return check_launch(e, "Newell tensor");
+}
+
 // The FP32 table of the Newell tensor, with the periodic images of g, at the
-// displacements O + j, j < K per axis (k_newell_reflayout's layout).  Where a
+// displacements O + j, j < K per axis (newell_table's layout).  Where a
 // displacement range reaches both signs the tensor is evaluated over the
 // absolute displacements only and expanded by the components' parities
 // (k_newell_expand_abs): for two overlapping grids a quarter to an eighth of
@@ -889,15 +936,18 @@ mpx_status build_pair_table(mpx_engine* e, const KernelGeom& g, const int K[3], 
     kt *= K[a];
   }
   if (2 * lt > kt) {
-    k_newell_reflayout<<<148 * 8, 128, 0, e->stream>>>(out, g, K[0], K[1], K[2], O[0], O[1], O[2]);
-    e->launches++;
+    MPX_TRY(newell_table(e, g, K, O, 6, out));
   } else {
     float* abs_tab = nullptr;
     MPX_TRY(palloc(e, (void**)&abs_tab, sizeof(float) * 6 * (size_t)lt));
-    k_newell_reflayout<<<148 * 8, 128, 0, e->stream>>>(abs_tab, g, L[0], L[1], L[2], A[0], A[1], A[2]);
+    const mpx_status st = newell_table(e, g, L, A, 6, abs_tab);
+    if (st != MPX_OK) {
+      pfree(e, abs_tab);
+      return st;
+    }
     k_newell_expand_abs<<<148 * 8, 256, 0, e->stream>>>(out, abs_tab, K[0], K[1], K[2], O[0], O[1], O[2], A[0], A[1],
                                                         A[2], L[0], L[1], L[2]);
-    e->launches += 2;
+    e->launches += 1;
     pfree(e, abs_tab);
   }
   return MPX_OK;
@@ -1163,6 +1213,23 @@ mpx_status launch_pairs(mpx_engine* e, int dst, int stage, int gate) {
 }
 
 // ------------------------------------------------ demag kernel construction
+// Complex lines per block of a kernel transform of length P (about 2048 points),
+// and its dynamic shared memory.
+int kernel_axis_lines(int P) { return std::max(1, std::min(128, 2048 / P)); }
+int kernel_axis_smem(int P) { return (2 * kernel_axis_lines(P) + 1) * P * (int)sizeof(double2); }
+
+// Device bytes the construction holds beside the spectrum: the octant table with
+// the lattice of its integrals, then with the two transform arrays.
+int64_t kernel_build_bytes(const KernelGeom& g, const int P[3], int kcomp) {
+  const int O[3] = {0, 0, 0};
+  NewellLattice L;
+  const int nc = newell_lattice(g, g.n, O, kcomp, &L);
+  const int64_t lat = nc > 0 ? 8 * (int64_t)nc * L.len[0] * L.len[1] * L.len[2] : 0;
+  const int64_t Fh = P[0] / 2 + 1, hy = P[1] / 2 + 1;
+  return 8 * (int64_t)kcomp * g.n[0] * g.n[1] * g.n[2] +
+         std::max(lat, 8 * (int64_t)kcomp * g.n[2] * Fh * (g.n[1] + hy));
+}
+
 mpx_status build_kernel_spectrum(mpx_engine* e, Magnet* m) {
   MagnetDev& d = m->dev;
   KernelGeom g;
@@ -1172,45 +1239,41 @@ mpx_status build_kernel_spectrum(mpx_engine* e, Magnet* m) {
     g.pbc[a] = m->kkey_pbc[a];
     g.cs[a] = m->kkey_cs[a];
   }
-  const long long noct = (long long)d.n[0] * d.n[1] * d.n[2];
-  const long long PP = (long long)m->P[0] * m->P[1] * m->P[2];
-  double* oct = nullptr;
-  double2 *f0 = nullptr, *f1 = nullptr;
-  mpx_status ast = palloc(e, (void**)&oct, sizeof(double) * 6 * noct);
-  if (ast == MPX_OK) ast = palloc(e, (void**)&f0, sizeof(double2) * PP);
-  if (ast == MPX_OK) ast = palloc(e, (void**)&f1, sizeof(double2) * PP);
-  if (ast != MPX_OK) {
-    pfree(e, oct);
-    pfree(e, f0);
-    return fail(MPX_ERR_NOMEM, "demag kernel construction: out of device memory");
+  // octant table, then one cosine / sine transform per axis (k_kernel_axis):
+  // [c][z][y][x] -> [c][z][kx][y] -> [c][kx][z][ky] -> kspec[kx][kz'][c][ky']
+  const int kcomp = d.kcomp, nx = d.n[0], ny = d.n[1], nz = d.n[2];
+  const int Fh = m->P[0] / 2 + 1, hy = m->P[1] / 2 + 1, hz = m->P[2] / 2 + 1;
+  double *oct = nullptr, *tx = nullptr, *ty = nullptr;
+  mpx_status st = palloc(e, (void**)&oct, sizeof(double) * kcomp * (size_t)d.N);
+  const int O[3] = {0, 0, 0};
+  if (st == MPX_OK) st = newell_table(e, g, d.n, O, kcomp, oct);
+  if (st == MPX_OK) st = palloc(e, (void**)&tx, sizeof(double) * kcomp * (size_t)nz * Fh * ny);
+  if (st == MPX_OK) st = palloc(e, (void**)&ty, sizeof(double) * kcomp * (size_t)nz * Fh * hy);
+  if (st == MPX_OK) {
+    KernelAxis ax{nx, m->P[0], ny, nz, 1, nx, (long long)nz * ny * nx, (long long)ny * nx,
+                  ny, 1, (long long)nz * Fh * ny, (long long)Fh * ny, 0x18, {1, 1, 1, 1, 1, 1}};
+    KernelAxis ay{ny, m->P[1], Fh, nz, 1, ny, (long long)nz * Fh * ny, (long long)Fh * ny,
+                  1, (long long)nz * hy, (long long)Fh * nz * hy, hy, 0x28, {1, 1, 1, 1, 1, 1}};
+    KernelAxis az{nz, m->P[2], hy, Fh, hy, 1, (long long)Fh * nz * hy, (long long)nz * hy,
+                  (long long)kcomp * hy, 1, hy, (long long)hz * kcomp * hy, 0x30, {}};
+    const double pref = -MU0_D / ((double)m->P[0] * m->P[1] * m->P[2]);
+    for (int c = 0; c < 6; ++c) az.scale[c] = c < 3 ? pref : -pref;  // two odd axes: (-i)^2
+    auto launch = [&](auto* kernel, const double* in, auto* out, const KernelAxis& A) {
+      const int TL = kernel_axis_lines(A.P);
+      kernel<<<kcomp * A.n2 * ((A.inner + 2 * TL - 1) / (2 * TL)), 256, kernel_axis_smem(A.P), e->stream>>>(in, out, A,
+                                                                                                           TL);
+      e->launches++;
+    };
+    launch(k_kernel_axis<double>, oct, tx, ax);
+    launch(k_kernel_axis<double>, tx, ty, ay);
+    launch(k_kernel_axis<float>, ty, m->kspec, az);
+    st = check_launch(e, "kernel build launch");
   }
-  const int grid = 148 * 8;
-  k_newell_octant<<<grid, 128, 0, e->stream>>>(oct, g);
-  e->launches++;
-  const int kcomp = d.kcomp;
-  const int comps6[6] = {0, 1, 2, 3, 4, 5};
-  const double pref = -MU0_D / (double)PP;
-  for (int kc = 0; kc < kcomp; ++kc) {
-    const int c = comps6[kc];
-    k_kernel_expand<<<grid, 256, 0, e->stream>>>(f0, oct, c, g, m->P[0], m->P[1], m->P[2]);
-    e->launches++;
-    double2 *in = f0, *out = f1;
-    for (int axis = 0; axis < 3; ++axis) {
-      for (int Ns = 1; Ns < m->P[axis]; Ns <<= 1) {
-        k_fft64_pass<<<grid, 256, 0, e->stream>>>(in, out, m->P[0], m->P[1], m->P[2], axis, Ns);
-        e->launches++;
-        std::swap(in, out);
-      }
-    }
-    k_kernel_extract<<<grid, 256, 0, e->stream>>>(m->kspec, in, kc, kcomp, m->P[0], m->P[1], m->P[2], pref);
-    e->launches++;
-  }
-  cudaError_t st = cudaGetLastError();
   pfree(e, oct);
-  pfree(e, f0);
-  pfree(e, f1);
-  cudaError_t st2 = cudaStreamSynchronize(e->stream);
-  if (st != cudaSuccess) return fail(MPX_ERR_CUDA, std::string("kernel build launch: ") + cudaGetErrorString(st));
+  pfree(e, tx);
+  pfree(e, ty);
+  if (st != MPX_OK) return st;
+  const cudaError_t st2 = cudaStreamSynchronize(e->stream);
   if (st2 != cudaSuccess) return fail(MPX_ERR_CUDA, std::string("kernel build: ") + cudaGetErrorString(st2));
   m->kspec_ready = true;
   return MPX_OK;
@@ -1698,7 +1761,7 @@ mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
       const Magnet* m = get_mag(e, sg->magnets[j]);
       if (!m) continue;
       k_sample_partial<<<256, 256, 0, e->stream>>>(e->d_mags, e->d_groups, m->slot, e->d_red);
-      k_sample_final<<<1, 32, 0, e->stream>>>(e->d_mags, e->d_groups, m->slot, e->d_red, 256, (long long)m->ngeo,
+      k_sample_final<<<1, 256, 0, e->stream>>>(e->d_mags, e->d_groups, m->slot, e->d_red, 256, (long long)m->ngeo,
                                              1 + 3 * (int)j);
       e->launches += 2;
     }
@@ -1804,7 +1867,7 @@ mpx_status sensible_timestep(mpx_engine* e, Group* g, double* out) {
     MPX_TRY(eval_into(e, m, g->torque_kind ? MPX_Q_DAMPING_TORQUE : MPX_Q_TORQUE, e->d_scratch));
     const int nb = 256;
     k_reduce_partial<<<nb, 256, 0, e->stream>>>(e->d_scratch, N, 3, m->geom, 1, e->d_red);
-    k_reduce_final<<<1, 32, 0, e->stream>>>(e->d_red, nb, 1, e->d_redout);
+    k_reduce_final<<<1, 256, 0, e->stream>>>(e->d_red, nb, 1, e->d_redout);
     e->launches += 2;
     double r[3];
     CUDA_TRY(cudaMemcpyAsync(r, e->d_redout, sizeof(r), cudaMemcpyDeviceToHost, e->stream));
@@ -1975,6 +2038,8 @@ mpx_status mpx_engine_create(int device, mpx_engine** out) {
     const void* tck[] = {(const void*)k_ydft_tc<-1>, (const void*)k_ydft_tc<1>};
     for (const void* k : tck) CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
   }
+  CUDA_TRY(cudaFuncSetAttribute(k_kernel_axis<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
+  CUDA_TRY(cudaFuncSetAttribute(k_kernel_axis<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
   for (const void* k : fft_kernels) {
     cudaFuncAttributes fa;
     CUDA_TRY(cudaFuncGetAttributes(&fa, k));
@@ -2383,7 +2448,14 @@ mpx_status mpx_magnet_bytes(const mpx_magnet_desc* d, int64_t* resident, int64_t
       const int64_t nkz = std::max(1, std::min(P[1], (YZ_VPT * YZ_THREADS) / (3 * P[2])));
       res += (int64_t)sizeof(Work) * ((Fh * 3 * d->size[2] + ncy - 1) / ncy + Fh * ((P[1] + nkz - 1) / nkz));
     }
-    tr += 8 * 6 * N + 2 * 16 * (int64_t)P[0] * P[1] * P[2];    // FP64 octant + two transform buffers
+    KernelGeom g;
+    for (int a = 0; a < 3; ++a) {
+      g.n[a] = d->size[a];
+      g.mg[a] = d->mastergrid_size[a];
+      g.pbc[a] = d->pbc_repetitions[a];
+      g.cs[a] = d->cellsize[a];
+    }
+    tr += kernel_build_bytes(g, P, kc);  // FP64 construction of the kernel spectrum
   }
   *resident = res;
   *transient = tr;
@@ -2463,7 +2535,7 @@ static mpx_status reduce_quantity(mpx_engine* e, Magnet* m, int quantity, int op
   MPX_TRY(eval_into(e, m, quantity, e->d_scratch));
   const int nb = 256;
   k_reduce_partial<<<nb, 256, 0, e->stream>>>(e->d_scratch, N, nc, m->geom, op, e->d_red);
-  k_reduce_final<<<1, 32, 0, e->stream>>>(e->d_red, nb, op, e->d_redout);
+  k_reduce_final<<<1, 256, 0, e->stream>>>(e->d_red, nb, op, e->d_redout);
   e->launches += 2;
   MPX_TRY(check_launch(e, "reduce"));
   CUDA_TRY(cudaMemcpyAsync(out, e->d_redout, sizeof(double) * 3, cudaMemcpyDeviceToHost, e->stream));
@@ -2797,8 +2869,11 @@ mpx_status mpx_demag_kernel(mpx_engine* e, int magnet, float* out, int dims[3]) 
   const size_t KK = (size_t)K[0] * K[1] * K[2];
   float* d = nullptr;
   MPX_TRY(palloc(e, (void**)&d, sizeof(float) * 6 * KK));
-  k_newell_reflayout<<<148 * 8, 128, 0, e->stream>>>(d, g, K[0], K[1], K[2], O[0], O[1], O[2]);
-  e->launches++;
+  const mpx_status ts = newell_table(e, g, K, O, 6, d);
+  if (ts != MPX_OK) {
+    pfree(e, d);
+    return ts;
+  }
   cudaError_t st = cudaMemcpyAsync(out, d, sizeof(float) * 6 * KK, cudaMemcpyDeviceToHost, e->stream);
   pfree(e, d);
   if (st == cudaSuccess) st = cudaStreamSynchronize(e->stream);
@@ -3116,7 +3191,7 @@ mpx_status mpx_minimize(mpx_engine* e, int group, double tol, int nsamples) {
       MagnetDev& D = ms[j]->dev;
       k_min_partial<<<nb, 256, 0, e->stream>>>(D.buf[G.map[m0]], D.buf[G.map[m1]], D.buf[G.map[t0]],
                                                D.buf[G.map[t1]], D.N, e->d_red);
-      k_min_final<<<1, 32, 0, e->stream>>>(e->d_red, nb, e->d_redout);
+      k_min_final<<<1, 256, 0, e->stream>>>(e->d_red, nb, e->d_redout);
       e->launches += 2;
       MPX_TRY(check_launch(e, "minimize"));
       double r[4];
@@ -3393,7 +3468,7 @@ extern "C" mpx_status mpx_reduce_noalloc(const float* field, int ncells, int nco
   // every partial slot the final pass reads is written by this call's partial
   // pass, and the final pass overwrites the results: nothing needs clearing
   k_reduce_partial<<<NOALLOC_BLOCKS, 256, 0, s>>>(field, ncells, ncomp, geometry, op, scratch);
-  k_reduce_final<<<1, 32, 0, s>>>(scratch, NOALLOC_BLOCKS, op, scratch + NOALLOC_RESULT);
+  k_reduce_final<<<1, 256, 0, s>>>(scratch, NOALLOC_BLOCKS, op, scratch + NOALLOC_RESULT);
   cudaError_t st = cudaGetLastError();
   if (st != cudaSuccess) return fail(MPX_ERR_CUDA, std::string("mpx_reduce_noalloc: ") + cudaGetErrorString(st));
   CUDA_TRY(cudaMemcpyAsync(out, scratch + NOALLOC_RESULT, sizeof(double) * 3, cudaMemcpyDeviceToHost, s));

@@ -53,6 +53,20 @@ YzFn yz_long_fn(int cls);
 YzFn ycols_fn(int dir, int maxlr);
 YzFn zmul_fn(int maxlr);
 
+// Their warp-column forms (k_ycw, k_zcw of yzsplit.cuh): block sizes, columns or ky
+// per block, and dynamic shared memory.
+constexpr int YCW_THREADS = 256;  // 8 warps, 32 / Q columns (1024 values) each
+__host__ __device__ constexpr int ycw_cols(int Py) { return YCW_THREADS * 32 / Py; }
+__host__ __device__ constexpr int ycw_smem(int Py) {
+  return ((YCW_THREADS / 32) * (1024 / Py) * qlen(Py) + Py) * (int)sizeof(float2);
+}
+
+constexpr int ZCW_UNITS = 3, ZCW_THREADS = 96 * ZCW_UNITS;
+__host__ __device__ constexpr int zcw_kys(int Pz) { return ZCW_UNITS * (1024 / Pz); }
+__host__ __device__ constexpr int zcw_smem(int Pz) {
+  return (ZCW_UNITS * 3 * (1024 / Pz) * qlen(Pz) + Pz) * (int)sizeof(float2);
+}
+
 // pairs.cu: stray fields on the pair grid
 using PairXfwdFn = void (*)(const MagnetDev*, const GroupDev*, int, int, int, const float*, PairFft, int, int,
                             const float2*);

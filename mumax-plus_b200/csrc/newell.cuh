@@ -4,11 +4,16 @@
 // 27-point weighted combination of the indefinite integrals, evaluated in
 // double precision exactly as physics/newell.cu:7-139 does, and summed over the
 // PBC images (2r+1 per periodic axis) as physics/strayfieldkernel.cu:25-56 does
-// -- here the image sum is also FP64.  It is evaluated once per octant point
-// |r| (the tensor is even in every axis for xx/yy/zz and odd in the axes its
-// off-diagonal indices name), expanded to the circular padded grid, transformed
-// with an FP64 radix-2 FFT, and the real, symmetry-reduced spectrum
-// (kx in [0,Px/2], ky in [0,Py/2], kz in [0,Pz/2]) is stored in FP32 with the
+// -- here the image sum is also FP64.  The integrals of the 27 points are shared:
+// they are evaluated once per lattice point (k_newell_lattice; neighbouring
+// displacements and periodic images meet the same points) and combined per
+// displacement in the order of the direct sum (k_newell_from_lattice).  It is
+// evaluated once per octant point |r| (the tensor is even in every axis for
+// xx/yy/zz and odd in the axes its off-diagonal indices name).  The spectrum of
+// such a tensor is real, and each axis is a cosine or sine transform of the
+// octant values alone: three passes (k_kernel_axis) of FP64 transforms in shared
+// memory take the octant table to the symmetry-reduced spectrum
+// (kx in [0,Px/2], ky in [0,Py/2], kz in [0,Pz/2]), stored in FP32 with the
 // convolution prefactor -mu0/(Px Py Pz) folded in.
 #pragma once
 #include <cuda_runtime.h>
@@ -85,31 +90,12 @@ struct KernelGeom {
   double cs[3];  // cell size
 };
 
-// Octant values N_c(|rx|, |ry|, |rz|) for |r_a| < n_a, all 6 components, FP64.
-// out layout: [c][rz][ry][rx]
-static __global__ void k_newell_octant(double* __restrict__ out, KernelGeom g) {
-  const long long total = (long long)g.n[0] * g.n[1] * g.n[2];
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int rx = (int)(t % g.n[0]);
-    const int ry = (int)((t / g.n[0]) % g.n[1]);
-    const int rz = (int)(t / ((long long)g.n[0] * g.n[1]));
-    double v[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = -g.pbc[0]; i <= g.pbc[0]; ++i)
-      for (int j = -g.pbc[1]; j <= g.pbc[1]; ++j)
-        for (int k = -g.pbc[2]; k <= g.pbc[2]; ++k) {
-          const int x = rx + i * g.mg[0], y = ry + j * g.mg[1], z = rz + k * g.mg[2];
-#pragma unroll 1
-          for (int c = 0; c < 6; ++c) v[c] += newell_comp(c, x, y, z, g.cs[0], g.cs[1], g.cs[2]);
-        }
-    for (int c = 0; c < 6; ++c) out[c * total + t] = v[c];
-  }
-}
-
-// Reference-layout real-space kernel (physics/strayfieldkernel.cu:80-99):
-// grid K with origin O (cells), 6 comps, cast to float.
-static __global__ void k_newell_reflayout(float* __restrict__ out, KernelGeom g, int K0, int K1, int K2, int O0, int O1,
-                                   int O2) {
+// Table of N_c at the displacements O + j, j < K per axis (layout [c][z][y][x]),
+// each with its images, evaluated point by point: for geometries whose lattice
+// (below) would take more memory than the transforms of the kernel do.
+template <typename T>
+__global__ void k_newell_direct(T* __restrict__ out, KernelGeom g, int K0, int K1, int K2, int O0, int O1, int O2,
+                                int ncomp) {
   const long long total = (long long)K0 * K1 * K2;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -121,9 +107,89 @@ static __global__ void k_newell_reflayout(float* __restrict__ out, KernelGeom g,
       for (int j = -g.pbc[1]; j <= g.pbc[1]; ++j)
         for (int k = -g.pbc[2]; k <= g.pbc[2]; ++k)
 #pragma unroll 1
-          for (int c = 0; c < 6; ++c)
+          for (int c = 0; c < ncomp; ++c)
             v[c] += newell_comp(c, x0 + i * g.mg[0], y0 + j * g.mg[1], z0 + k * g.mg[2], g.cs[0], g.cs[1], g.cs[2]);
-    for (int c = 0; c < 6; ++c) out[c * total + t] = (float)v[c];
+    for (int c = 0; c < ncomp; ++c) out[c * total + t] = (T)v[c];
+  }
+}
+
+// The lattice points |q| = a0 + p, p < len per axis (q in cells), that a table of
+// displacements meets: every displacement, image included, and its neighbours.
+struct NewellLattice {
+  int a0[3], len[3];
+};
+
+// Axes (u, v, w) of the arguments of component c (newell_comp's permutations).
+__device__ __forceinline__ void newell_axes(int c, int& u, int& v, int& w) {
+  u = c == 0 || c == 3 || c == 4 ? 0 : c == 2 ? 2 : 1;
+  v = c == 0 || c == 3 ? 1 : c == 2 ? 0 : 2;
+  w = 3 - u - v;
+}
+
+// Indefinite integrals of components c0 .. c0 + nc - 1 at every lattice point
+// (layout [c - c0][z][y][x]).  FP64 arithmetic bounds it (3 to 5 transcendental
+// functions per value); sharing the values takes 27 evaluations per displacement
+// and component to about one.
+static __global__ void k_newell_lattice(double* __restrict__ lat, KernelGeom g, NewellLattice L, int c0, int nc) {
+  const long long total = (long long)L.len[0] * L.len[1] * L.len[2];
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total * nc;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int c = c0 + (int)(t / total);
+    const long long e = t % total;
+    const int q[3] = {L.a0[0] + (int)(e % L.len[0]), L.a0[1] + (int)((e / L.len[0]) % L.len[1]),
+                      L.a0[2] + (int)(e / ((long long)L.len[0] * L.len[1]))};
+    int u, v, w;
+    newell_axes(c, u, v, w);
+    const int qu = u == 0 ? q[0] : u == 1 ? q[1] : q[2], qv = v == 0 ? q[0] : v == 1 ? q[1] : q[2];
+    const int qw = w == 0 ? q[0] : w == 1 ? q[1] : q[2];
+    lat[t] = c < 3 ? nxx_indef(qu, qv, qw, g.cs[u], g.cs[v], g.cs[w]) : nxy_indef(qu, qv, qw, g.cs[u], g.cs[v], g.cs[w]);
+  }
+}
+
+// k_newell_direct's table of components c0 .. c0 + nc - 1 from the lattice.  The
+// integrals of the diagonal components are even in every argument, those of the
+// off-diagonal ones odd in the first two; the 27 terms and the images are added
+// in the order of the direct sum.
+template <typename T>
+__global__ void k_newell_from_lattice(T* __restrict__ out, const double* __restrict__ lat, KernelGeom g,
+                                      NewellLattice L, int c0, int nc, int K0, int K1, int K2, int O0, int O1, int O2) {
+  const long long total = (long long)K0 * K1 * K2, ltot = (long long)L.len[0] * L.len[1] * L.len[2];
+  const long long ls[3] = {1, L.len[0], (long long)L.len[0] * L.len[1]};
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total * nc;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int c = c0 + (int)(t / total);
+    const long long e = t % total;
+    const int d[3] = {O0 + (int)(e % K0), O1 + (int)((e / K0) % K1), O2 + (int)(e / ((long long)K0 * K1))};
+    int u, v, w;
+    newell_axes(c, u, v, w);
+    const double norm = 4 * M_PI * g.cs[u] * g.cs[v] * g.cs[w];
+    const double* __restrict__ F = lat + (c - c0) * ltot;
+    double sum = 0;
+    for (int i = -g.pbc[0]; i <= g.pbc[0]; ++i)
+      for (int j = -g.pbc[1]; j <= g.pbc[1]; ++j)
+        for (int k = -g.pbc[2]; k <= g.pbc[2]; ++k) {
+          const int q[3] = {d[0] + i * g.mg[0], d[1] + j * g.mg[1], d[2] + k * g.mg[2]};
+          const int qu = u == 0 ? q[0] : u == 1 ? q[1] : q[2], qv = v == 0 ? q[0] : v == 1 ? q[1] : q[2];
+          const int qw = w == 0 ? q[0] : w == 1 ? q[1] : q[2];
+          double r = 0;
+          if (c < 3 || (qu != 0 && qv != 0)) {
+            const long long su = ls[u], sv = ls[v], sw = ls[w];
+#pragma unroll
+            for (int du = -1; du <= 1; ++du)
+#pragma unroll
+              for (int dv = -1; dv <= 1; ++dv)
+#pragma unroll
+                for (int dw = -1; dw <= 1; ++dw) {
+                  double f = F[su * (abs(qu + du) - L.a0[u]) + sv * (abs(qv + dv) - L.a0[v]) +
+                               sw * (abs(qw + dw) - L.a0[w])];
+                  if (c >= 3 && ((qu + du < 0) != (qv + dv < 0))) f = -f;
+                  r += newell_w(du, dv, dw) * f;
+                }
+            r /= norm;
+          }
+          sum += r;
+        }
+    out[c * total + e] = (T)sum;
   }
 }
 
@@ -152,71 +218,114 @@ static __global__ void k_newell_expand_abs(float* __restrict__ out, const float*
   }
 }
 
-// Expand component c of the octant table to the circular P-grid (imag = 0).
-// Parity: xy odd in x,y; xz odd in x,z; yz odd in y,z; diagonal even.
-static __global__ void k_kernel_expand(double2* __restrict__ full, const double* __restrict__ oct, int c, KernelGeom g,
-                                int P0, int P1, int P2) {
-  const long long total = (long long)P0 * P1 * P2;
-  const long long noct = (long long)g.n[0] * g.n[1] * g.n[2];
-  const int oddx = (c == 3 || c == 4), oddy = (c == 3 || c == 5), oddz = (c == 4 || c == 5);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % P0), j = (int)((t / P0) % P1), k = (int)(t / ((long long)P0 * P1));
-    auto circ = [](int q, int P, int n) { return q <= n - 1 ? q : (q >= P - (n - 1) ? q - P : INT_MIN); };
-    const int rx = circ(i, P0, g.n[0]), ry = circ(j, P1, g.n[1]), rz = circ(k, P2, g.n[2]);
-    double v = 0.0;
-    if (rx != INT_MIN && ry != INT_MIN && rz != INT_MIN) {
-      const int ax = abs(rx), ay = abs(ry), az = abs(rz);
-      v = oct[c * noct + ((long long)az * g.n[1] + ay) * g.n[0] + ax];
-      if (oddx && rx < 0) v = -v;
-      if (oddy && ry < 0) v = -v;
-      if (oddz && rz < 0) v = -v;
+// One axis of the kernel transform.  A line of n octant values f_j (j = 0 .. n-1)
+// stands for the circular sequence of length P with x[j] = f_j, x[P - j] = +-f_j
+// (even or odd component); its transform is real, f_0 + 2 sum f_j cos(2 pi j k/P),
+// or -i times the real 2 sum f_j sin(2 pi j k/P).  Two lines share one complex
+// FFT.  `inner` lines lie si apart, (o1, o2) groups of them further; elements of a
+// line lie sj apart.  Output k in [0, P/2] likewise.
+struct KernelAxis {
+  int n, P, inner, n2;                 // n2: number of o2 groups
+  long long sj, si, so1, so2;          // input strides
+  long long tk, ti, to1, to2;          // output strides
+  unsigned odd;                        // bit c: component c (o1) is odd along this axis
+  double scale[6];                     // factor per component
+};
+
+// Stockham pass of radix R over `nl` complex lines of length P (line l at l*P),
+// from a to b; tw[m] = exp(-2 pi i m / P).
+template <int R>
+__device__ __forceinline__ void fft64_pass(const double2* a, double2* b, int nl, int P, int Ns, const double2* tw) {
+  const int NB = P / R, total = nl * NB, step = P / (Ns * R);
+  for (int t = threadIdx.x; t < total; t += blockDim.x) {
+    const int l = t / NB, j = t - l * NB, k = j % Ns;
+    double2 x[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const double2 v = a[l * P + j + r * NB], w = tw[r * k * step];
+      x[r] = r == 0 ? v : make_double2(v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x);
     }
-    full[t] = make_double2(v, 0.0);
+    double2* o = b + l * P + (j - k) * R + k;
+    if constexpr (R == 2) {
+      o[0] = make_double2(x[0].x + x[1].x, x[0].y + x[1].y);
+      o[Ns] = make_double2(x[0].x - x[1].x, x[0].y - x[1].y);
+    } else {
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        double2 y = x[0];
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+          const double2 w = tw[((q * r) % R) * NB];
+          y.x += x[r].x * w.x - x[r].y * w.y;
+          y.y += x[r].x * w.y + x[r].y * w.x;
+        }
+        o[q * Ns] = y;
+      }
+    }
   }
+  __syncthreads();
 }
 
-// One radix-2 Stockham pass (FP64) along `axis` of a P0 x P1 x P2 array.
-// Consecutive threads take consecutive butterflies of a line along x and
-// consecutive lines (adjacent x) along y and z, so that every load and store
-// of a warp is contiguous.
-static __global__ void k_fft64_pass(const double2* __restrict__ in, double2* __restrict__ out, int P0, int P1, int P2,
-                             int axis, int Ns) {
-  const int L = axis == 0 ? P0 : axis == 1 ? P1 : P2;
-  const long long stride = axis == 0 ? 1 : axis == 1 ? P0 : (long long)P0 * P1;
-  const long long nlines = (long long)P0 * P1 * P2 / L;
-  const long long total = nlines * (L / 2);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int j = axis == 0 ? (int)(t % (L / 2)) : (int)(t / nlines);
-    const long long line = axis == 0 ? t / (L / 2) : t % nlines;
-    long long base;
-    if (axis == 0) base = line * P0;
-    else if (axis == 1) base = (line / P0) * ((long long)P0 * P1) + (line % P0);
-    else base = line;
-    const int k = j & (Ns - 1);
-    const double2 a = in[base + j * stride];
-    double2 b = in[base + (j + L / 2) * stride];
+// Blocks of TL complex lines (2 TL real ones); dynamic shared memory
+// (2 TL + 1) P double2.  Grid: o1 * n2 * ceil(inner / (2 TL)).  Bound by shared
+// memory (log2 P passes over 16-byte values); the transforms touch the octant's
+// lines only, about an eighth of the padded grid, in 3 launches for all components.
+template <typename TO>
+__global__ void __launch_bounds__(256) k_kernel_axis(const double* __restrict__ in, TO* __restrict__ out, KernelAxis A,
+                                                     int TL) {
+  extern __shared__ double2 sd[];
+  const int P = A.P, nt = (A.inner + 2 * TL - 1) / (2 * TL);
+  const int tile = blockIdx.x % nt, o2 = (blockIdx.x / nt) % A.n2, o1 = blockIdx.x / (nt * A.n2);
+  const int i0 = tile * 2 * TL, ni = min(2 * TL, A.inner - i0);
+  const bool odd = (A.odd >> o1) & 1;
+  double2 *a = sd, *b = sd + TL * P, *tw = sd + 2 * TL * P;
+  double* ar = reinterpret_cast<double*>(a);
+  for (int t = threadIdx.x; t < P; t += blockDim.x) {
     double s, c;
-    sincospi(-(double)k / Ns, &s, &c);
-    b = make_double2(b.x * c - b.y * s, b.x * s + b.y * c);
-    const int o = (j - k) * 2 + k;
-    out[base + o * stride] = make_double2(a.x + b.x, a.y + b.y);
-    out[base + (o + Ns) * stride] = make_double2(a.x - b.x, a.y - b.y);
+    sincospi(-2.0 * t / P, &s, &c);
+    tw[t] = make_double2(c, s);
   }
-}
-
-// Store the real, symmetry-reduced spectrum of component c (slot kc of kcomp)
-// in the layout read by k_yz: [kx][kz'][kcomp][ky'].
-static __global__ void k_kernel_extract(float* __restrict__ kspec, const double2* __restrict__ full, int kc, int kcomp,
-                                 int P0, int P1, int P2, double pref) {
-  const int Fh = P0 / 2 + 1, hy = P1 / 2 + 1, hz = P2 / 2 + 1;
-  const long long total = (long long)Fh * hy * hz;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int ky = (int)(t % hy), kz = (int)((t / hy) % hz), kx = (int)(t / ((long long)hy * hz));
-    const double v = full[kx + (long long)P0 * (ky + (long long)P1 * kz)].x;
-    kspec[(((long long)kx * hz + kz) * kcomp + kc) * hy + ky] = (float)(pref * v);
+  for (int t = threadIdx.x; t < TL * P; t += blockDim.x) a[t] = make_double2(0, 0);
+  __syncthreads();
+  const double* src = in + o1 * A.so1 + o2 * A.so2 + i0 * A.si;
+  for (int t = threadIdx.x; t < ni * A.n; t += blockDim.x) {  // consecutive threads along the unit stride
+    const int i = A.sj == 1 ? t / A.n : t % ni, j = A.sj == 1 ? t % A.n : t / ni;
+    const double v = src[j * A.sj + i * A.si];
+    double* line = ar + 2 * (i >> 1) * P + (i & 1);  // real part: even lines, imaginary: odd lines
+    if (j == 0) {
+      line[0] = odd ? 0.0 : v;
+    } else {
+      line[2 * j] = v;
+      line[2 * (P - j)] = odd ? -v : v;
+    }
+  }
+  __syncthreads();
+  int Ns = 1, rest = P;
+  while (rest % 3 == 0) {
+    fft64_pass<3>(a, b, TL, P, Ns, tw);
+    double2* x = a;
+    a = b;
+    b = x;
+    Ns *= 3;
+    rest /= 3;
+  }
+  while (rest > 1) {
+    fft64_pass<2>(a, b, TL, P, Ns, tw);
+    double2* x = a;
+    a = b;
+    b = x;
+    Ns *= 2;
+    rest /= 2;
+  }
+  const int H = P / 2 + 1;
+  TO* dst = out + o1 * A.to1 + o2 * A.to2 + i0 * A.ti;
+  const double sc = A.scale[o1];
+  for (int t = threadIdx.x; t < ni * H; t += blockDim.x) {
+    const int i = A.tk == 1 ? t / H : t % ni, k = A.tk == 1 ? t % H : t / ni;
+    const double2 X = a[(i >> 1) * P + k];
+    // even: X = A + i B; odd: X = -i A + B of the two real transforms A, B
+    const double v = odd ? ((i & 1) ? X.x : -X.y) : ((i & 1) ? X.y : X.x);
+    dst[k * A.tk + i * A.ti] = (TO)(sc * v);
   }
 }
 

@@ -5,7 +5,7 @@
 //
 // The Newell tensor is tabulated at the displacements O + j, j in [0, K) with
 // K = n_A + n_B - 1 and O = o_B - o_A - (n_A - 1) per axis (periodic images
-// included, k_newell_reflayout), and convolved with Ms m of A by FFTs of
+// included, FP64), and convolved with Ms m of A by FFTs of
 // power-of-two lengths P >= K.  With A zero-padded to P the circular sum at
 // n = i + n_A - 1 never wraps (n - i' runs over [i, i + n_A - 1], inside
 // [0, K)), so destination cell i reads the output at the window w = n_A - 1.

@@ -48,16 +48,23 @@ static __global__ void k_reduce_partial(const float* __restrict__ a, int N, int 
     for (int c = 0; c < 3; ++c) partial[blockIdx.x * 3 + c] = sh[c][0];
 }
 
-static __global__ void k_reduce_final(const double* __restrict__ partial, int nblocks, int op, double* out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double r[3] = {0, 0, 0};
-  for (int b = 0; b < nblocks; ++b)
-    for (int c = 0; c < 3; ++c) {
-      const double v = partial[b * 3 + c];
-      if (op != 1) r[c] += v;
-      else if (v > r[c] || v != v) r[c] = v;
-    }
-  for (int c = 0; c < 3; ++c) out[c] = r[c];
+// The block partials are added in block order by one thread per component;
+// staging them in shared memory first takes the serial chain from a global load
+// per term (27 us for 256 blocks) to an FP64 add per term.
+constexpr int REDUCE_MAX_BLOCKS = 256;
+static __global__ void __launch_bounds__(256) k_reduce_final(const double* __restrict__ partial, int nblocks, int op,
+                                                             double* out) {
+  __shared__ double sp[3 * REDUCE_MAX_BLOCKS];
+  for (int i = threadIdx.x; i < 3 * nblocks; i += blockDim.x) sp[i] = partial[i];
+  __syncthreads();
+  if (threadIdx.x >= 3) return;
+  double r = 0;
+  for (int b = 0; b < nblocks; ++b) {
+    const double v = sp[b * 3 + threadIdx.x];
+    if (op != 1) r += v;
+    else if (v > r || v != v) r = v;
+  }
+  out[threadIdx.x] = r;
 }
 
 // Sampled run: <m> of one magnet into the due rows of its group's table, with
@@ -90,16 +97,20 @@ static __global__ void __launch_bounds__(256) k_sample_partial(const MagnetDev* 
     for (int c = 0; c < 3; ++c) partial[blockIdx.x * 3 + c] = sh[c][0];
 }
 
-static __global__ void k_sample_final(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, int slot,
-                               const double* __restrict__ partial, int nblocks, long long ngeo, int col) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+static __global__ void __launch_bounds__(256) k_sample_final(const MagnetDev* __restrict__ mags,
+                                                             const GroupDev* __restrict__ groups, int slot,
+                                                             const double* __restrict__ partial, int nblocks,
+                                                             long long ngeo, int col) {
+  __shared__ double sp[3 * REDUCE_MAX_BLOCKS];
   const GroupDev& G = groups[mags[slot].group];
   if (G.samp_hi <= G.samp_lo) return;
-  double r[3] = {0, 0, 0};
-  for (int b = 0; b < nblocks; ++b)
-    for (int c = 0; c < 3; ++c) r[c] += partial[b * 3 + c];
+  for (int i = threadIdx.x; i < 3 * nblocks; i += blockDim.x) sp[i] = partial[i];
+  __syncthreads();
+  if (threadIdx.x >= 3) return;
+  double r = 0;
+  for (int b = 0; b < nblocks; ++b) r += sp[b * 3 + threadIdx.x];
   for (int row = G.samp_lo; row < G.samp_hi; ++row)
-    for (int c = 0; c < 3; ++c) G.samp_out[(size_t)row * G.samp_row + col + c] = ngeo > 0 ? r[c] / ngeo : 0.0;
+    G.samp_out[(size_t)row * G.samp_row + col + threadIdx.x] = ngeo > 0 ? r / ngeo : 0.0;
 }
 
 // Set m: normalise per cell inside the geometry (core/variable.cpp:76-87).
@@ -193,15 +204,19 @@ static __global__ void k_min_partial(const float* __restrict__ m0, const float* 
     for (int k = 0; k < 4; ++k) partial[blockIdx.x * 4 + k] = sh[k][0];
 }
 
-static __global__ void k_min_final(const double* __restrict__ partial, int nblocks, double* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double r[4] = {0, 0, 0, 0};
+static __global__ void __launch_bounds__(256) k_min_final(const double* __restrict__ partial, int nblocks,
+                                                          double* __restrict__ out) {
+  __shared__ double sp[4 * REDUCE_MAX_BLOCKS];
+  for (int i = threadIdx.x; i < 4 * nblocks; i += blockDim.x) sp[i] = partial[i];
+  __syncthreads();
+  if (threadIdx.x >= 4) return;
+  double r = 0;
   for (int b = 0; b < nblocks; ++b) {
-    for (int k = 0; k < 3; ++k) r[k] += partial[b * 4 + k];
-    const double v = partial[b * 4 + 3];
-    if (v > r[3] || v != v) r[3] = v;
+    const double v = sp[b * 4 + threadIdx.x];
+    if (threadIdx.x < 3) r += v;
+    else if (v > r || v != v) r = v;
   }
-  for (int k = 0; k < 4; ++k) out[k] = r[k];
+  out[threadIdx.x] = r;
 }
 
 }  // namespace mpx

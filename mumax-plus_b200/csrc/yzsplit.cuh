@@ -15,7 +15,7 @@
 // Same arithmetic as k_yz (the same FFT passes, the same kernel spectrum
 // lookup); the spectrum makes two extra round trips through global memory.
 #pragma once
-#include "kernels.cuh"
+#include "launch.h"
 
 namespace mpx {
 
@@ -144,6 +144,173 @@ __global__ void __launch_bounds__(384, MAXLR == 3 ? 2 : 1)
     const int c = rest % 3, z = rest / 3;
     if (span_ok(((size_t)c * nz + z) * Py + ky0 + kyl, tleft))
       Tw[((size_t)c * nz + z) * Py + ky0 + kyl] = D[(c * nky + kyl) * cs + pidx(z)];
+  }
+}
+
+// --------------------------------------------------- warp columns (k_ycw, k_zcw)
+// The three passes for y lengths 64 .. 1024 and z lengths 32 .. 256 in the
+// four-step warp transforms of fft.cuh: a warp loads its columns straight from
+// global memory, transposes once through its own shared memory and stores
+// straight back, without a block barrier.  On 80 x 80 x 40 cells (padded 256 x
+// 256 x 128) the block-wide passes above are bound by their barriers and
+// shared-memory round trips (36 - 44 % issue active, 70.6 M warp instructions
+// for k_zmul).
+
+template <int Q, int DIR>
+__device__ __forceinline__ void ycw_body(const MagnetDev& M, int col0, int ncol, float2* sm, const float2* twq) {
+  constexpr int W = 32 / Q, Py = 32 * Q, cs = qlen(Py);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ny = M.n[1], first = warp * W;
+  if (first >= ncol) return;
+  const int nc = min(W, ncol - first);
+  const size_t c0 = (size_t)col0 + first, ncols_all = (size_t)M.Fh * 3 * M.n[2];
+  float2* __restrict__ S = M.spec + c0 * ny;
+  float2* __restrict__ T = M.tspec + c0 * Py;
+  const size_t sleft = (ncols_all - c0) * ny, tleft = (ncols_all - c0) * Py;  // checked build
+  float2* C = sm + warp * W * cs;
+  float2 v[32];
+#pragma unroll
+  for (int c = 0; c < W; ++c)
+#pragma unroll
+    for (int r = 0; r < Q; ++r) {
+      const int y = lane + 32 * r;
+      if constexpr (DIR < 0)  // S: ny rows, zero padding above (y < Py / 2 only)
+        v[c * Q + r] = (c < nc && r < Q / 2 && y < ny && span_ok((size_t)c * ny + y, sleft)) ? S[(size_t)c * ny + y]
+                                                                                              : make_float2(0.f, 0.f);
+      else
+        v[c * Q + r] = (c < nc && span_ok((size_t)c * Py + y, tleft)) ? T[(size_t)c * Py + y] : make_float2(0.f, 0.f);
+    }
+  four_step_inner<Q, DIR, (DIR < 0)>(v, twq, lane);
+  four_step_outer<Q, DIR, (DIR > 0)>(v, C, cs, nc, lane);
+  const int lc = lane / Q, ls = lane % Q;
+  if (lc >= nc) return;
+#pragma unroll
+  for (int t = 0; t < (DIR > 0 ? 16 : 32); ++t) {  // element s + Q t of column c
+    const int y = ls + Q * t;
+    if constexpr (DIR < 0) {
+      if (span_ok((size_t)lc * Py + y, tleft)) T[(size_t)lc * Py + y] = v[t];
+    } else {
+      if (y < ny && span_ok((size_t)lc * ny + y, sleft)) S[(size_t)lc * ny + y] = v[t];
+    }
+  }
+}
+
+// Work item as k_ycols (at most ycw_cols(Py) columns).
+template <int DIR>
+__global__ void __launch_bounds__(YCW_THREADS, 2)
+    k_ycw(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, const Work* __restrict__ work,
+          int stage, int gate, const float2* __restrict__ tw) {
+  extern __shared__ float2 sm[];
+  __shared__ MagnetDev M;
+  __shared__ GroupDev G;
+  pdl_trigger();
+  const Work wk = work[blockIdx.x];
+  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) {
+    pdl_wait();
+    return;
+  }
+  const int logPy = M.logP[1];
+  float2* twq = sm + (YCW_THREADS / 32) * (1024 >> logPy) * qlen(1 << logPy);
+  load_twq(twq, tw, logPy);
+  __syncthreads();
+  pdl_wait();  // the columns are written by the previous pass
+  switch (logPy) {
+    case 6: ycw_body<2, DIR>(M, wk.z, wk.y0, sm, twq); break;
+    case 7: ycw_body<4, DIR>(M, wk.z, wk.y0, sm, twq); break;
+    case 8: ycw_body<8, DIR>(M, wk.z, wk.y0, sm, twq); break;
+    case 9: ycw_body<16, DIR>(M, wk.z, wk.y0, sm, twq); break;
+    default: ycw_body<32, DIR>(M, wk.z, wk.y0, sm, twq); break;
+  }
+}
+
+// z stage: a unit is the W = 32 / Q = 1024 / Pz consecutive ky of one kx, taken by
+// three warps (one per component, W columns of length Pz = 32 Q); they meet in
+// shared memory for the 3x3 multiply (a 96-thread barrier per unit).
+__device__ __forceinline__ void unit_sync(int unit) { asm volatile("bar.sync %0, 96;" ::"r"(1 + unit) : "memory"); }
+
+template <int Q>
+__device__ __forceinline__ void zcw_body(const MagnetDev& M, int kx, int ky00, int nky, float2* sm,
+                                         const float2* twq) {
+  constexpr int W = 32 / Q, Pz = 32 * Q, cs = qlen(Pz);
+  const int lane = threadIdx.x & 31, unit = threadIdx.x / 96, ut = threadIdx.x - 96 * unit, comp = ut >> 5;
+  if (unit * W >= nky) return;
+  const int nz = M.n[2], Py = M.P[1], ky0 = ky00 + unit * W;
+  const size_t t0 = ((size_t)kx * 3 + comp) * nz * Py + ky0;
+  const size_t tleft = (size_t)M.Fh * 3 * nz * Py - t0;  // checked build
+  float2* __restrict__ T = M.tspec + t0;
+  float2* D = sm + unit * 3 * W * cs;  // [comp][ky] columns
+  float2* C = D + comp * W * cs;
+  float2 v[32];
+#pragma unroll
+  for (int r = 0; r < Q; ++r) {  // z = lane + 32 r: W consecutive ky each, 16-byte loads
+    const int z = lane + 32 * r;
+    const bool in = (2 * r < Q || Q == 1) && z < nz;
+#pragma unroll
+    for (int c = 0; c < W; c += 2) {
+      const size_t ti = (size_t)z * Py + c;
+      const float4 w = (in && span_ok(ti + 1, tleft)) ? *reinterpret_cast<const float4*>(T + ti)
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[c * Q + r] = make_float2(w.x, w.y);
+      v[(c + 1) * Q + r] = make_float2(w.z, w.w);
+    }
+  }
+  const int lc = lane / Q, ls = lane % Q;
+  four_step_inner<Q, -1, true>(v, twq, lane);
+  four_step_outer<Q, -1, false>(v, C, cs, W, lane);
+#pragma unroll
+  for (int t = 0; t < 32; ++t) C[lc * cs + qidx(ls + Q * t)] = v[t];  // kz = s + Q t
+  unit_sync(unit);
+  const int hy = Py / 2 + 1, kc = M.kcomp;
+  const size_t kn = (size_t)(Pz / 2 + 1) * kc * hy;
+  const float* __restrict__ Kx = M.kspec + kx * kn;
+  for (int t = ut; t < W * Pz; t += 96) {
+    const int kyl = t % W, kz = t / W, ky = ky0 + kyl;
+    const int kyp = min(ky, Py - ky);
+    const float sy = (ky > Py / 2) ? -1.f : 1.f;
+    float kxx, kyy, kzz, kxy, kxz, kyz;
+    kernel_at<Pz>(Kx, kc, hy, kyp, sy, kz, kxx, kyy, kzz, kxy, kxz, kyz, (M.Fh - kx) * kn);
+    float2* p = D + kyl * cs + qidx(kz);
+    apply3(p, p + W * cs, p + 2 * W * cs, kxx, kyy, kzz, kxy, kxz, kyz);
+  }
+  unit_sync(unit);
+#pragma unroll
+  for (int c = 0; c < W; ++c)
+#pragma unroll
+    for (int r = 0; r < Q; ++r) v[c * Q + r] = C[c * cs + lane + 33 * r];
+  four_step_inner<Q, 1, false>(v, twq, lane);
+  __syncwarp();  // the columns were read by every lane
+  four_step_outer<Q, 1, true>(v, C, cs, W, lane);
+#pragma unroll
+  for (int t = 0; t < 16; ++t) {
+    const int z = ls + Q * t;
+    const size_t ti = (size_t)z * Py + lc;
+    if (z < nz && span_ok(ti, tleft)) T[ti] = v[t];
+  }
+}
+
+// Work item as k_zmul (at most zcw_kys(Pz) ky, a multiple of 1024 / Pz).
+static __global__ void __launch_bounds__(ZCW_THREADS, 2)
+    k_zcw(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, const Work* __restrict__ work,
+          int stage, int gate, const float2* __restrict__ tw) {
+  extern __shared__ float2 sm[];
+  __shared__ MagnetDev M;
+  __shared__ GroupDev G;
+  pdl_trigger();
+  const Work wk = work[blockIdx.x];
+  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) {
+    pdl_wait();
+    return;
+  }
+  const int logPz = M.logP[2];
+  float2* twq = sm + ZCW_UNITS * 3 * (1024 >> logPz) * qlen(1 << logPz);
+  load_twq(twq, tw, logPz);
+  __syncthreads();
+  pdl_wait();  // T is written by k_ycw<-1>
+  switch (logPz) {
+    case 5: zcw_body<1>(M, wk.z, wk.y0, wk.ty, sm, twq); break;
+    case 6: zcw_body<2>(M, wk.z, wk.y0, wk.ty, sm, twq); break;
+    case 7: zcw_body<4>(M, wk.z, wk.y0, wk.ty, sm, twq); break;
+    default: zcw_body<8>(M, wk.z, wk.y0, wk.ty, sm, twq); break;
   }
 }
 
