@@ -161,7 +161,8 @@ struct Magnet {
   int nkx = 1;   // consecutive kx per y/z block
   int ty_def = 4, nkx_def = 1;  // the shapes for a magnet launched with many others
   bool split = false;        // y/z in three passes (k_ycols, k_zmul, k_ycols)
-  int ncy = 1, nkz = 1;      // columns per k_ycols block, ky per k_zmul block
+  bool wsplit = false;       // ... in their warp-column forms (k_ycw, k_zcw, k_ycw)
+  int ncy = 1, nkz = 1;      // columns per y block, ky per z block of the split path
   float2* tspec = nullptr;
   int64_t tspec_bytes = 0;
   std::vector<Work> ycw, zmw;            // k_ycols / k_zmul work items
@@ -256,6 +257,18 @@ struct PairPlan {
   int launches() const { return s_yz > 0 ? 3 : 5; }
 };
 
+// Launch of the split y/z path over one magnet or all started ones: block-wide
+// y columns, z stages (both block-wide and tensor-core y), tensor-core y tiles,
+// and the warp-column forms; dynamic shared memory and largest lengths.
+struct SplitLaunch {
+  const Work *yc = nullptr, *zm = nullptr, *tc = nullptr, *yw = nullptr, *zw = nullptr;
+  int nyc = 0, nzm = 0, ntc = 0, nyw = 0, nzw = 0;
+  int smem_y = 0, smem_z = 0, max_py = 0, max_pz = 0, smem_yw = 0, smem_zw = 0;
+  int launches() const {
+    return (nyc > 0 ? 2 : 0) + (ntc > 0 ? 2 : 0) + (nzm > 0 ? 1 : 0) + (nyw > 0 ? 3 : 0);
+  }
+};
+
 struct mpx_engine {
   int device = 0;
   cudaStream_t own = nullptr, stream = nullptr;
@@ -276,7 +289,7 @@ struct mpx_engine {
   size_t scratch_bytes = 0;
   // run tables over all magnets: x tiles (demag / local), y/z blocks per
   // class, split path (k_ycols, k_zmul, k_ydft_tc)
-  enum { TT_DEMAG = 0, TT_LOCAL, TT_YCOLS, TT_ZMUL, TT_TC, TT_YZ0 };
+  enum { TT_DEMAG = 0, TT_LOCAL, TT_YCOLS, TT_ZMUL, TT_TC, TT_YCW, TT_ZCW, TT_YZ0 };
   SlotTable tt[TT_YZ0 + YZ_CLASSES];
   uint64_t next_uid = 1;
   bool tables_dirty = true;
@@ -288,11 +301,7 @@ struct mpx_engine {
   Work* d_kx_demag[YZ_CLASSES] = {};
   int n_kx_demag[YZ_CLASSES] = {};
   int smem_yz[YZ_CLASSES] = {};
-  // split y/z path over all split magnets
-  Work *d_t_ycols = nullptr, *d_t_zmul = nullptr;
-  int n_t_ycols = 0, n_t_zmul = 0, smem_ycols = 0, smem_zmul = 0, maxpy_split = 0, maxpz_split = 0;
-  Work* d_t_tc = nullptr;  // k_ydft_tc items over all started tensor-core magnets
-  int n_t_tc = 0;
+  SplitLaunch split;  // split y/z path over all split magnets
   // y transforms of the demag convolution: MPX_DFT_FP32 (shared-memory FFT) or
   // MPX_DFT_TF32X3 (tcgen05 GEMMs, for y lengths 1024 and 2048); the DFT32
   // matrix (hi, lo) of the tensor-core form
@@ -560,47 +569,19 @@ int choose_nkx(int nz, int Py, int Pz, int Fh) {
   return std::max(1, std::min(Fh, pts / (3 * nz * Py)));
 }
 
+// Split path: the warp-column forms at the lengths their transforms cover.  At
+// 80 x 80 x 40 cells (Py 256, Pz 128) 18 Dormand-Prince attempts take 15.3 ms
+// with them and 28.4 ms with the block-wide passes; y lengths below 64 or above
+// 1024 and z lengths below 32 or above 256 keep the block-wide passes.
+bool split_warp(int Py, int Pz) { return Py >= 64 && Py <= 1024 && Pz >= 32 && Pz <= 256; }
+// Columns per y block and ky per z block of the split path.
+void split_shapes(int ncols, int Py, int Pz, bool warp, int* ncy, int* nkz) {
+  *ncy = std::max(1, std::min(ncols, warp ? ycw_cols(Py) : (YZ_VPT * YZ_THREADS) / Py));
+  *nkz = std::max(1, std::min(Py, warp ? zcw_kys(Pz) : (YZ_VPT * YZ_THREADS) / (3 * Pz)));
+}
+
 int ycols_smem(const Magnet* m) { return (m->ncy * plen(m->P[1]) + m->P[1]) * (int)sizeof(float2); }
 int zmul_smem(const Magnet* m) { return (3 * m->nkz * plen(m->P[2]) + m->P[2]) * (int)sizeof(float2); }
-
-// The three passes of the split y/z path (radix-8 forms when the lengths allow);
-// magnets with the tensor-core y transforms take k_ydft_tc (work list tcw)
-// instead of k_ycols.
-constexpr int TC_GRID_PER_SM = TC_BLOCKS_PER_SM;
-mpx_status launch_split(mpx_engine* e, const Work* ycw, int nyc, const Work* zmw, int nzm, int smem_y, int smem_z,
-                        int max_py, int max_pz, int stage, int gate, const Work* tcw = nullptr, int ntc = 0) {
-  if (nyc <= 0 && ntc <= 0) return MPX_OK;
-  const bool ry = max_py <= 2048, rz = max_pz <= 2048;
-  const int gtc = std::min(ntc, TC_GRID_PER_SM * e->n_sm);
-  if (ntc > 0) {
-    k_ydft_tc<-1><<<gtc, 128, TC_SMEM, e->stream>>>(e->d_mags, e->d_groups, tcw, ntc, stage, gate, e->d_dftB);
-    e->launches++;
-  }
-  if (nyc > 0) {
-    if (ry)
-      ycols_fn(-1, 3)<<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
-    else
-      ycols_fn(-1, 4)<<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
-    e->launches++;
-  }
-  if (rz)
-    zmul_fn(3)<<<nzm, YZ_THREADS, smem_z, e->stream>>>(e->d_mags, e->d_groups, zmw, stage, gate, e->d_tw);
-  else
-    zmul_fn(4)<<<nzm, YZ_THREADS, smem_z, e->stream>>>(e->d_mags, e->d_groups, zmw, stage, gate, e->d_tw);
-  e->launches++;
-  if (nyc > 0) {
-    if (ry)
-      ycols_fn(1, 3)<<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
-    else
-      ycols_fn(1, 4)<<<nyc, YZ_THREADS, smem_y, e->stream>>>(e->d_mags, e->d_groups, ycw, stage, gate, e->d_tw);
-    e->launches++;
-  }
-  if (ntc > 0) {
-    k_ydft_tc<1><<<gtc, 128, TC_SMEM, e->stream>>>(e->d_mags, e->d_groups, tcw, ntc, stage, gate, e->d_dftB);
-    e->launches++;
-  }
-  return MPX_OK;
-}
 
 // Launch with programmatic dependent launch allowed: the kernel may start its
 // prologue while the previous kernel of the stream finishes (the kernel calls
@@ -618,6 +599,58 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, int smem, 
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// The three passes of the split y/z path (radix-8 forms when the lengths allow);
+// magnets with the tensor-core y transforms take k_ydft_tc (work list tcw)
+// instead of k_ycols.
+constexpr int TC_GRID_PER_SM = TC_BLOCKS_PER_SM;
+mpx_status launch_split(mpx_engine* e, const SplitLaunch& L, int stage, int gate) {
+  const int gtc = std::min(L.ntc, TC_GRID_PER_SM * e->n_sm);
+  const YzFn y_fwd = ycols_fn(-1, L.max_py <= 2048 ? 3 : 4), y_inv = ycols_fn(1, L.max_py <= 2048 ? 3 : 4);
+  if (L.ntc > 0)
+    k_ydft_tc<-1><<<gtc, 128, TC_SMEM, e->stream>>>(e->d_mags, e->d_groups, L.tc, L.ntc, stage, gate, e->d_dftB);
+  if (L.nyc > 0) y_fwd<<<L.nyc, YZ_THREADS, L.smem_y, e->stream>>>(e->d_mags, e->d_groups, L.yc, stage, gate, e->d_tw);
+  if (L.nzm > 0)
+    zmul_fn(L.max_pz <= 2048 ? 3 : 4)<<<L.nzm, YZ_THREADS, L.smem_z, e->stream>>>(e->d_mags, e->d_groups, L.zm, stage,
+                                                                                 gate, e->d_tw);
+  if (L.nyc > 0) y_inv<<<L.nyc, YZ_THREADS, L.smem_y, e->stream>>>(e->d_mags, e->d_groups, L.yc, stage, gate, e->d_tw);
+  if (L.ntc > 0)
+    k_ydft_tc<1><<<gtc, 128, TC_SMEM, e->stream>>>(e->d_mags, e->d_groups, L.tc, L.ntc, stage, gate, e->d_dftB);
+  if (L.nyw > 0) {
+    CUDA_TRY(launch_pdl(ycw_fn(-1), L.nyw, YCW_THREADS, L.smem_yw, e->stream, e->d_mags, e->d_groups, L.yw, stage,
+                        gate, e->d_tw));
+    CUDA_TRY(launch_pdl(zcw_fn(), L.nzw, ZCW_THREADS, L.smem_zw, e->stream, e->d_mags, e->d_groups, L.zw, stage, gate,
+                        e->d_tw));
+    CUDA_TRY(launch_pdl(ycw_fn(1), L.nyw, YCW_THREADS, L.smem_yw, e->stream, e->d_mags, e->d_groups, L.yw, stage, gate,
+                        e->d_tw));
+  }
+  e->launches += L.launches();
+  return MPX_OK;
+}
+// The split path of one magnet.
+SplitLaunch split_of(const Magnet* m) {
+  SplitLaunch L;
+  if (m->wsplit) {
+    L.yw = m->d_ycw;
+    L.nyw = (int)m->ycw.size();
+    L.zw = m->d_zmw;
+    L.nzw = (int)m->zmw.size();
+    L.smem_yw = ycw_smem(m->P[1]);
+    L.smem_zw = zcw_smem(m->P[2]);
+    return L;
+  }
+  L.yc = m->d_ycw;
+  L.nyc = (int)m->ycw.size();
+  L.zm = m->d_zmw;
+  L.nzm = (int)m->zmw.size();
+  L.tc = m->d_tcw;
+  L.ntc = (int)m->tcw.size();
+  L.smem_y = ycols_smem(m);
+  L.smem_z = zmul_smem(m);
+  L.max_py = m->P[1];
+  L.max_pz = m->P[2];
+  return L;
 }
 
 // y/z launch for one class: warp columns for y lengths 64 .. 1024 (k_yzw);
@@ -731,7 +764,7 @@ mpx_status rebuild_tables(mpx_engine* e) {
   // (finished and idle solves cost no blocks), in slot order
   const int NT = mpx_engine::TT_YZ0 + YZ_CLASSES;
   std::vector<std::pair<Magnet*, const std::vector<Work>*>> want[mpx_engine::TT_YZ0 + YZ_CLASSES];
-  e->smem_ycols = e->smem_zmul = e->maxpy_split = e->maxpz_split = 0;
+  e->split = SplitLaunch();
   e->smem_x = 0;
   e->nt_x = 256;
   e->x_pair = false;
@@ -744,14 +777,19 @@ mpx_status rebuild_tables(mpx_engine* e) {
     if (m->demag) {
       want[mpx_engine::TT_DEMAG].push_back({m, &m->tiles});
       e->smem_x = std::max(e->smem_x, x_smem(m));
-      if (m->split) {
+      if (m->wsplit) {
+        want[mpx_engine::TT_YCW].push_back({m, &m->ycw});
+        want[mpx_engine::TT_ZCW].push_back({m, &m->zmw});
+        e->split.smem_yw = std::max(e->split.smem_yw, ycw_smem(m->P[1]));
+        e->split.smem_zw = std::max(e->split.smem_zw, zcw_smem(m->P[2]));
+      } else if (m->split) {
         want[mpx_engine::TT_YCOLS].push_back({m, &m->ycw});
         want[mpx_engine::TT_TC].push_back({m, &m->tcw});
         want[mpx_engine::TT_ZMUL].push_back({m, &m->zmw});
-        e->smem_ycols = std::max(e->smem_ycols, ycols_smem(m));
-        e->smem_zmul = std::max(e->smem_zmul, zmul_smem(m));
-        e->maxpy_split = std::max(e->maxpy_split, m->P[1]);
-        e->maxpz_split = std::max(e->maxpz_split, m->P[2]);
+        e->split.smem_y = std::max(e->split.smem_y, ycols_smem(m));
+        e->split.smem_z = std::max(e->split.smem_z, zmul_smem(m));
+        e->split.max_py = std::max(e->split.max_py, m->P[1]);
+        e->split.max_pz = std::max(e->split.max_pz, m->P[2]);
       } else {
         const int cls = yz_class(m);
         want[mpx_engine::TT_YZ0 + cls].push_back({m, &m->kxw});
@@ -829,12 +867,15 @@ mpx_status rebuild_tables(mpx_engine* e) {
   e->n_t_demag = (int)e->tt[mpx_engine::TT_DEMAG].items.size();
   e->d_t_local = e->tt[mpx_engine::TT_LOCAL].dev;
   e->n_t_local = (int)e->tt[mpx_engine::TT_LOCAL].items.size();
-  e->d_t_ycols = e->tt[mpx_engine::TT_YCOLS].dev;
-  e->n_t_ycols = (int)e->tt[mpx_engine::TT_YCOLS].items.size();
-  e->d_t_zmul = e->tt[mpx_engine::TT_ZMUL].dev;
-  e->n_t_zmul = (int)e->tt[mpx_engine::TT_ZMUL].items.size();
-  e->d_t_tc = e->tt[mpx_engine::TT_TC].dev;
-  e->n_t_tc = (int)e->tt[mpx_engine::TT_TC].items.size();
+  auto table = [&](int t, const Work** dev, int* n) {
+    *dev = e->tt[t].dev;
+    *n = (int)e->tt[t].items.size();
+  };
+  table(mpx_engine::TT_YCOLS, &e->split.yc, &e->split.nyc);
+  table(mpx_engine::TT_ZMUL, &e->split.zm, &e->split.nzm);
+  table(mpx_engine::TT_TC, &e->split.tc, &e->split.ntc);
+  table(mpx_engine::TT_YCW, &e->split.yw, &e->split.nyw);
+  table(mpx_engine::TT_ZCW, &e->split.zw, &e->split.nzw);
   for (int c = 0; c < YZ_CLASSES; ++c) {
     e->d_kx_demag[c] = e->tt[mpx_engine::TT_YZ0 + c].dev;
     e->n_kx_demag[c] = (int)e->tt[mpx_engine::TT_YZ0 + c].items.size();
@@ -846,8 +887,8 @@ mpx_status rebuild_tables(mpx_engine* e) {
   std::vector<long long> sig;
   for (int t = 0; t < NT; ++t) sig.insert(sig.end(), {(long long)(uintptr_t)e->tt[t].dev, (long long)e->tt[t].items.size()});
   for (int c = 0; c < YZ_CLASSES; ++c) sig.push_back(e->smem_yz[c]);
-  sig.insert(sig.end(), {e->smem_x, e->nt_x, e->x_pair ? 1 : 0, e->smem_ycols, e->smem_zmul, e->maxpy_split,
-                         e->maxpz_split});
+  sig.insert(sig.end(), {e->smem_x, e->nt_x, e->x_pair ? 1 : 0, e->split.smem_y, e->split.smem_z, e->split.max_py,
+                         e->split.max_pz, e->split.smem_yw, e->split.smem_zw});
   e->tables_dirty = false;
   if (e->tables_valid && sig == e->tables_sig) return MPX_OK;
   e->tables_sig = std::move(sig);
@@ -1540,7 +1581,7 @@ mpx_status setup_magnet(mpx_engine* e, Magnet* m, const mpx_magnet_desc* d, bool
   m->ty = m->ty_def;
   m->nkx = m->nkx_def;
   plan_shapes({m}, &m->ty, &m->nkx);  // alone (plain evaluations, single solves)
-  m->split = false;
+  m->split = m->wsplit = false;
   if (m->demag) {
     if (m->P[0] > X_VPT * X_THREADS_MAX || m->P[1] > std::min(MAX_FFT, YZ_VPT * YZ_THREADS))
       return fail(MPX_ERR_UNSUPPORTED, "demag: padded FFT length above 2048 along x or 4096 along y "
@@ -1551,9 +1592,12 @@ mpx_status setup_magnet(mpx_engine* e, Magnet* m, const mpx_magnet_desc* d, bool
     m->split = m->tc || m->P[2] > 16 || yz_smem(m) > SMEM_DYN_MAX;
     if (m->split) {
       if (m->P[2] > MAX_FFT) return fail(MPX_ERR_UNSUPPORTED, "demag: padded FFT length above 4096 along z");
-      m->ncy = std::max(1, std::min(D.Fh * 3 * D.n[2], (YZ_VPT * YZ_THREADS) / m->P[1]));
-      m->nkz = std::max(1, std::min(m->P[1], (YZ_VPT * YZ_THREADS) / (3 * m->P[2])));
-      if (ycols_smem(m) > SMEM_DYN_MAX || zmul_smem(m) > SMEM_DYN_MAX)
+      m->wsplit = !m->tc && split_warp(m->P[1], m->P[2]);
+      split_shapes(D.Fh * 3 * D.n[2], m->P[1], m->P[2], m->wsplit, &m->ncy, &m->nkz);
+      if (m->wsplit) {
+        if (ycw_smem(m->P[1]) > SMEM_DYN_MAX || zcw_smem(m->P[2]) > SMEM_DYN_MAX)
+          return fail(MPX_ERR_UNSUPPORTED, "demag: y/z transforms exceed shared memory");
+      } else if (ycols_smem(m) > SMEM_DYN_MAX || zmul_smem(m) > SMEM_DYN_MAX)
         return fail(MPX_ERR_UNSUPPORTED, "demag: y/z transforms exceed shared memory");
     }
     if (x_smem(m) > SMEM_DYN_MAX) return fail(MPX_ERR_UNSUPPORTED, "demag: x-pass tile exceeds shared memory");
@@ -1679,9 +1723,7 @@ mpx_status eval_into(mpx_engine* e, Magnet* m, int q, float* out) {
     xfwd_fn(false, x_pair_of(m))<<<ntile, nt, sx, e->stream>>>(e->d_mags, e->d_groups, m->d_tiles, 0, 0, nullptr,
                                                                 e->d_tw);
     if (m->split)
-      MPX_TRY(launch_split(e, m->d_ycw, (int)m->ycw.size(), m->d_zmw, (int)m->zmw.size(), ycols_smem(m),
-                           zmul_smem(m), m->P[1], m->P[2], 0, 0, m->d_tcw,
-                           (int)m->tcw.size()));
+      MPX_TRY(launch_split(e, split_of(m), 0, 0));
     else
       MPX_TRY(launch_yz(e, yz_class(m), m->d_kxw, (int)m->kxw.size(), syz, 0, 0));
     CUDA_TRY(launch_pdl(xinv_fn(x_pair_of(m)), ntile, nt, sx, e->stream, e->d_mags, e->d_groups, m->d_tiles, ea,
@@ -1730,8 +1772,7 @@ mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
     if (e->n_t_demag > 0) {
       for (int c = 0; c < YZ_CLASSES; ++c)
         MPX_TRY(launch_yz(e, c, e->d_kx_demag[c], e->n_kx_demag[c], e->smem_yz[c], s, 1));
-      MPX_TRY(launch_split(e, e->d_t_ycols, e->n_t_ycols, e->d_t_zmul, e->n_t_zmul, e->smem_ycols, e->smem_zmul,
-                           e->maxpy_split, e->maxpz_split, s, 1, e->d_t_tc, e->n_t_tc));
+      MPX_TRY(launch_split(e, e->split, s, 1));
       CUDA_TRY(launch_pdl(xinv_fn(e->x_pair), e->n_t_demag, e->nt_x, e->smem_x, e->stream, e->d_mags, e->d_groups,
                           e->d_t_demag, ea, e->d_tw));
       e->launches++;
@@ -1817,7 +1858,7 @@ int attempt_launches(const mpx_engine* e, const TableauDev& T, int first_stage) 
   const int S = T.S, ns = S - first_stage;
   int nyz = 0;
   for (int c = 0; c < YZ_CLASSES; ++c) nyz += e->n_kx_demag[c] > 0 ? 1 : 0;
-  if (e->n_t_ycols > 0) nyz += 3;
+  nyz += e->split.launches();
   int npair = 0;
   for (const auto& p : e->pairs) npair += p.launches;
   int per = 1 + npair * ns + 2 * e->samp_magnets;  // controller, stray-field pairs, samples
@@ -2000,6 +2041,9 @@ mpx_status mpx_engine_create(int device, mpx_engine** out) {
   for (int l = 0; l < 4; ++l) fft_kernels.push_back((const void*)pair_yz_fn(l));
   for (int c = 0; c < YZ_CLASSES; ++c)
     fft_kernels.push_back((const void*)(c >= 15 ? yz_long_fn(c) : c >= 10 ? yz_warp_fn(c) : yz_block_fn(c)));
+  fft_kernels.push_back((const void*)ycw_fn(-1));
+  fft_kernels.push_back((const void*)ycw_fn(1));
+  fft_kernels.push_back((const void*)zcw_fn());
   for (int lr = 3; lr <= 4; ++lr) {
     fft_kernels.push_back((const void*)ycols_fn(-1, lr));
     fft_kernels.push_back((const void*)ycols_fn(1, lr));
@@ -2444,8 +2488,8 @@ mpx_status mpx_magnet_bytes(const mpx_magnet_desc* d, int64_t* resident, int64_t
     const int yzs = yz_smem_of(d->size[2], nkx, P[1], P[2]);
     if (P[2] > 16 || yzs > SMEM_DYN_MAX) {  // split y/z path: T and its work items
       res += 8 * Fh * 3 * d->size[2] * P[1];
-      const int64_t ncy = std::max<int64_t>(1, std::min<int64_t>(Fh * 3 * d->size[2], (YZ_VPT * YZ_THREADS) / P[1]));
-      const int64_t nkz = std::max(1, std::min(P[1], (YZ_VPT * YZ_THREADS) / (3 * P[2])));
+      int ncy, nkz;
+      split_shapes((int)(Fh * 3 * d->size[2]), P[1], P[2], split_warp(P[1], P[2]), &ncy, &nkz);
       res += (int64_t)sizeof(Work) * ((Fh * 3 * d->size[2] + ncy - 1) / ncy + Fh * ((P[1] + nkz - 1) / nkz));
     }
     KernelGeom g;
@@ -2728,8 +2772,7 @@ mpx_status mpx_profile_attempt(mpx_engine* e, int method, int reps, double ms[4]
     if (e->n_t_demag > 0) {
       for (int c = 0; c < YZ_CLASSES; ++c)
         MPX_TRY(launch_yz(e, c, e->d_kx_demag[c], e->n_kx_demag[c], e->smem_yz[c], s, 1));
-      MPX_TRY(launch_split(e, e->d_t_ycols, e->n_t_ycols, e->d_t_zmul, e->n_t_zmul, e->smem_ycols, e->smem_zmul,
-                           e->maxpy_split, e->maxpz_split, s, 1, e->d_t_tc, e->n_t_tc));
+      MPX_TRY(launch_split(e, e->split, s, 1));
     }
     CUDA_TRY(cudaEventRecord(ev[3], e->stream));
     if (e->n_t_demag > 0)
@@ -2812,9 +2855,7 @@ mpx_status mpx_profile_eval(mpx_engine* e, int magnet, int reps, double ms[4]) {
       xfwd_fn(false, x_pair_of(m))<<<ntile, nt, sx, e->stream>>>(e->d_mags, e->d_groups, m->d_tiles, 0, 0, nullptr, e->d_tw);
       CUDA_TRY(cudaEventRecord(ev[1], e->stream));
       if (m->split)
-        MPX_TRY(launch_split(e, m->d_ycw, (int)m->ycw.size(), m->d_zmw, (int)m->zmw.size(), ycols_smem(m),
-                             zmul_smem(m), m->P[1], m->P[2], 0, 0, m->d_tcw,
-                           (int)m->tcw.size()));
+        MPX_TRY(launch_split(e, split_of(m), 0, 0));
       else
         MPX_TRY(launch_yz(e, yz_class(m), m->d_kxw, (int)m->kxw.size(), syz, 0, 0));
       CUDA_TRY(cudaEventRecord(ev[2], e->stream));

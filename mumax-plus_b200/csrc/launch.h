@@ -52,6 +52,8 @@ YzFn yz_long_fn(int cls);
 // thick.cu: the split y/z path
 YzFn ycols_fn(int dir, int maxlr);
 YzFn zmul_fn(int maxlr);
+YzFn ycw_fn(int dir);
+YzFn zcw_fn();
 
 // Their warp-column forms (k_ycw, k_zcw of yzsplit.cuh): block sizes, columns or ky
 // per block, and dynamic shared memory.

@@ -9,5 +9,7 @@ YzFn ycols_fn(int dir, int maxlr) {
   return maxlr == 3 ? k_ycols<1, 3> : k_ycols<1, 4>;
 }
 YzFn zmul_fn(int maxlr) { return maxlr == 3 ? k_zmul<3> : k_zmul<4>; }
+YzFn ycw_fn(int dir) { return dir < 0 ? k_ycw<-1> : k_ycw<1>; }
+YzFn zcw_fn() { return k_zcw; }
 
 }  // namespace mpx
