@@ -92,7 +92,9 @@ __device__ __forceinline__ bool load_descs(MagnetDev& sM, GroupDev& sG, const Ma
 // exited): before pdl_wait it reads only data that no kernel of the current
 // attempt writes (magnet and group descriptors, twiddle tables); pdl_wait
 // returns once the previous kernel has completed and its writes are visible.
-// Both are no-ops for a kernel launched without the attribute.
+// A block with nothing to do waits too: a kernel whose blocks all left at once would
+// be complete before its predecessor, and the kernel after it would no longer wait
+// for that one.  Both are no-ops for a kernel launched without the attribute.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -234,7 +236,10 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __re
   __shared__ GroupDev G;
   pdl_trigger();  // the y/z pass may start its prologue during this kernel's last wave
   const Work wk = work[blockIdx.x];
-  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) return;
+  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) {
+    pdl_wait();
+    return;
+  }
   const int z = wk.z, y0 = wk.y0, ty = wk.ty;
   const int nx = M.n[0], ny = M.n[1], nz = M.n[2], N = M.N;
   const int logL = M.logP[0], L = 1 << logL, cs = xrow_stride(L, ty);
@@ -653,7 +658,10 @@ __global__ void __launch_bounds__(384, MAXLR == 3 ? 2 : 1)
   __shared__ GroupDev G;
   pdl_trigger();
   const Work wk = work[blockIdx.x];
-  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) return;
+  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) {
+    pdl_wait();
+    return;
+  }
   const int kx0 = wk.z, nkx = wk.y0;
   const int ny = M.n[1], nz = M.n[2];
   const int logPy = M.logP[1], Py = 1 << logPy, cs = plen(Py);
@@ -832,7 +840,10 @@ __global__ void __launch_bounds__(yzw_threads<PZ>(), PZ == 16 ? 1 : 2)
   __shared__ GroupDev G;
   pdl_trigger();  // the x-inverse pass may start its prologue during the last wave
   const Work wk = work[blockIdx.x];
-  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) return;
+  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) {
+    pdl_wait();
+    return;
+  }
   const int kx0 = wk.z, nkx = wk.y0;
   switch (M.logP[1]) {
     case 6: yzw_body<PZ, 2>(M, kx0, nkx, sm, tw); break;
@@ -854,7 +865,10 @@ __global__ void __launch_bounds__(yzw_threads<PZ>(), PZ == 16 ? 1 : 2)
   __shared__ GroupDev G;
   pdl_trigger();  // the x-inverse pass may start its prologue during the last wave
   const Work wk = work[blockIdx.x];
-  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) return;
+  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) {
+    pdl_wait();
+    return;
+  }
   yzw_body<PZ, 32>(M, wk.z, wk.y0, sm, tw);
 }
 
@@ -873,7 +887,10 @@ __global__ void __launch_bounds__(YZP_THREADS, 1)
   __shared__ GroupDev G;
   pdl_trigger();  // the x-inverse pass may start its prologue during the last wave
   const Work wk = work[blockIdx.x];
-  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) return;
+  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) {
+    pdl_wait();
+    return;
+  }
   constexpr int Py = 2048, LOGPY = 11, cs = qlen(Py);
   const int kx0 = wk.z, nkx = wk.y0;
   const int ny = M.n[1], nz = M.n[2];
@@ -1547,7 +1564,10 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __re
   __shared__ GroupDev G;
   pdl_trigger();  // the next stage's x pass may start its prologue during the last wave
   const Work wk = work[blockIdx.x];
-  if (!load_descs(M, G, mags, groups, wk.mag, ea.gate, ea.stage)) return;
+  if (!load_descs(M, G, mags, groups, wk.mag, ea.gate, ea.stage)) {
+    pdl_wait();
+    return;
+  }
   const int z = wk.z, y0 = wk.y0, ty = wk.ty;
   const int nx = M.n[0], ny = M.n[1], nz = M.n[2];
   const int logL = M.logP[0], L = 1 << logL, cs = xrow_stride(L, ty);
