@@ -24,7 +24,7 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC",
-    "--expt-relaxed-constexpr",
+    "--expt-relaxed-constexpr", "-Xfatbin", "-compress-all",
 ]
 
 

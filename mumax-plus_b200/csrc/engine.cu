@@ -309,7 +309,8 @@ struct mpx_engine {
   float* d_dftB = nullptr;
   int n_sm = 148;  // multiprocessors of the engine's device
   int smem_x = 0, nt_x = 256;
-  bool x_pair = false;  // a launched magnet has 2048-point x rows: the PAIR forms of the x passes
+  XForm x_form;                   // of the launched magnets
+  bool yz_one[YZ_CLASSES] = {};   // all blocks of the class have no more columns than warps
   bool any_nodemag = false;
   int64_t bytes = 0;
   int64_t launches = 0;
@@ -656,9 +657,9 @@ SplitLaunch split_of(const Magnet* m) {
 // y/z launch for one class: warp columns for y lengths 64 .. 1024 (k_yzw);
 // else the radix-8 form for z lengths up to 8 and y lengths up to 2048, the
 // radix-16 form otherwise (k_yz)
-mpx_status launch_yz(mpx_engine* e, int cls, const Work* work, int n, int smem, int stage, int gate) {
+mpx_status launch_yz(mpx_engine* e, int cls, const Work* work, int n, int smem, bool one, int stage, int gate) {
   if (n <= 0) return MPX_OK;
-  const YzFn fn = cls >= 15 ? yz_long_fn(cls) : cls >= 10 ? yz_warp_fn(cls) : yz_block_fn(cls);
+  const YzFn fn = cls >= 15 ? yz_long_fn(cls) : cls >= 10 ? yz_warp_fn(cls, one) : yz_block_fn(cls);
   CUDA_TRY(launch_pdl(fn, n, yz_threads(cls), smem, e->stream, e->d_mags, e->d_groups, work, stage, gate, e->d_tw));
   e->launches++;
   return MPX_OK;
@@ -666,13 +667,29 @@ mpx_status launch_yz(mpx_engine* e, int cls, const Work* work, int n, int smem, 
 // The x-pass kernels of a launch: the PAIR forms (2048-point warp-pair rows
 // compiled in) when one of its magnets has 2048-point x rows, else the forms
 // without them (the shorter lengths keep their registers and code).
-bool x_pair_of(const Magnet* m) { return m->P[0] == 2048; }
 
 int x_threads(const Magnet* m) {
   int rows = m->ty + (m->ty + 1) / 2;
   int t = (rows * m->P[0] + 7) / 8;  // 8 values per thread in the x FFTs
   t = ((t + 31) / 32) * 32;
   return std::min(X_THREADS_MAX, std::max(64, t));
+}
+
+// The x passes of a launch of blocks of nt threads: the form that all its magnets
+// can take (join) from each one's (x_form_of).  `one` stays with launches that have
+// 512-point rows at all.
+XForm x_form_of(const Magnet* m, int nt) {
+  XForm f;
+  f.pair = m->P[0] == 2048;
+  f.mask = (m->dev.terms & FLAG_LEAN) && !m->dev.fast;
+  f.one = m->P[0] <= 512 && 32 * (m->ty + (m->ty + 1) / 2) <= nt;
+  return f;
+}
+// The y/z blocks of the magnet have no more columns than warps (z lengths 1 and 4:
+// the others have more columns per kx).
+bool yz_one_of(const Magnet* m) {
+  return yz_warp(m->P[1]) && m->P[1] < 1024 && (m->P[2] == 1 || m->P[2] == 4) &&
+         32 * 3 * m->dev.n[2] * m->nkx <= yzw_threads_of(m->P[2]);
 }
 
 // Tile shapes for magnets launched together: from each magnet's default
@@ -767,8 +784,10 @@ mpx_status rebuild_tables(mpx_engine* e) {
   e->split = SplitLaunch();
   e->smem_x = 0;
   e->nt_x = 256;
-  e->x_pair = false;
-  for (int c = 0; c < YZ_CLASSES; ++c) e->smem_yz[c] = 0;
+  for (int c = 0; c < YZ_CLASSES; ++c) {
+    e->smem_yz[c] = 0;
+    e->yz_one[c] = false;
+  }
   for (auto& mp : e->mags) {
     if (!mp || mp->probe) continue;  // probe grids of stray-field evaluations
     Magnet* m = mp.get();
@@ -793,14 +812,31 @@ mpx_status rebuild_tables(mpx_engine* e) {
       } else {
         const int cls = yz_class(m);
         want[mpx_engine::TT_YZ0 + cls].push_back({m, &m->kxw});
+        e->yz_one[cls] = yz_one_of(m) && (e->smem_yz[cls] == 0 || e->yz_one[cls]);
         e->smem_yz[cls] = std::max(e->smem_yz[cls], yz_smem(m));
       }
       e->nt_x = std::max(e->nt_x, x_threads(m));
-      e->x_pair = e->x_pair || x_pair_of(m);
     } else {
       want[mpx_engine::TT_LOCAL].push_back({m, &m->tiles});
     }
   }
+  // one row / column per warp only in an engine with a single group (a world, one
+  // served solve): in a batch the launched set keeps changing, and a form that
+  // comes and goes with it would instantiate the attempt graphs anew each time
+  // (batches lost 4 %)
+  const int ngroups = (int)std::count_if(e->groups.begin(), e->groups.end(), [](const auto& g) { return g != nullptr; });
+  e->x_form = XForm();
+  e->x_form.one = ngroups == 1;
+  for (int c = 0; c < YZ_CLASSES; ++c) e->yz_one[c] = e->yz_one[c] && ngroups == 1;
+  bool any512 = false;
+  for (auto& pr : want[mpx_engine::TT_DEMAG]) {
+    const XForm f = x_form_of(pr.first, e->nt_x);
+    e->x_form.pair = e->x_form.pair || f.pair;
+    e->x_form.mask = e->x_form.mask || f.mask;
+    e->x_form.one = e->x_form.one && f.one;
+    any512 = any512 || pr.first->P[0] == 512;
+  }
+  e->x_form.one = e->x_form.one && any512;
   // each table: holes for the magnets that left (or whose lists changed), the
   // newcomers appended, compaction when the holes outnumber the live entries,
   // and an upload of the changed entries only
@@ -886,8 +922,8 @@ mpx_status rebuild_tables(mpx_engine* e) {
   // changed launch size updates the captured graphs in place.
   std::vector<long long> sig;
   for (int t = 0; t < NT; ++t) sig.insert(sig.end(), {(long long)(uintptr_t)e->tt[t].dev, (long long)e->tt[t].items.size()});
-  for (int c = 0; c < YZ_CLASSES; ++c) sig.push_back(e->smem_yz[c]);
-  sig.insert(sig.end(), {e->smem_x, e->nt_x, e->x_pair ? 1 : 0, e->split.smem_y, e->split.smem_z, e->split.max_py,
+  for (int c = 0; c < YZ_CLASSES; ++c) sig.insert(sig.end(), {e->smem_yz[c], e->yz_one[c]});
+  sig.insert(sig.end(), {e->smem_x, e->nt_x, e->x_form.pair, e->x_form.mask, e->x_form.one, e->split.smem_y, e->split.smem_z, e->split.max_py,
                          e->split.max_pz, e->split.smem_yw, e->split.smem_zw});
   e->tables_dirty = false;
   if (e->tables_valid && sig == e->tables_sig) return MPX_OK;
@@ -1473,14 +1509,16 @@ mpx_status load_params(mpx_engine* e, Magnet* m, const mpx_magnet_desc* d) {
   m->stray_dst = !d->stray_destination_off;
   e->pairs_dirty = true;
   for (int c = 0; c < 3; ++c) D.wb[c] = (float)e->wb[c];
-  // fast path: every parameter uniform, no geometry, no regions
-  bool uniform = !d->geometry && !d->regions;
-  for (const mpx_scalar* s : {&d->msat, &d->aex, &d->alpha, &d->ku1, &d->ku2, &d->frozen_spins, &d->kc1, &d->kc2,
-                               &d->kc3})
+  // lean path: every field parameter uniform, no regions; fast path: damping and
+  // frozen spins too, no geometry
+  bool uniform = !d->regions;
+  for (const mpx_scalar* s : {&d->msat, &d->aex, &d->ku1, &d->ku2, &d->kc1, &d->kc2, &d->kc3})
     uniform = uniform && !s->cells;
   for (int c = 0; c < 9; ++c) uniform = uniform && !d->dmi[c].cells;
   uniform = uniform && !d->anis_u.cells && !d->bias_magnetic_field.cells && !d->anis_c1.cells && !d->anis_c2.cells;
-  D.fast = uniform ? 1 : 0;
+  if (uniform) D.terms = terms |= FLAG_LEAN;
+  m->terms_base = terms;
+  D.fast = uniform && !d->geometry && !d->alpha.cells && !d->frozen_spins.cells;
   if (uniform) {
     const float a = D.aex.u, ms = D.msat.u;
     for (int ax = 0; ax < 3; ++ax) D.fe[ax] = (2 * a) * D.w[ax];  // 2 A w, as physics/exchange.cu:100
@@ -1720,13 +1758,13 @@ mpx_status eval_into(mpx_engine* e, Magnet* m, int q, float* out) {
   if (m->hstray) MPX_TRY(launch_pairs(e, m->slot, 0, 0));  // stray fields of the other magnets' states
   if (m->demag && needs_demag) {
     const int sx = x_smem(m), syz = yz_smem(m), nt = x_threads(m);
-    xfwd_fn(false, x_pair_of(m))<<<ntile, nt, sx, e->stream>>>(e->d_mags, e->d_groups, m->d_tiles, 0, 0, nullptr,
+    xfwd_fn(false, x_form_of(m, nt))<<<ntile, nt, sx, e->stream>>>(e->d_mags, e->d_groups, m->d_tiles, 0, 0, nullptr,
                                                                 e->d_tw);
     if (m->split)
       MPX_TRY(launch_split(e, split_of(m), 0, 0));
     else
-      MPX_TRY(launch_yz(e, yz_class(m), m->d_kxw, (int)m->kxw.size(), syz, 0, 0));
-    CUDA_TRY(launch_pdl(xinv_fn(x_pair_of(m)), ntile, nt, sx, e->stream, e->d_mags, e->d_groups, m->d_tiles, ea,
+      MPX_TRY(launch_yz(e, yz_class(m), m->d_kxw, (int)m->kxw.size(), syz, yz_one_of(m), 0, 0));
+    CUDA_TRY(launch_pdl(xinv_fn(x_form_of(m, nt)), ntile, nt, sx, e->stream, e->d_mags, e->d_groups, m->d_tiles, ea,
                         e->d_tw));
     e->launches += 2;
   } else {
@@ -1751,15 +1789,15 @@ mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
     // stage states: combination fused into the x-forward pass, or k_combine
     if (e->n_t_demag > 0) {
       if (s == 0)
-        xfwd_fn(false, e->x_pair)<<<e->n_t_demag, e->nt_x, e->smem_x, e->stream>>>(e->d_mags, e->d_groups,
+        xfwd_fn(false, e->x_form)<<<e->n_t_demag, e->nt_x, e->smem_x, e->stream>>>(e->d_mags, e->d_groups,
                                                                                     e->d_t_demag, 0, 1, nullptr,
                                                                                     e->d_tw);
       else if (s == first_stage)  // after the step controller: fully serialised
-        xfwd_fn(true, e->x_pair)<<<e->n_t_demag, e->nt_x, e->smem_x, e->stream>>>(e->d_mags, e->d_groups,
+        xfwd_fn(true, e->x_form)<<<e->n_t_demag, e->nt_x, e->smem_x, e->stream>>>(e->d_mags, e->d_groups,
                                                                                    e->d_t_demag, s, 1, nullptr,
                                                                                    e->d_tw);
       else  // after the previous stage (the group state is constant within an attempt)
-        CUDA_TRY(launch_pdl(xfwd_fn(true, e->x_pair), e->n_t_demag, e->nt_x, e->smem_x, e->stream, e->d_mags,
+        CUDA_TRY(launch_pdl(xfwd_fn(true, e->x_form), e->n_t_demag, e->nt_x, e->smem_x, e->stream, e->d_mags,
                             e->d_groups, e->d_t_demag, s, 1, (const float*)nullptr, e->d_tw));
       e->launches++;
     }
@@ -1771,9 +1809,9 @@ mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
     MPX_TRY(launch_pairs(e, -1, s, 1));
     if (e->n_t_demag > 0) {
       for (int c = 0; c < YZ_CLASSES; ++c)
-        MPX_TRY(launch_yz(e, c, e->d_kx_demag[c], e->n_kx_demag[c], e->smem_yz[c], s, 1));
+        MPX_TRY(launch_yz(e, c, e->d_kx_demag[c], e->n_kx_demag[c], e->smem_yz[c], e->yz_one[c], s, 1));
       MPX_TRY(launch_split(e, e->split, s, 1));
-      CUDA_TRY(launch_pdl(xinv_fn(e->x_pair), e->n_t_demag, e->nt_x, e->smem_x, e->stream, e->d_mags, e->d_groups,
+      CUDA_TRY(launch_pdl(xinv_fn(e->x_form), e->n_t_demag, e->nt_x, e->smem_x, e->stream, e->d_mags, e->d_groups,
                           e->d_t_demag, ea, e->d_tw));
       e->launches++;
     }
@@ -2029,10 +2067,17 @@ mpx_status mpx_engine_create(int device, mpx_engine** out) {
   CUDA_TRY(cudaMalloc(&e->d_redout, sizeof(double) * 4));  // 3 reduction results, or the 4 of k_min_final
   // large dynamic shared memory and the max-shared carveout for the FFT kernels
   std::vector<const void*> fft_kernels;
+  for (int f = 0; f < 6; ++f) {  // the forms of the x passes (warp pairs and one row per warp exclude each other)
+    XForm xf;
+    xf.pair = f >> 1 == 1;
+    xf.one = f >> 1 == 2;
+    xf.mask = f & 1;
+    fft_kernels.push_back((const void*)xfwd_fn(f & 1, xf));
+    fft_kernels.push_back((const void*)xinv_fn(xf));
+  }
+  fft_kernels.push_back((const void*)yz_warp_fn(10, true));
+  fft_kernels.push_back((const void*)yz_warp_fn(12, true));
   for (int pair = 0; pair < 2; ++pair) {
-    fft_kernels.push_back((const void*)xfwd_fn(false, pair));
-    fft_kernels.push_back((const void*)xfwd_fn(true, pair));
-    fft_kernels.push_back((const void*)xinv_fn(pair));
     fft_kernels.push_back((const void*)pair_xfwd_fn(pair));
     fft_kernels.push_back((const void*)pair_zmul_fn(pair));
     fft_kernels.push_back((const void*)pair_yfft_fn(pair ? 1 : -1));
@@ -2040,7 +2085,7 @@ mpx_status mpx_engine_create(int device, mpx_engine** out) {
   fft_kernels.push_back((const void*)pair_xinv_fn());
   for (int l = 0; l < 4; ++l) fft_kernels.push_back((const void*)pair_yz_fn(l));
   for (int c = 0; c < YZ_CLASSES; ++c)
-    fft_kernels.push_back((const void*)(c >= 15 ? yz_long_fn(c) : c >= 10 ? yz_warp_fn(c) : yz_block_fn(c)));
+    fft_kernels.push_back((const void*)(c >= 15 ? yz_long_fn(c) : c >= 10 ? yz_warp_fn(c, false) : yz_block_fn(c)));
   fft_kernels.push_back((const void*)ycw_fn(-1));
   fft_kernels.push_back((const void*)ycw_fn(1));
   fft_kernels.push_back((const void*)zcw_fn());
@@ -2762,7 +2807,7 @@ mpx_status mpx_profile_attempt(mpx_engine* e, int method, int reps, double ms[4]
   for (int r = 0; r <= reps; ++r) {
     CUDA_TRY(cudaEventRecord(ev[0], e->stream));
     if (e->n_t_demag > 0)
-      xfwd_fn(true, e->x_pair)<<<e->n_t_demag, e->nt_x, e->smem_x, e->stream>>>(e->d_mags, e->d_groups, e->d_t_demag, s, 1,
+      xfwd_fn(true, e->x_form)<<<e->n_t_demag, e->nt_x, e->smem_x, e->stream>>>(e->d_mags, e->d_groups, e->d_t_demag, s, 1,
                                                                     nullptr, e->d_tw);
     if (e->n_t_local > 0)
       combine_fn()<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, s, 0);
@@ -2771,12 +2816,12 @@ mpx_status mpx_profile_attempt(mpx_engine* e, int method, int reps, double ms[4]
     CUDA_TRY(cudaEventRecord(ev[2], e->stream));
     if (e->n_t_demag > 0) {
       for (int c = 0; c < YZ_CLASSES; ++c)
-        MPX_TRY(launch_yz(e, c, e->d_kx_demag[c], e->n_kx_demag[c], e->smem_yz[c], s, 1));
+        MPX_TRY(launch_yz(e, c, e->d_kx_demag[c], e->n_kx_demag[c], e->smem_yz[c], e->yz_one[c], s, 1));
       MPX_TRY(launch_split(e, e->split, s, 1));
     }
     CUDA_TRY(cudaEventRecord(ev[3], e->stream));
     if (e->n_t_demag > 0)
-      CUDA_TRY(launch_pdl(xinv_fn(e->x_pair), e->n_t_demag, e->nt_x, e->smem_x, e->stream, e->d_mags, e->d_groups, e->d_t_demag, ea,
+      CUDA_TRY(launch_pdl(xinv_fn(e->x_form), e->n_t_demag, e->nt_x, e->smem_x, e->stream, e->d_mags, e->d_groups, e->d_t_demag, ea,
                           e->d_tw));
     if (e->n_t_local > 0) local_fn()<<<e->n_t_local, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_local, ea);
     CUDA_TRY(cudaEventRecord(ev[4], e->stream));
@@ -2852,14 +2897,14 @@ mpx_status mpx_profile_eval(mpx_engine* e, int magnet, int reps, double ms[4]) {
     float t[4] = {0, 0, 0, 0};
     if (m->demag) {
       CUDA_TRY(cudaEventRecord(ev[0], e->stream));
-      xfwd_fn(false, x_pair_of(m))<<<ntile, nt, sx, e->stream>>>(e->d_mags, e->d_groups, m->d_tiles, 0, 0, nullptr, e->d_tw);
+      xfwd_fn(false, x_form_of(m, nt))<<<ntile, nt, sx, e->stream>>>(e->d_mags, e->d_groups, m->d_tiles, 0, 0, nullptr, e->d_tw);
       CUDA_TRY(cudaEventRecord(ev[1], e->stream));
       if (m->split)
         MPX_TRY(launch_split(e, split_of(m), 0, 0));
       else
-        MPX_TRY(launch_yz(e, yz_class(m), m->d_kxw, (int)m->kxw.size(), syz, 0, 0));
+        MPX_TRY(launch_yz(e, yz_class(m), m->d_kxw, (int)m->kxw.size(), syz, yz_one_of(m), 0, 0));
       CUDA_TRY(cudaEventRecord(ev[2], e->stream));
-      CUDA_TRY(launch_pdl(xinv_fn(x_pair_of(m)), ntile, nt, sx, e->stream, e->d_mags, e->d_groups, m->d_tiles, ea, e->d_tw));
+      CUDA_TRY(launch_pdl(xinv_fn(x_form_of(m, nt)), ntile, nt, sx, e->stream, e->d_mags, e->d_groups, m->d_tiles, ea, e->d_tw));
       CUDA_TRY(cudaEventRecord(ev[3], e->stream));
       e->launches += 2;
       CUDA_TRY(cudaEventSynchronize(ev[3]));

@@ -401,12 +401,17 @@ __device__ __forceinline__ void load_twq(float2* dst, const float2* __restrict__
   }
 }
 
+// Units of W columns: 32 / Q fill the warp's lanes in both steps.  W = 1 (lanes
+// s < Q in the outer step) is the form for blocks with no more columns than
+// warps: the same operations per column, about half the instructions per warp, so
+// half the latency of the transform where a small solve leaves the other warps
+// idle.
+//
 // Inner step of lane j for W = 32 / Q columns of length L = 32 Q held together:
 // v[c Q + r] = x_c[j + 32 r] (r < Q; with ZH the values r >= Q/2 are zero and
 // unread).  On return v[c Q + s] holds W_L^{j s} sum_r x_c[j + 32 r] W_Q^{r s}.
-template <int Q, int DIR, bool ZH>
+template <int Q, int DIR, bool ZH, int W = 32 / Q>
 __device__ __forceinline__ void four_step_inner(float2 (&v)[32], const float2* twq, int lane) {
-  constexpr int W = 32 / Q;
 #pragma unroll
   for (int c = 0; c < W; ++c) {
     float2 u[Q];
@@ -433,10 +438,9 @@ __device__ __forceinline__ void four_step_inner(float2 (&v)[32], const float2* t
 // (t < 16 only with LO).  The columns are free again when this returns.
 // With cs = qlen(L) = 33 Q (mod 16: Q) the reads of the outer step, lanes
 // (c, s) at element j + 32 s of column c, hit 16 different banks per half-warp.
-template <int Q, int DIR, bool LO>
+template <int Q, int DIR, bool LO, int W = 32 / Q>
 __device__ __forceinline__ void four_step_outer(float2 (&v)[32], float2* base, int cs, int nc, int lane) {
-  constexpr int W = 32 / Q;
-  if constexpr (W == 1) {  // one column: no column index, no guard
+  if constexpr (Q == 32) {  // one column: no column index, no guard
 #pragma unroll
     for (int s = 0; s < 32; ++s) base[lane + 33 * s] = v[s];  // element lane + 32 s
     __syncwarp();
@@ -539,9 +543,8 @@ __device__ __forceinline__ void pair_rows(float2* buf, int nrows, int cs, const 
 // the upper half of every input row is zero padding (not read).  LO: only the
 // lower half of every output row is written.  No block barrier: the caller
 // synchronises before (rows and twiddles written) and after.
-template <int Q, int DIR, bool ZIN, bool LO>
+template <int Q, int DIR, bool ZIN, bool LO, int W = 32 / Q>
 __device__ __forceinline__ void warp_rows(float2* buf, int nrows, int cs, const float2* twq) {
-  constexpr int W = 32 / Q;
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int r0 = (threadIdx.x >> 5) * W; r0 < nrows; r0 += nw * W) {
     float2* R = buf + r0 * cs;
@@ -552,9 +555,9 @@ __device__ __forceinline__ void warp_rows(float2* buf, int nrows, int cs, const 
 #pragma unroll
       for (int r = 0; r < Q; ++r)
         v[c * Q + r] = (c < nc && (!ZIN || r < Q / 2)) ? R[c * cs + lane + 33 * r] : make_float2(0.f, 0.f);
-    four_step_inner<Q, DIR, ZIN>(v, twq, lane);
-    four_step_outer<Q, DIR, LO>(v, R, cs, nc, lane);
-    if constexpr (W == 1) {
+    four_step_inner<Q, DIR, ZIN, W>(v, twq, lane);
+    four_step_outer<Q, DIR, LO, W>(v, R, cs, nc, lane);
+    if constexpr (Q == 32) {
 #pragma unroll
       for (int t = 0; t < (LO ? 16 : 32); ++t) R[lane + 33 * t] = v[t];
     } else {

@@ -226,7 +226,9 @@ __device__ __forceinline__ int tile_log(int ty) { return ty <= 1 ? 0 : 32 - __cl
 // PAIR: the 2048-point rows of the warp pairs are compiled in (the forms launched
 // when a magnet with such rows is in the launch; without them the others keep
 // the registers and code of the shorter lengths).
-template <bool COMBINE, bool PAIR = false>
+// ONE: 512-point rows one per warp, for launches of rows up to 512 points whose
+// tiles have no more rows than warps (see k_yzw).
+template <bool COMBINE, bool PAIR = false, bool ONE = false>
 __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups,
                                               const Work* __restrict__ work, int stage, int gate,
                                               const float* __restrict__ msrc_override,
@@ -338,8 +340,8 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __re
   __syncthreads();
   if (wrow) {
     if (PAIR && logL == 11) pair_rows<-1, true, false>(sm, ty + nzrows, cs, tws);
-    else if (logL == 10) warp_rows<32, -1, true, false>(sm, ty + nzrows, cs, tws);
-    else warp_rows<16, -1, true, false>(sm, ty + nzrows, cs, tws);
+    else if (!ONE && logL == 10) warp_rows<32, -1, true, false>(sm, ty + nzrows, cs, tws);
+    else warp_rows<16, -1, true, false, ONE ? 1 : 2>(sm, ty + nzrows, cs, tws);
     __syncthreads();
   } else {
     fft_many<-1, 3, 1>(sm, logL, ty + nzrows, cs, tws);
@@ -724,10 +726,10 @@ __global__ void __launch_bounds__(384, MAXLR == 3 ? 2 : 1)
 
 // Forward y transforms of the ncol columns of S (ny rows each, zero padding
 // above) into D.
-template <int Q>
+template <int Q, int W = 32 / Q>
 __device__ __forceinline__ void yzw_forward(const float2* __restrict__ S, int ny, float2* D, int ncol,
                                             const float2* twq, size_t sleft) {
-  constexpr int W = 32 / Q, cs = qlen(32 * Q);
+  constexpr int cs = qlen(32 * Q);
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int lc = lane / Q, ls = lane % Q;  // column and s of this lane in the outer step
   for (int col0 = (threadIdx.x >> 5) * W; col0 < ncol; col0 += nw * W) {
@@ -742,10 +744,10 @@ __device__ __forceinline__ void yzw_forward(const float2* __restrict__ S, int ny
                            ? __ldg(S + (size_t)(col0 + c) * ny + y)
                            : make_float2(0.f, 0.f);
       }
-    four_step_inner<Q, -1, true>(v, twq, lane);
+    four_step_inner<Q, -1, true, W>(v, twq, lane);
     float2* C = D + col0 * cs;
-    four_step_outer<Q, -1, false>(v, C, cs, nc, lane);
-    if constexpr (W == 1) {
+    four_step_outer<Q, -1, false, W>(v, C, cs, nc, lane);
+    if constexpr (Q == 32) {
 #pragma unroll
       for (int t = 0; t < 32; ++t) C[lane + 33 * t] = v[t];  // ky = lane + 32 t
     } else if (lc < nc) {
@@ -756,10 +758,10 @@ __device__ __forceinline__ void yzw_forward(const float2* __restrict__ S, int ny
 }
 
 // Inverse y transforms of the columns of D; the y < ny outputs go to S.
-template <int Q>
+template <int Q, int W = 32 / Q>
 __device__ __forceinline__ void yzw_inverse(float2* __restrict__ S, int ny, float2* D, int ncol, const float2* twq,
                                             size_t sleft) {
-  constexpr int W = 32 / Q, cs = qlen(32 * Q);
+  constexpr int cs = qlen(32 * Q);
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int lc = lane / Q, ls = lane % Q;
   for (int col0 = (threadIdx.x >> 5) * W; col0 < ncol; col0 += nw * W) {
@@ -770,9 +772,9 @@ __device__ __forceinline__ void yzw_inverse(float2* __restrict__ S, int ny, floa
     for (int c = 0; c < W; ++c)
 #pragma unroll
       for (int r = 0; r < Q; ++r) v[c * Q + r] = (c < nc) ? C[c * cs + lane + 33 * r] : make_float2(0.f, 0.f);
-    four_step_inner<Q, 1, false>(v, twq, lane);
-    four_step_outer<Q, 1, true>(v, C, cs, nc, lane);
-    const int cl = W == 1 ? 0 : lc, sl = W == 1 ? lane : ls;
+    four_step_inner<Q, 1, false, W>(v, twq, lane);
+    four_step_outer<Q, 1, true, W>(v, C, cs, nc, lane);
+    const int cl = Q == 32 ? 0 : lc, sl = Q == 32 ? lane : ls;
     if (cl < nc) {
       float2* __restrict__ Sc = S + (size_t)(col0 + cl) * ny;
 #pragma unroll
@@ -791,7 +793,7 @@ constexpr int yzw_threads() { return PZ == 16 ? 384 : 256; }
 
 // The whole y/z pass of one block for y length Py = 32 Q (every length and
 // stride a compile-time constant).
-template <int PZ, int Q>
+template <int PZ, int Q, bool ONE = false>
 __device__ __forceinline__ void yzw_body(const MagnetDev& M, int kx0, int nkx, float2* sm,
                                          const float2* __restrict__ tw) {
   constexpr int Py = 32 * Q, cs = qlen(Py);
@@ -806,7 +808,8 @@ __device__ __forceinline__ void yzw_body(const MagnetDev& M, int kx0, int nkx, f
   pdl_wait();  // the spectrum is written by the x pass
   float2* S = M.spec + (size_t)kx0 * 3 * nz * ny;
   const size_t sleft = (size_t)(M.Fh - kx0) * 3 * nz * ny;  // elements from S on (checked build)
-  yzw_forward<Q>(S, ny, D, ncol, twq, sleft);
+  constexpr int W = ONE ? 1 : 32 / Q;
+  yzw_forward<Q, W>(S, ny, D, ncol, twq, sleft);
   __syncthreads();
   if constexpr (PZ == 1) {
     for (int t = threadIdx.x; t < nkx << LOGPY; t += blockDim.x) {
@@ -827,11 +830,16 @@ __device__ __forceinline__ void yzw_body(const MagnetDev& M, int kx0, int nkx, f
     }
   }
   __syncthreads();
-  yzw_inverse<Q>(S, ny, D, ncol, twq, sleft);
+  yzw_inverse<Q, W>(S, ny, D, ncol, twq, sleft);
 }
 
 // Work item: magnet, first kx in z, number of consecutive kx in y0.  y lengths 64 .. 512.
-template <int PZ>
+// ONE: a column per warp, for launches whose blocks have no more columns than
+// warps (the same numbers).  A 256 x 64 film has one kx of three columns per block,
+// where 32 / Q columns per warp leave 6 or 7 of 8 warps idle and double the
+// transform's latency.  Kernels of their own: with both forms in one kernel the
+// batches lost 7 % to its size.
+template <int PZ, bool ONE = false>
 __global__ void __launch_bounds__(yzw_threads<PZ>(), PZ == 16 ? 1 : 2)
     k_yzw(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, const Work* __restrict__ work,
           int stage, int gate, const float2* __restrict__ tw) {
@@ -846,10 +854,10 @@ __global__ void __launch_bounds__(yzw_threads<PZ>(), PZ == 16 ? 1 : 2)
   }
   const int kx0 = wk.z, nkx = wk.y0;
   switch (M.logP[1]) {
-    case 6: yzw_body<PZ, 2>(M, kx0, nkx, sm, tw); break;
-    case 7: yzw_body<PZ, 4>(M, kx0, nkx, sm, tw); break;
-    case 8: yzw_body<PZ, 8>(M, kx0, nkx, sm, tw); break;
-    default: yzw_body<PZ, 16>(M, kx0, nkx, sm, tw); break;
+    case 6: yzw_body<PZ, 2, ONE>(M, kx0, nkx, sm, tw); break;
+    case 7: yzw_body<PZ, 4, ONE>(M, kx0, nkx, sm, tw); break;
+    case 8: yzw_body<PZ, 8, ONE>(M, kx0, nkx, sm, tw); break;
+    default: yzw_body<PZ, 16, ONE>(M, kx0, nkx, sm, tw); break;
   }
 }
 
@@ -1140,12 +1148,14 @@ __device__ __forceinline__ void nb_rows_fill(NbRows& T, const MagnetDev& M, int 
   }
 }
 
-// The lean epilogue applies to magnets on the fast path (uniform parameters,
-// no geometry) whose x range lies inside one mastergrid period, so that the
+// The lean epilogue applies to magnets on the fast path, and in the MASK kernels to
+// all with uniform field parameters (a geometry mask, per-cell damping and
+// per-cell frozen spins allowed), whose x range lies inside one mastergrid period, so that the
 // x neighbours of inner cells are x - 1 and x + 1.
+template <bool MASK>
 __device__ __forceinline__ bool lean_ok(const MagnetDev& M) {
   const int off = M.o[0] - M.mgo[0];
-  return M.fast && !M.geom && (M.mg[0] == 0 || (off >= 0 && off + M.n[0] <= M.mg[0]));
+  return (M.fast || (MASK && (M.terms & FLAG_LEAN))) && (M.mg[0] == 0 || (off >= 0 && off + M.n[0] <= M.mg[0]));
 }
 
 // DMI tensor kinds of the lean path: DMI_IFACE when the only nonzero entries
@@ -1236,7 +1246,7 @@ __device__ __forceinline__ float3 llg_torque_rn(float3 m, float3 h, float a) {
 }
 
 __device__ __forceinline__ float3 finish_cell_lean(const MagnetDev& M, const GroupDev& G, float3 mc, float3 he,
-                                                   float3 hd, float3 ext, float3 bdemag) {
+                                                   float3 hd, float3 ext, float3 bdemag, float alpha) {
   const unsigned terms = M.terms;
   const float s = M.finv_ms;
   float3 exch = f3(0, 0, 0), dmi = f3(0, 0, 0), anis = f3(0, 0, 0);
@@ -1255,17 +1265,19 @@ __device__ __forceinline__ float3 finish_cell_lean(const MagnetDev& M, const Gro
   const float3 h = f3(__fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(exch.x, anis.x), ext.x), dmi.x), bdemag.x),
                       __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(exch.y, anis.y), ext.y), dmi.y), bdemag.y),
                       __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(exch.z, anis.z), ext.z), dmi.z), bdemag.z));
-  return G.torque_kind ? damping_torque(mc, h) : llg_torque_rn(mc, h, M.alpha.u);
+  return G.torque_kind ? damping_torque(mc, h) : llg_torque_rn(mc, h, alpha);
 }
 
 // Right-hand side of one cell of a stage on the lean path: the arithmetic of
 // local_terms_fast and of the torque in epilogue_cell, in the same order,
-// with the neighbours taken from the block's row table.
+// with the neighbours taken from the block's row table.  MASK: the magnet has a
+// geometry mask or per-cell damping / frozen spins.
+template <bool MASK>
 __device__ __forceinline__ float3 stage_cell_lean(const MagnetDev& M, const GroupDev& G, const NbRows& T,
                                                   const float* __restrict__ m, int i, int x, int yl, int y, int z,
                                                   float3 bdemag) {
   const int N = M.N;
-  if (M.frozen.u != 0.0f) return f3(0.f, 0.f, 0.f);
+  if (MASK ? (!in_geom(M, i) || M.frozen.at(i) != 0.0f) : M.frozen.u != 0.0f) return f3(0.f, 0.f, 0.f);
   const unsigned terms = M.terms;
   const float3 mc = ldg3(m, N, i);
   float3 he = f3(0, 0, 0), hd = f3(0, 0, 0);
@@ -1285,6 +1297,14 @@ __device__ __forceinline__ float3 stage_cell_lean(const MagnetDev& M, const Grou
       const int b = T.r[yl][q];
       nb[2 + q] = b >= 0 ? b + x : -1;
     }
+    if (MASK && M.geom) {  // a neighbour outside the geometry is a missing one
+      unsigned char g[6];
+#pragma unroll
+      for (int q = 0; q < 6; ++q) g[q] = nb[q] >= 0 ? M.geom[nb[q]] : 0;
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+        if (!g[q]) nb[q] = -1;
+    }
     const bool inner = nb[0] >= 0 && nb[1] >= 0 && nb[2] >= 0 && nb[3] >= 0 && nb[4] >= 0 && nb[5] >= 0;
     const bool ifc = do_dmi && dmi_kind(M) == DMI_IFACE;
     if (__all_sync(__activemask(), inner)) {  // every neighbour present: no ghost cells
@@ -1303,7 +1323,7 @@ __device__ __forceinline__ float3 stage_cell_lean(const MagnetDev& M, const Grou
       ext = f3(ext.x + s.x, ext.y + s.y, ext.z + s.z);
     }
   }
-  float3 k = finish_cell_lean(M, G, mc, he, hd, ext, bdemag);
+  float3 k = finish_cell_lean(M, G, mc, he, hd, ext, bdemag, MASK ? M.alpha.at(i) : M.alpha.u);
   if (!G.torque_kind && (terms & (FLAG_STT_ZL | FLAG_STT_SL))) k = k + stt_torque(M, m, x, y, z, i, mc);
   if (terms & FLAG_THERMAL) k = k + thermal_term(M, i, G.steps, G.dt);
   return k;
@@ -1546,7 +1566,7 @@ __device__ __forceinline__ void stage_quad_lean(const MagnetDev& M, const GroupD
   const float3 ext = (terms & TERM_EXT) ? f3(M.fb[0], M.fb[1], M.fb[2]) : f3(0.f, 0.f, 0.f);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const float3 k = finish_cell_lean(M, G, mc[q], he[q], hd[q], ext, bdemag(q));
+    const float3 k = finish_cell_lean(M, G, mc[q], he[q], hd[q], ext, bdemag(q), M.alpha.u);
     f4set(kx, q, k.x);
     f4set(ky, q, k.y);
     f4set(kz, q, k.z);
@@ -1554,8 +1574,13 @@ __device__ __forceinline__ void stage_quad_lean(const MagnetDev& M, const GroupD
 }
 
 // ------------------------------------------------------------------ k_xinv
-// PAIR as for k_xfwd.
-template <bool PAIR = false>
+// PAIR as for k_xfwd.  MASK: the lean epilogue of magnets with a geometry mask or
+// per-cell damping / frozen spins is compiled in (launched when such a magnet is
+// among the launch's; in the other forms it would cost the common path 2 - 7 %
+// by its registers).  A 200 x 200 disc took 21 us of a 45 us stage in the general
+// path (epilogue_cell), whose cells fetch their neighbours one after the other
+// and divide per neighbour: 18 Fehlberg attempts 4.91 -> 3.18 ms.
+template <bool PAIR = false, bool MASK = false, bool ONE = false>
 __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __restrict__ mags, GroupDev* __restrict__ groups,
                                               const Work* __restrict__ work, EpiArgs ea,
                                               const float2* __restrict__ tw) {
@@ -1583,7 +1608,7 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __re
   __shared__ NbRows T;
   __shared__ float cf[8];  // FSAL error weights dt (b1 - b2) of the stages
   __shared__ int s_quad;   // lean epilogue four cells at a time (16-byte loads and stores)
-  const bool lean = ea.mode == EPI_STAGE && lean_ok(M);
+  const bool lean = ea.mode == EPI_STAGE && lean_ok<MASK>(M);
   if (lean) {
     nb_rows_fill(T, M, y0, ty, z);
     if (threadIdx.x < c_tab.S) cf[threadIdx.x] = (float)(G.dt * (c_tab.b1[threadIdx.x] - c_tab.b2[threadIdx.x]));
@@ -1593,7 +1618,7 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __re
       uintptr_t a = (uintptr_t)stage_m(M, G, ea.stage) | (uintptr_t)M.buf[G.map[2 + ea.stage]];
       if (ea.fsal_err)
         for (int j = 0; j < c_tab.S; ++j) a |= (uintptr_t)M.buf[G.map[2 + j]];
-      s_quad = (a & 15) == 0 && (nx & 3) == 0 && (M.N & 3) == 0 &&
+      s_quad = (a & 15) == 0 && (nx & 3) == 0 && (M.N & 3) == 0 && M.fast &&
                !(M.terms & (FLAG_STRAY | FLAG_STT_ZL | FLAG_STT_SL | FLAG_THERMAL));
     }
   }
@@ -1674,8 +1699,8 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __re
   __syncthreads();
   if (wrow) {  // only x < nx <= L/2 is used
     if (PAIR && logL == 11) pair_rows<1, false, true>(sm, ty + nzrows, cs, tws);
-    else if (logL == 10) warp_rows<32, 1, false, true>(sm, ty + nzrows, cs, tws);
-    else warp_rows<16, 1, false, true>(sm, ty + nzrows, cs, tws);
+    else if (!ONE && logL == 10) warp_rows<32, 1, false, true>(sm, ty + nzrows, cs, tws);
+    else warp_rows<16, 1, false, true, ONE ? 1 : 2>(sm, ty + nzrows, cs, tws);
     __syncthreads();
   } else {
     fft_many<1, 3, 2>(sm, logL, ty + nzrows, cs, tws);
@@ -1749,7 +1774,7 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __re
       const float2 hxy = sm[yl * cs + xidx(x, sh)];
       const float2 hz2 = rows_z[(yl >> 1) * cs + xidx(x, sh)];
       const float3 bd = f3(hxy.x, hxy.y, (yl & 1) ? hz2.y : hz2.x);
-      const float3 k = stage_cell_lean(M, G, T, m, i, x, yl, y0 + yl, z, bd);
+      const float3 k = stage_cell_lean<MASK>(M, G, T, m, i, x, yl, y0 + yl, z, bd);
       store3(kout, N, i, k);
       if (ea.fsal_err) {
         float3 er = f3(0, 0, 0);

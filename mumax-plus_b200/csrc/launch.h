@@ -34,8 +34,12 @@ using ControllerFn = void (*)(GroupDev*, int);
 using YzFn = void (*)(const MagnetDev*, const GroupDev*, const Work*, int, int, const float2*);
 
 // xpass.cu: everything that reads the Butcher tableau
-XfwdFn xfwd_fn(bool combine, bool pair);
-XinvFn xinv_fn(bool pair);
+// Forms of the x passes: warp-pair rows, rows one per warp, masked magnets (kernels.cuh).
+struct XForm {
+  bool pair = false, one = false, mask = false;
+};
+XfwdFn xfwd_fn(bool combine, XForm f);
+XinvFn xinv_fn(XForm f);
 LocalFn local_fn();
 CombineFn combine_fn();
 ControllerFn controller_fn();
@@ -46,7 +50,7 @@ cudaError_t upload_tableau_symbol(const TableauDev& t, cudaStream_t stream);
 // 15 .. 23 y lengths 1024 and 2048 (yzlong.cu).
 constexpr int YZ_CLASSES = 24;
 YzFn yz_block_fn(int cls);
-YzFn yz_warp_fn(int cls);
+YzFn yz_warp_fn(int cls, bool one);
 YzFn yz_long_fn(int cls);
 
 // thick.cu: the split y/z path

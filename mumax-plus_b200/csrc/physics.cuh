@@ -30,7 +30,8 @@ enum : unsigned {
   FLAG_CUBIC = 1024u,  // the anisotropy term is cubic (uniaxial otherwise)
   FLAG_STRAY = 2048u,  // stray fields of other magnets in `hstray`
   FLAG_STT_ZL = 4096u, FLAG_STT_SL = 8192u,  // spin-transfer torque: Zhang-Li or Slonczewski
-  FLAG_THERMAL = 16384u  // thermal noise (temperature not zero)
+  FLAG_THERMAL = 16384u,  // thermal noise (temperature not zero)
+  FLAG_LEAN = 32768u  // field parameters uniform; geometry, per-cell damping and frozen spins allowed
 };
 
 struct DScalar {  // uniform value or per-cell array

@@ -6,11 +6,16 @@
 
 namespace mpx {
 
-XfwdFn xfwd_fn(bool combine, bool pair) {
-  if (combine) return pair ? k_xfwd<true, true> : k_xfwd<true, false>;
-  return pair ? k_xfwd<false, true> : k_xfwd<false, false>;
+XfwdFn xfwd_fn(bool combine, XForm f) {
+  if (f.one) return combine ? k_xfwd<true, false, true> : k_xfwd<false, false, true>;
+  if (combine) return f.pair ? k_xfwd<true, true> : k_xfwd<true, false>;
+  return f.pair ? k_xfwd<false, true> : k_xfwd<false, false>;
 }
-XinvFn xinv_fn(bool pair) { return pair ? k_xinv<true> : k_xinv<false>; }
+XinvFn xinv_fn(XForm f) {
+  if (f.one) return f.mask ? k_xinv<false, true, true> : k_xinv<false, false, true>;
+  if (f.mask) return f.pair ? k_xinv<true, true> : k_xinv<false, true>;
+  return f.pair ? k_xinv<true, false> : k_xinv<false, false>;
+}
 LocalFn local_fn() { return k_local; }
 CombineFn combine_fn() { return k_combine; }
 ControllerFn controller_fn() { return k_controller; }

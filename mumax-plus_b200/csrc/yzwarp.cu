@@ -3,7 +3,8 @@
 
 namespace mpx {
 
-YzFn yz_warp_fn(int cls) {
+YzFn yz_warp_fn(int cls, bool one) {
+  if (one) return cls == 10 ? k_yzw<1, true> : k_yzw<4, true>;
   switch (cls) {
     case 10: return k_yzw<1>;
     case 11: return k_yzw<2>;
