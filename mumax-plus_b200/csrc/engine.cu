@@ -247,14 +247,14 @@ struct SlotTable {
 // FFT form of a stray-field pair on its own kernel grid (pairfft.cuh): the
 // lengths, buffers and launch shapes of its five passes.
 struct PairPlan {
-  PairFft pf{};
+  PairItem it{};
   float2* t = nullptr;   // work spectrum, 3 components
   float2* ks = nullptr;  // kernel spectrum, 6 components
-  int ry_f = 1, zc_f = 1, tky = 1, zc_i = 1, ry_i = 1;  // rows / columns per block of each pass
-  int g_xf = 0, g_yf = 0, g_z = 0, g_yi = 0, g_xi = 0;  // grids
+  int threads = 256;
   int s_xf = 0, s_yf = 0, s_z = 0, s_yi = 0, s_xi = 0;  // dynamic shared memory (bytes)
   int s_yz = 0;  // > 0: the fused y / z pass k_pair_yz (one block per kx) with this shared memory
-  int launches() const { return s_yz > 0 ? 3 : 5; }
+  // plans that can share launches: the same kernels and block size
+  int shape() const { return (s_yz > 0 ? it.pf.logP[2] : 100) + 1000 * threads; }
 };
 
 // Launch of the split y/z path over one magnet or all started ones: block-wide
@@ -327,9 +327,9 @@ struct mpx_engine {
     StrayTable tab;
     bool fft = false;  // FFT form on the pair's kernel grid (plan), else the direct sum (k, tab)
     PairPlan plan;
-    int launches = 1;  // kernels per evaluation
   };
   std::vector<Pair> pairs;
+  int pair_launches = 0;  // kernels of one stage's stray fields (of the last captured attempt)
   // FFT plans of recent stray-field evaluations on other grids (mpx_stray_field),
   // by geometry: source and destination grids, cell size, periodic images
   struct PairCacheEntry {
@@ -592,9 +592,9 @@ int zmul_smem(const Magnet* m) { return (3 * m->nkz * plen(m->P[2]) + m->P[2]) *
 // prologue while the previous kernel of the stream finishes (the kernel calls
 // pdl_wait before it reads anything the earlier kernels write).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, int smem, cudaStream_t st, Args&&... args) {
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int block, int smem, cudaStream_t st, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -1056,27 +1056,31 @@ bool pair_fft_lengths(const int nA[3], const int nB[3], int logP[3]) {
 
 // Launch shapes of the passes for `ncomp` components with input rows nin and
 // output window rows nout (pairfft.cuh); rows per block fill one transform
-// group of PF_POINTS points.
+// group of 8 points per thread.
 void pair_shapes(PairPlan& pl, int ncomp) {
-  const PairFft& pf = pl.pf;
+  PairItem& it = pl.it;
+  const PairFft& pf = it.pf;
   const int Px = 1 << pf.logP[0], Py = 1 << pf.logP[1], Pz = 1 << pf.logP[2], Hx = Px / 2 + 1;
   auto cdiv = [](int a, int b) { return (a + b - 1) / b; };
   const int f2 = (int)sizeof(float2);
-  pl.ry_f = std::max(1, std::min(pf.nin[1], PF_POINTS / Px));
-  pl.g_xf = ncomp * pf.nin[2] * cdiv(pf.nin[1], pl.ry_f);
-  pl.s_xf = (pl.ry_f * plen(Px) + Px) * f2;
-  pl.zc_f = std::max(1, std::min(pf.nin[2], PF_POINTS / Py));
-  pl.g_yf = Hx * ncomp * cdiv(pf.nin[2], pl.zc_f);
-  pl.s_yf = (pl.zc_f * plen(Py) + Py) * f2;
-  pl.tky = std::max(1, std::min(Py, PF_POINTS / (ncomp * Pz)));
-  pl.g_z = Hx * cdiv(Py, pl.tky);
-  pl.s_z = (ncomp * pl.tky * plen(Pz) + Pz) * f2;
-  pl.zc_i = std::max(1, std::min(pf.nout[2], PF_POINTS / Py));
-  pl.g_yi = Hx * ncomp * cdiv(pf.nout[2], pl.zc_i);
-  pl.s_yi = (pl.zc_i * plen(Py) + Py) * f2;
-  pl.ry_i = std::max(1, std::min(pf.nout[1], PF_POINTS / Px));
-  pl.g_xi = ncomp * pf.nout[2] * cdiv(pf.nout[1], pl.ry_i);
-  pl.s_xi = (pl.ry_i * plen(Px) + Px) * f2;
+  pl.threads = std::max({Px, Py, Pz}) > 2048 ? PF_THREADS : PF_THREADS / 2;
+  const int points = pl.threads << PF_LR;  // of one transform group
+  it.ncomp = ncomp;
+  it.ry_f = std::max(1, std::min(pf.nin[1], points / Px));
+  it.g_xf = ncomp * pf.nin[2] * cdiv(pf.nin[1], it.ry_f);
+  pl.s_xf = (it.ry_f * plen(Px) + Px) * f2;
+  it.zc_f = std::max(1, std::min(pf.nin[2], points / Py));
+  it.g_yf = Hx * ncomp * cdiv(pf.nin[2], it.zc_f);
+  pl.s_yf = (it.zc_f * plen(Py) + Py) * f2;
+  it.tky = std::max(1, std::min(Py, points / (ncomp * Pz)));
+  it.g_z = Hx * cdiv(Py, it.tky);
+  pl.s_z = (ncomp * it.tky * plen(Pz) + Pz) * f2;
+  it.zc_i = std::max(1, std::min(pf.nout[2], points / Py));
+  it.g_yi = Hx * ncomp * cdiv(pf.nout[2], it.zc_i);
+  pl.s_yi = (it.zc_i * plen(Py) + Py) * f2;
+  it.ry_i = std::max(1, std::min(pf.nout[1], points / Px));
+  it.g_xi = ncomp * pf.nout[2] * cdiv(pf.nout[1], it.ry_i);
+  pl.s_xi = (it.ry_i * plen(Px) + Px) * f2;
   const int syz = (3 * Pz * plen(Py) + Py) * f2;
   pl.s_yz = (ncomp == 3 && Pz <= 8 && syz <= SMEM_MAX - 8192) ? syz : 0;
 }
@@ -1092,7 +1096,7 @@ void free_pair_plan(mpx_engine* e, PairPlan& pl) {
 // displacements (periodic images of `gimg`: mastergrid and repetitions).
 mpx_status build_pair_fft(mpx_engine* e, const Magnet* A, const int nB[3], const int oB[3], const KernelGeom& gimg,
                           PairPlan& pl) {
-  PairFft& pf = pl.pf;
+  PairFft& pf = pl.it.pf;
   if (!pair_fft_lengths(A->dev.n, nB, pf.logP)) return fail(MPX_ERR_UNSUPPORTED, "stray-field FFT grid too large");
   int K[3], O[3];
   for (int a = 0; a < 3; ++a) {
@@ -1117,18 +1121,21 @@ mpx_status build_pair_fft(mpx_engine* e, const Magnet* A, const int nB[3], const
   }
   // kernel spectrum: the forward passes over the six tabulated components
   PairPlan kp;
-  kp.pf = pf;
-  kp.pf.t = pl.ks;
-  kp.pf.ks = nullptr;
-  for (int a = 0; a < 3; ++a) kp.pf.nin[a] = kp.pf.nout[a] = K[a];
-  kp.pf.win[0] = kp.pf.win[1] = kp.pf.win[2] = 0;
+  kp.it.pf = pf;
+  kp.it.pf.t = pl.ks;
+  kp.it.pf.ks = nullptr;
+  for (int a = 0; a < 3; ++a) kp.it.pf.nin[a] = kp.it.pf.nout[a] = K[a];
+  kp.it.pf.win[0] = kp.it.pf.win[1] = kp.it.pf.win[2] = 0;
+  kp.it.src = -1;
+  kp.it.tab = tab;
   pair_shapes(kp, 6);
-  pair_xfwd_fn(true)<<<kp.g_xf, PF_THREADS, kp.s_xf, e->stream>>>(e->d_mags, e->d_groups, -1, 0, 0, tab, kp.pf, 6,
-                                                                  kp.ry_f, e->d_tw);
-  pair_yfft_fn(-1)<<<kp.g_yf, PF_THREADS, kp.s_yf, e->stream>>>(e->d_mags, e->d_groups, -1, 0, 0, kp.pf, 6, kp.zc_f,
-                                                                e->d_tw);
-  pair_zmul_fn(false)<<<kp.g_z, PF_THREADS, kp.s_z, e->stream>>>(e->d_mags, e->d_groups, -1, 0, 0, kp.pf, 6, kp.tky,
-                                                                 e->d_tw);
+  {
+    PairBatch kb{};
+    kb.p[0] = kp.it;
+    pair_xfwd_fn(true)<<<kp.it.g_xf, kp.threads, kp.s_xf, e->stream>>>(e->d_mags, e->d_groups, 0, 0, kb, e->d_tw);
+    pair_yfft_fn(-1)<<<kp.it.g_yf, kp.threads, kp.s_yf, e->stream>>>(e->d_mags, e->d_groups, 0, 0, kb, e->d_tw);
+    pair_zmul_fn(false)<<<kp.it.g_z, kp.threads, kp.s_z, e->stream>>>(e->d_mags, e->d_groups, 0, 0, kb, e->d_tw);
+  }
   e->launches += 3;
   pfree(e, tab);
   pf.t = pl.t;
@@ -1187,27 +1194,46 @@ mpx_status cached_pair_plan(mpx_engine* e, const Magnet* A, const Magnet* B, con
   return MPX_OK;
 }
 
-// The five passes of one evaluation: the field of `src`'s state for `stage`
-// into out (3 x N of `dst`, added with `add`); `gate` as the stage kernels.
-void launch_pair_fft(mpx_engine* e, const PairPlan& pl, int src, int dst, int stage, int gate, int add, float* out) {
-  const PairFft& pf = pl.pf;
-  pair_xfwd_fn(false)<<<pl.g_xf, PF_THREADS, pl.s_xf, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, nullptr,
-                                                                   pf, 3, pl.ry_f, e->d_tw);
-  if (pl.s_yz > 0) {
-    const int Hx = (1 << pf.logP[0]) / 2 + 1;
-    pair_yz_fn(pf.logP[2])<<<Hx, PF_THREADS, pl.s_yz, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf,
-                                                                   e->d_tw);
-  } else {
-    pair_yfft_fn(-1)<<<pl.g_yf, PF_THREADS, pl.s_yf, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, 3,
-                                                                  pl.zc_f, e->d_tw);
-    pair_zmul_fn(true)<<<pl.g_z, PF_THREADS, pl.s_z, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, 3,
-                                                                  pl.tky, e->d_tw);
-    pair_yfft_fn(1)<<<pl.g_yi, PF_THREADS, pl.s_yi, e->stream>>>(e->d_mags, e->d_groups, src, stage, gate, pf, 3,
-                                                                 pl.zc_i, e->d_tw);
+// The passes of one evaluation of `n` pairs of one shape (PairPlan::shape) and
+// of distinct destinations: each plan's item gives the source and destination
+// slots, where the field goes (3 x N of the destination) and whether it is added.
+mpx_status launch_pair_fft(mpx_engine* e, const PairPlan* const* pl, int n, int stage, int gate) {
+  for (int i0 = 0; i0 < n; i0 += PAIR_BATCH) {
+    const int nb = std::min(PAIR_BATCH, n - i0), nt = pl[i0]->threads;
+    PairBatch b{};
+    PairItem g{};  // the largest grids
+    int xf = 0, yf = 0, z = 0, yi = 0, xi = 0, yz = 0, hx = 0;
+    for (int i = 0; i < nb; ++i) {
+      const PairPlan& p = *pl[i0 + i];
+      b.p[i] = p.it;
+      g.g_xf = std::max(g.g_xf, p.it.g_xf);
+      g.g_yf = std::max(g.g_yf, p.it.g_yf);
+      g.g_z = std::max(g.g_z, p.it.g_z);
+      g.g_yi = std::max(g.g_yi, p.it.g_yi);
+      g.g_xi = std::max(g.g_xi, p.it.g_xi);
+      xf = std::max(xf, p.s_xf);
+      yf = std::max(yf, p.s_yf);
+      z = std::max(z, p.s_z);
+      yi = std::max(yi, p.s_yi);
+      xi = std::max(xi, p.s_xi);
+      yz = std::max(yz, p.s_yz);
+      hx = std::max(hx, (1 << p.it.pf.logP[0]) / 2 + 1);
+    }
+    auto launch = [&](PairFn fn, int grid, int smem) {
+      return launch_pdl(fn, dim3(grid, nb), nt, smem, e->stream, e->d_mags, e->d_groups, stage, gate, b, e->d_tw);
+    };
+    CUDA_TRY(launch(pair_xfwd_fn(false), g.g_xf, xf));
+    if (yz > 0) {
+      CUDA_TRY(launch(pair_yz_fn(pl[i0]->it.pf.logP[2]), hx, yz));
+    } else {
+      CUDA_TRY(launch(pair_yfft_fn(-1), g.g_yf, yf));
+      CUDA_TRY(launch(pair_zmul_fn(true), g.g_z, z));
+      CUDA_TRY(launch(pair_yfft_fn(1), g.g_yi, yi));
+    }
+    CUDA_TRY(launch(pair_xinv_fn(), g.g_xi, xi));
+    e->launches += yz > 0 ? 3 : 5;
   }
-  pair_xinv_fn()<<<pl.g_xi, PF_THREADS, pl.s_xi, e->stream>>>(e->d_mags, e->d_groups, dst, stage, gate, pf, pl.ry_i, add,
-                                                           out, e->d_tw);
-  e->launches += pl.launches();
+  return MPX_OK;
 }
 
 mpx_status rebuild_pairs(mpx_engine* e) {
@@ -1243,7 +1269,6 @@ mpx_status rebuild_pairs(mpx_engine* e) {
         if ((long long)A->dev.N * B->dev.N >= STRAY_FFT_MIN_INTERACTIONS && pair_fft_lengths(A->dev.n, B->dev.n, logP)) {
           MPX_TRY(build_pair_fft(e, A, B->dev.n, B->dev.o, g, p.plan));
           p.fft = true;
-          p.launches = p.plan.launches();
           e->pairs.push_back(p);
           is_dst[b] = true;
           continue;
@@ -1280,21 +1305,42 @@ mpx_status rebuild_pairs(mpx_engine* e) {
   return MPX_OK;
 }
 
-// Stray fields of the sources of `dst` (all destinations when dst < 0) for `stage`.
+// Stray fields of the sources of `dst` (all destinations when dst < 0) for
+// `stage`: in rounds, the r-th source of every destination together.
 mpx_status launch_pairs(mpx_engine* e, int dst, int stage, int gate) {
-  std::vector<int> seen;
-  for (const auto& p : e->pairs) {
-    if (dst >= 0 && p.dst != dst) continue;
-    const bool add = std::find(seen.begin(), seen.end(), p.dst) != seen.end();
-    if (!add) seen.push_back(p.dst);
-    Magnet* B = get_mag(e, p.dst);
-    if (p.fft) {
-      launch_pair_fft(e, p.plan, p.src, p.dst, stage, gate, add ? 1 : 0, B->hstray);
-      continue;
+  std::vector<int> round(e->pairs.size(), -1);
+  std::unordered_map<int, int> seen;  // sources of a destination so far
+  int rounds = 0;
+  for (size_t i = 0; i < e->pairs.size(); ++i) {
+    if (dst >= 0 && e->pairs[i].dst != dst) continue;
+    round[i] = seen[e->pairs[i].dst]++;
+    rounds = std::max(rounds, round[i] + 1);
+  }
+  for (int r = 0; r < rounds; ++r) {
+    std::vector<PairPlan*> fft;
+    for (size_t i = 0; i < e->pairs.size(); ++i) {
+      if (round[i] != r) continue;
+      auto& p = e->pairs[i];
+      Magnet* B = get_mag(e, p.dst);
+      if (p.fft) {
+        p.plan.it.src = p.src;
+        p.plan.it.dst = p.dst;
+        p.plan.it.out = B->hstray;
+        p.plan.it.add = r > 0 ? 1 : 0;
+        fft.push_back(&p.plan);
+        continue;
+      }
+      k_stray_pair<<<(B->dev.N + 255) / 256, 256, 0, e->stream>>>(e->d_mags, e->d_groups, p.src, p.dst, p.tab, stage,
+                                                                  gate, r > 0 ? 1 : 0, B->hstray);
+      e->launches++;
     }
-    k_stray_pair<<<(B->dev.N + 255) / 256, 256, 0, e->stream>>>(e->d_mags, e->d_groups, p.src, p.dst, p.tab, stage,
-                                                                gate, add ? 1 : 0, B->hstray);
-    e->launches++;
+    std::stable_sort(fft.begin(), fft.end(), [](const PairPlan* x, const PairPlan* y) { return x->shape() < y->shape(); });
+    for (size_t i = 0; i < fft.size();) {
+      size_t j = i;
+      while (j < fft.size() && fft[j]->shape() == fft[i]->shape()) ++j;
+      MPX_TRY(launch_pair_fft(e, fft.data() + i, (int)(j - i), stage, gate));
+      i = j;
+    }
   }
   return MPX_OK;
 }
@@ -1784,6 +1830,20 @@ mpx_status eval_into(mpx_engine* e, Magnet* m, int q, float* out) {
   return check_launch(e, "eval");
 }
 
+// The side streams and their events, made when a batch first has several y/z
+// classes (outside a capture).
+mpx_status ensure_side_streams(mpx_engine* e) {
+  int classes = 0;
+  for (int c = 0; c < YZ_CLASSES; ++c) classes += e->n_kx_demag[c] > 0 ? 1 : 0;
+  if (classes < 2 || e->fork) return MPX_OK;
+  for (int k = 0; k < N_SIDE; ++k) {
+    if (!e->side[k]) CUDA_TRY(cudaStreamCreateWithFlags(&e->side[k], cudaStreamNonBlocking));
+    if (!e->join[k]) CUDA_TRY(cudaEventCreateWithFlags(&e->join[k], cudaEventDisableTiming));
+  }
+  CUDA_TRY(cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming));
+  return MPX_OK;
+}
+
 // One Runge-Kutta attempt for every running group (core/rungekutta.cpp:39-83).
 mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
   const int S = T.S;
@@ -1816,8 +1876,16 @@ mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
       e->launches++;
     }
     // stray fields of the stage states of the other magnets
+    const int64_t before_pairs = e->launches;
     MPX_TRY(launch_pairs(e, -1, s, 1));
+    e->pair_launches = (int)(e->launches - before_pairs);
     if (e->n_t_demag > 0) {
+      // The y/z classes of a batch run beside each other: each is a few waves of
+      // blocks, and one after the other every class leaves the SMs idle in its
+      // last wave and in the gap to the next.  The first class follows the x pass
+      // by programmatic launch; the others fork from it into side streams.  The
+      // 24-solve batch (z lengths 1 and 4): 18.38 -> 18.0 ms.
+      int last = -1, forked = 0;
       for (int c = 0; c < YZ_CLASSES; ++c)
         if (e->n_kx_demag[c] > 0) last = c;
       for (int c = 0; c < last; ++c) {
@@ -1847,20 +1915,6 @@ mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
       e->launches++;
     }
   }
-// The side streams and their events, made when a batch first has several y/z
-// classes (outside a capture).
-mpx_status ensure_side_streams(mpx_engine* e) {
-  int classes = 0;
-  for (int c = 0; c < YZ_CLASSES; ++c) classes += e->n_kx_demag[c] > 0 ? 1 : 0;
-  if (classes < 2 || e->fork) return MPX_OK;
-  for (int k = 0; k < N_SIDE; ++k) {
-    if (!e->side[k]) CUDA_TRY(cudaStreamCreateWithFlags(&e->side[k], cudaStreamNonBlocking));
-    if (!e->join[k]) CUDA_TRY(cudaEventCreateWithFlags(&e->join[k], cudaEventDisableTiming));
-  }
-  CUDA_TRY(cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming));
-  return MPX_OK;
-}
-
   if (!T.fsal) {
     if (e->n_t_demag > 0) {
       combine_fn()<<<e->n_t_demag, 256, 0, e->stream>>>(e->d_mags, e->d_groups, e->d_t_demag, S, 1);
@@ -1892,17 +1946,12 @@ mpx_status ensure_side_streams(mpx_engine* e) {
 mpx_status prepare_run(mpx_engine* e, int method) {
   if (e->pairs_dirty) MPX_TRY(rebuild_pairs(e));
   if (e->tables_dirty) MPX_TRY(rebuild_tables(e));
+  MPX_TRY(ensure_side_streams(e));
   MPX_TRY(upload_tableau(e, method));
   return MPX_OK;
 }
 
 // Captures one attempt (from `first_stage` on) as an executable graph.
-      // The y/z classes of a batch run beside each other: each is a few waves of
-      // blocks, and one after the other every class leaves the SMs idle in its
-      // last wave and in the gap to the next.  The first class follows the x pass
-      // by programmatic launch; the others fork from it into side streams.  The
-      // 24-solve batch (z lengths 1 and 4): 18.38 -> 18.0 ms.
-      int last = -1, forked = 0;
 // Captures one attempt into *out.  When *out already holds an attempt graph of
 // the same shape (the same kernels in the same order; a solve that arrives or
 // finishes changes only grid sizes and table pointers), the executable graph
@@ -1944,9 +1993,7 @@ int attempt_launches(const mpx_engine* e, const TableauDev& T, int first_stage) 
   int nyz = 0;
   for (int c = 0; c < YZ_CLASSES; ++c) nyz += e->n_kx_demag[c] > 0 ? 1 : 0;
   nyz += e->split.launches();
-  int npair = 0;
-  for (const auto& p : e->pairs) npair += p.launches;
-  MPX_TRY(ensure_side_streams(e));
+  const int npair = e->pair_launches;
   int per = 1 + npair * ns + 2 * e->samp_magnets;  // controller, stray-field pairs, samples
   if (e->n_t_demag > 0) per += (2 + nyz) * ns + (T.fsal ? 0 : 1);
   if (e->n_t_local > 0) per += ns + (ns - (first_stage == 0 ? 1 : 0)) + (T.fsal ? 0 : 1);
@@ -2209,6 +2256,11 @@ mpx_status mpx_engine_destroy(mpx_engine* e) {
   cudaStreamSynchronize(e->stream);
   if (e->pool) cudaMemPoolDestroy(e->pool);
   if (e->own) cudaStreamDestroy(e->own);
+  for (int k = 0; k < N_SIDE; ++k) {
+    if (e->side[k]) cudaStreamDestroy(e->side[k]);
+    if (e->join[k]) cudaEventDestroy(e->join[k]);
+  }
+  if (e->fork) cudaEventDestroy(e->fork);
   delete e;
   return MPX_OK;
 }
@@ -2256,11 +2308,6 @@ mpx_status mpx_engine_synchronize(mpx_engine* e) {
   CUDA_TRY(cudaStreamSynchronize(e->stream));
   return MPX_OK;
 }
-  for (int k = 0; k < N_SIDE; ++k) {
-    if (e->side[k]) cudaStreamDestroy(e->side[k]);
-    if (e->join[k]) cudaEventDestroy(e->join[k]);
-  }
-  if (e->fork) cudaEventDestroy(e->fork);
 
 mpx_status mpx_engine_set_world_bias(mpx_engine* e, const double b[3]) {
   if (!e || !b) return fail(MPX_ERR_INVALID, "null argument");
@@ -2808,7 +2855,13 @@ mpx_status mpx_stray_field(mpx_engine* e, int src, int dst_magnet, const int siz
     if (method == MPX_STRAY_FFT && pair_fft_lengths(A->dev.n, B->dev.n, logP)) {
       PairPlan* pl = nullptr;
       st = cached_pair_plan(e, A, B, g, &pl);
-      if (st == MPX_OK) launch_pair_fft(e, *pl, src, dst, 0, 0, 0, dout);
+      if (st == MPX_OK) {
+        pl->it.src = src;
+        pl->it.dst = dst;
+        pl->it.out = dout;
+        pl->it.add = 0;
+        st = launch_pair_fft(e, &pl, 1, 0, 0);
+      }
     } else {  // the direct sum (also the FFT method's form for pair grids beyond the FFT lengths)
       StrayTable tab;
       for (int ax = 0; ax < 3; ++ax) {

@@ -12,9 +12,10 @@
 namespace mpx {
 
 // ---- the pair grid of stray fields (pairfft.cuh)
-constexpr int PF_THREADS = 512;
-constexpr int PF_LR = 3;                              // log2 of the largest radix
-constexpr int PF_POINTS = (1 << PF_LR) * PF_THREADS;  // points of one transform group
+// Blocks of 256 threads with 8 values each (2048 points of a transform group), 512
+// where a length is 4096.
+constexpr int PF_THREADS = 512;  // at most
+constexpr int PF_LR = 3;         // log2 of the largest radix
 
 struct PairFft {
   float2* t;         // work spectrum (or, while it is made, the kernel spectrum)
@@ -24,6 +25,25 @@ struct PairFft {
   int win[3];   // first row of the output window per axis (n_A - 1)
   int nout[3];  // rows of the output window per axis (n_B)
   float scale;  // -mu0 / (Px Py Pz)
+};
+
+// One evaluation of a pair (or the transform of its table): source and
+// destination magnet slots (src -1: no gate), components, rows / columns per
+// block and number of blocks of each pass.
+struct PairItem {
+  PairFft pf;
+  int src, dst, ncomp;
+  int ry_f, zc_f, tky, zc_i, ry_i;
+  int g_xf, g_yf, g_z, g_yi, g_xi;
+  int add;           // accumulate into out (a later source of the destination)
+  const float* tab;  // the tabulated tensor (TABLE form)
+  float* out;
+};
+// The pairs of one launch (blockIdx.y): the pairs of a world take their passes
+// together, one source of every destination at a time.
+constexpr int PAIR_BATCH = 8;
+struct PairBatch {
+  PairItem p[PAIR_BATCH];
 };
 
 using XfwdFn = void (*)(const MagnetDev*, const GroupDev*, const Work*, int, int, const float*, const float2*);
@@ -74,15 +94,11 @@ __host__ __device__ constexpr int zcw_smem(int Pz) {
 }
 
 // pairs.cu: stray fields on the pair grid
-using PairXfwdFn = void (*)(const MagnetDev*, const GroupDev*, int, int, int, const float*, PairFft, int, int,
-                            const float2*);
-using PairYfftFn = void (*)(const MagnetDev*, const GroupDev*, int, int, int, PairFft, int, int, const float2*);
-using PairYzFn = void (*)(const MagnetDev*, const GroupDev*, int, int, int, PairFft, const float2*);
-using PairXinvFn = void (*)(const MagnetDev*, const GroupDev*, int, int, int, PairFft, int, int, float*, const float2*);
-PairXfwdFn pair_xfwd_fn(bool table);
-PairYfftFn pair_yfft_fn(int dir);
-PairYfftFn pair_zmul_fn(bool mul);
-PairYzFn pair_yz_fn(int logPz);
-PairXinvFn pair_xinv_fn();
+using PairFn = void (*)(const MagnetDev*, const GroupDev*, int, int, const PairBatch, const float2*);
+PairFn pair_xfwd_fn(bool table);
+PairFn pair_yfft_fn(int dir);
+PairFn pair_zmul_fn(bool mul);
+PairFn pair_yz_fn(int logPz);
+PairFn pair_xinv_fn();
 
 }  // namespace mpx

@@ -31,9 +31,12 @@
 //                    into the destination (zero outside its geometry)
 // KS is made once per pair by the first three passes over the table (six
 // components, no multiply).  All transforms are the shared-memory Stockham
-// FFTs of fft.cuh with radix-8 passes: 512 threads of 8 values (4096 points
-// per group) and at most 64 registers, so that two blocks share an SM (the
-// radix-16 form needed ~150 registers: one 8-warp block per SM).
+// FFTs of fft.cuh with radix-8 passes, 8 values per thread.  At the sizes of a
+// device (two 256 x 256 films: 257 blocks of the y/z pass, 3 columns each) the
+// passes are bound by latency, so the pairs of a world share their launches
+// (blockIdx.y), the passes are launched with programmatic dependent launch, and
+// blocks have 256 threads without a register cap (with 512 threads and 64
+// registers each pass spilled 300 - 1000 bytes per thread).
 #pragma once
 #include "launch.h"
 
@@ -43,23 +46,30 @@ namespace mpx {
 // `ncomp` = 6 components; else Ms m of the source magnet's state for `stage`
 // (zero outside its geometry).  Block: rows y0 .. y0 + ry - 1 of (c, z).
 template <bool TABLE>
-__global__ void __launch_bounds__(PF_THREADS, 2) k_pair_xfwd(const MagnetDev* __restrict__ mags,
-                                                          const GroupDev* __restrict__ groups, int src, int stage,
-                                                          int gate, const float* __restrict__ tab, PairFft pf,
-                                                          int ncomp, int ry, const float2* __restrict__ tw) {
+__global__ void __launch_bounds__(PF_THREADS, 1)
+    k_pair_xfwd(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, int stage, int gate,
+             const __grid_constant__ PairBatch batch, const float2* __restrict__ tw) {
   extern __shared__ float2 sm[];
   __shared__ MagnetDev MA;
   __shared__ GroupDev G;
+  pdl_trigger();
+  const PairItem& it = batch.p[blockIdx.y];
+  const PairFft& pf = it.pf;
+  if ((int)blockIdx.x >= it.g_xf || (!TABLE && !load_descs(MA, G, mags, groups, it.src, gate, stage))) {
+    pdl_wait();
+    return;
+  }
+  const int ncomp = it.ncomp, ry = it.ry_f;
+  const float* __restrict__ tab = it.tab;
   const int logPx = pf.logP[0], Px = 1 << logPx, cs = plen(Px);
   const int nxi = pf.nin[0], nyi = pf.nin[1], nzi = pf.nin[2];
   const int nyt = (nyi + ry - 1) / ry;
   const int yt = blockIdx.x % nyt, z = (blockIdx.x / nyt) % nzi, c = blockIdx.x / (nyt * nzi);
-  if (c >= ncomp) return;
-  if (!TABLE && !load_descs(MA, G, mags, groups, src, gate, stage)) return;
   const int y0 = yt * ry, nr = min(ry, nyi - y0);
   float2* D = sm;
   float2* tws = sm + ry * cs;
   load_twiddles<PF_LR>(tws, tw, logPx);
+  pdl_wait();  // the state is written by the previous pass
   const float* m = TABLE ? nullptr : stage_m(MA, G, stage);
   for (int e = threadIdx.x; e < (nr << logPx); e += blockDim.x) {
     const int r = e >> logPx, x = e & (Px - 1);
@@ -92,14 +102,21 @@ __global__ void __launch_bounds__(PF_THREADS, 2) k_pair_xfwd(const MagnetDev* __
 // window's rows out).  Block: zc consecutive columns of one (kx, c).  src >= 0:
 // the source magnet decides the group gate.
 template <int DIR>
-__global__ void __launch_bounds__(PF_THREADS, 2) k_pair_yfft(const MagnetDev* __restrict__ mags,
-                                                          const GroupDev* __restrict__ groups, int src, int stage,
-                                                          int gate, PairFft pf, int ncomp, int zc,
-                                                          const float2* __restrict__ tw) {
+__global__ void __launch_bounds__(PF_THREADS, 1)
+    k_pair_yfft(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, int stage, int gate,
+             const __grid_constant__ PairBatch batch, const float2* __restrict__ tw) {
   extern __shared__ float2 sm[];
   __shared__ MagnetDev MA;
   __shared__ GroupDev G;
-  if (src >= 0 && !load_descs(MA, G, mags, groups, src, gate, stage)) return;
+  pdl_trigger();
+  const PairItem& it = batch.p[blockIdx.y];
+  const PairFft& pf = it.pf;
+  if ((int)blockIdx.x >= (DIR < 0 ? it.g_yf : it.g_yi) ||
+      (it.src >= 0 && !load_descs(MA, G, mags, groups, it.src, gate, stage))) {
+    pdl_wait();
+    return;
+  }
+  const int ncomp = it.ncomp, zc = DIR < 0 ? it.zc_f : it.zc_i;
   const int logPy = pf.logP[1], Py = 1 << logPy, Pz = 1 << pf.logP[2], cs = plen(Py);
   const int zlo = DIR < 0 ? 0 : pf.win[2], nzc = DIR < 0 ? pf.nin[2] : pf.nout[2];
   const int nzt = (nzc + zc - 1) / zc;
@@ -108,6 +125,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) k_pair_yfft(const MagnetDev* __
   float2* D = sm;
   float2* tws = sm + zc * cs;
   load_twiddles<PF_LR>(tws, tw, logPy);
+  pdl_wait();  // the columns are written by the previous pass
   const size_t t0 = (((size_t)kx * ncomp + c) * Pz + z0) * Py;
   const size_t tleft = (size_t)((1 << pf.logP[0]) / 2 + 1) * ncomp * Pz * Py - t0;  // elements from T on (checked build)
   float2* __restrict__ T = pf.t + t0;
@@ -139,14 +157,20 @@ __global__ void __launch_bounds__(PF_THREADS, 2) k_pair_yfft(const MagnetDev* __
 // 3x3 product with the kernel spectrum, the inverse z FFT and the window's
 // planes back into T; without MUL (making the kernel spectrum) all Pz planes.
 template <bool MUL>
-__global__ void __launch_bounds__(PF_THREADS, 2) k_pair_zmul(const MagnetDev* __restrict__ mags,
-                                                          const GroupDev* __restrict__ groups, int src, int stage,
-                                                          int gate, PairFft pf, int ncomp, int tky,
-                                                          const float2* __restrict__ tw) {
+__global__ void __launch_bounds__(PF_THREADS, 1)
+    k_pair_zmul(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, int stage, int gate,
+             const __grid_constant__ PairBatch batch, const float2* __restrict__ tw) {
   extern __shared__ float2 sm[];
   __shared__ MagnetDev MA;
   __shared__ GroupDev G;
-  if (src >= 0 && !load_descs(MA, G, mags, groups, src, gate, stage)) return;
+  pdl_trigger();
+  const PairItem& it = batch.p[blockIdx.y];
+  const PairFft& pf = it.pf;
+  if ((int)blockIdx.x >= it.g_z || (it.src >= 0 && !load_descs(MA, G, mags, groups, it.src, gate, stage))) {
+    pdl_wait();
+    return;
+  }
+  const int ncomp = it.ncomp, tky = it.tky;
   const int Py = 1 << pf.logP[1], logPz = pf.logP[2], Pz = 1 << logPz, cs = plen(Pz);
   const int nyt = (Py + tky - 1) / tky;
   const int kx = blockIdx.x / nyt, ky0 = (blockIdx.x % nyt) * tky, nky = min(tky, Py - ky0);
@@ -154,6 +178,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) k_pair_zmul(const MagnetDev* __
   float2* D = sm;
   float2* tws = sm + ncomp * tky * cs;
   load_twiddles<PF_LR>(tws, tw, logPz);
+  pdl_wait();  // the columns are written by the previous pass
   const size_t tk0 = (size_t)kx * ncomp * Pz * Py + ky0;
   const int Hx = (1 << pf.logP[0]) / 2 + 1;
   const size_t tleft = (size_t)Hx * ncomp * Pz * Py - tk0;  // elements from Tk on (checked build)
@@ -213,18 +238,25 @@ __global__ void __launch_bounds__(PF_THREADS, 2) k_pair_zmul(const MagnetDev* __
 // k_pair_yfft<-1>, k_pair_zmul<true> and k_pair_yfft<+1> (same arithmetic
 // order: y, z, multiply, z, y) without their two round trips through T.
 template <int PZ>
-__global__ void __launch_bounds__(PF_THREADS, 2) k_pair_yz(const MagnetDev* __restrict__ mags,
-                                                        const GroupDev* __restrict__ groups, int src, int stage,
-                                                        int gate, PairFft pf, const float2* __restrict__ tw) {
+__global__ void __launch_bounds__(PF_THREADS, 1)
+    k_pair_yz(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, int stage, int gate,
+             const __grid_constant__ PairBatch batch, const float2* __restrict__ tw) {
   extern __shared__ float2 sm[];
   __shared__ MagnetDev MA;
   __shared__ GroupDev G;
-  if (!load_descs(MA, G, mags, groups, src, gate, stage)) return;
+  pdl_trigger();
+  const PairItem& it = batch.p[blockIdx.y];
+  const PairFft& pf = it.pf;
+  if ((int)blockIdx.x >= (1 << pf.logP[0]) / 2 + 1 || !load_descs(MA, G, mags, groups, it.src, gate, stage)) {
+    pdl_wait();
+    return;
+  }
   const int kx = blockIdx.x;
   const int logPy = pf.logP[1], Py = 1 << logPy, cs = plen(Py);
   float2* D = sm;  // column (z, c) at D + (3 z + c) cs
   float2* tws = sm + 3 * PZ * cs;
   load_twiddles<PF_LR>(tws, tw, logPy);
+  pdl_wait();  // the spectrum is written by k_pair_xfwd
   float2* __restrict__ Tk = pf.t + (size_t)kx * 3 * PZ * Py;  // [c][z][y]
   const size_t tleft = (size_t)((1 << pf.logP[0]) / 2 + 1 - kx) * 3 * PZ * Py;  // elements from Tk on (checked build)
   const int nzi = pf.nin[2], nyi = pf.nin[1];
@@ -285,24 +317,31 @@ __global__ void __launch_bounds__(PF_THREADS, 2) k_pair_yz(const MagnetDev* __re
 // rest by Hermitian symmetry, inverse FFT; x of the window, scaled, into
 // `out` (3 x N_B, component-major; added with `add`), zero outside the
 // destination's geometry.  Block: rows y0 .. y0 + ry - 1 of (c, z).
-static __global__ void __launch_bounds__(PF_THREADS, 2) k_pair_xinv(const MagnetDev* __restrict__ mags,
-                                                          const GroupDev* __restrict__ groups, int dst, int stage,
-                                                          int gate, PairFft pf, int ry, int add,
-                                                          float* __restrict__ out, const float2* __restrict__ tw) {
+static __global__ void __launch_bounds__(PF_THREADS, 1)
+    k_pair_xinv(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, int stage, int gate,
+             const __grid_constant__ PairBatch batch, const float2* __restrict__ tw) {
   extern __shared__ float2 sm[];
   __shared__ MagnetDev MB;
   __shared__ GroupDev G;
-  if (!load_descs(MB, G, mags, groups, dst, gate, stage)) return;
+  pdl_trigger();
+  const PairItem& it = batch.p[blockIdx.y];
+  const PairFft& pf = it.pf;
+  if ((int)blockIdx.x >= it.g_xi || !load_descs(MB, G, mags, groups, it.dst, gate, stage)) {
+    pdl_wait();
+    return;
+  }
+  const int ry = it.ry_i, add = it.add;
+  float* __restrict__ out = it.out;
   const int logPx = pf.logP[0], Px = 1 << logPx, Hx = Px / 2 + 1, cs = plen(Px);
   const int Py = 1 << pf.logP[1], Pz = 1 << pf.logP[2];
   const int nxo = pf.nout[0], nyo = pf.nout[1], nzo = pf.nout[2];
   const int nyt = (nyo + ry - 1) / ry;
   const int yt = blockIdx.x % nyt, zz = (blockIdx.x / nyt) % nzo, c = blockIdx.x / (nyt * nzo);
-  if (c >= 3) return;
   const int y0 = yt * ry, nr = min(ry, nyo - y0);
   float2* D = sm;
   float2* tws = sm + ry * cs;
   load_twiddles<PF_LR>(tws, tw, logPx);
+  pdl_wait();  // the spectrum is written by the y/z pass
   const size_t t0 = ((size_t)c * Pz + pf.win[2] + zz) * Py + pf.win[1] + y0;
   const size_t tleft = (size_t)Hx * 3 * Pz * Py - t0;  // elements from T on (checked build)
   const float2* __restrict__ T = pf.t + t0;

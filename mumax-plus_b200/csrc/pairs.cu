@@ -4,10 +4,10 @@
 
 namespace mpx {
 
-PairXfwdFn pair_xfwd_fn(bool table) { return table ? k_pair_xfwd<true> : k_pair_xfwd<false>; }
-PairYfftFn pair_yfft_fn(int dir) { return dir < 0 ? k_pair_yfft<-1> : k_pair_yfft<1>; }
-PairYfftFn pair_zmul_fn(bool mul) { return mul ? k_pair_zmul<true> : k_pair_zmul<false>; }
-PairYzFn pair_yz_fn(int logPz) {
+PairFn pair_xfwd_fn(bool table) { return table ? k_pair_xfwd<true> : k_pair_xfwd<false>; }
+PairFn pair_yfft_fn(int dir) { return dir < 0 ? k_pair_yfft<-1> : k_pair_yfft<1>; }
+PairFn pair_zmul_fn(bool mul) { return mul ? k_pair_zmul<true> : k_pair_zmul<false>; }
+PairFn pair_yz_fn(int logPz) {
   switch (logPz) {
     case 0: return k_pair_yz<1>;
     case 1: return k_pair_yz<2>;
@@ -15,6 +15,6 @@ PairYzFn pair_yz_fn(int logPz) {
     default: return k_pair_yz<8>;
   }
 }
-PairXinvFn pair_xinv_fn() { return k_pair_xinv; }
+PairFn pair_xinv_fn() { return k_pair_xinv; }
 
 }  // namespace mpx
