@@ -16,7 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
-UNITS = ["engine", "xpass", "yz", "yzwarp", "yzlong", "thick", "pairs"]
+UNITS = ["xthree", "xpass", "yz", "engine", "yzwarp", "yzlong", "yzthree", "thick", "pairs"]
 OUT = os.path.join(HERE, "libmpx.so")
 OUT_CHECKED = os.path.join(HERE, "libmpx_checked.so")
 

@@ -2,8 +2,10 @@
 // the first bad index is one device variable).
 #include "engine.cu"
 #include "xpass.cu"
+#include "xthree.cu"
 #include "yz.cu"
 #include "yzwarp.cu"
 #include "yzlong.cu"
+#include "yzthree.cu"
 #include "thick.cu"
 #include "pairs.cu"

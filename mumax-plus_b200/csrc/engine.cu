@@ -68,6 +68,13 @@ int ilog2(int v) {
 
 // padded FFT length: smallest power of two >= 2n-1 (1 when n == 1)
 int padded(int n) { return n == 1 ? 1 : 1 << ilog2(2 * n - 1); }
+// the length 3 2^k (96 .. 768) >= 2n-1 where it is below the power of two, else that
+int padded3(int n, int from) {
+  for (int p = from; p <= 768; p *= 2)
+    if (p >= 2 * n - 1 && p < padded(n)) return p;
+  return padded(n);
+}
+int log_length(int P) { return P % 3 ? ilog2(P) : LOG_THREE + ilog2(P / 96); }
 
 constexpr int MAX_FFT = 4096;
 constexpr int SMEM_MAX = 227 * 1024;
@@ -531,14 +538,34 @@ int yzw_threads_of(int Pz) { return Pz == 16 ? 384 : 256; }
 int yz_smem_of(int nz, int nkx, int Py, int Pz) {
   return (nkx * 3 * nz * (yz_warp(Py) || yz_pair(Py, Pz) ? qlen(Py) : plen(Py)) + Py) * (int)sizeof(float2);
 }
+bool split_warp(int Py, int Pz);
+// FFT lengths of a magnet of n cells per axis.  From THREE_MIN_CELLS cells on, along
+// x and y the lengths 384 and 768 (x: the warp rows; shorter rows are Stockham passes
+// of powers of two), and 96 .. 768 (y), where they are shorter; all powers of two with
+// the tensor-core y transforms and on the block-wide split path.  300 x 180 x 3 cells
+// (768 x 384 for 1024 x 512): 10.56 -> 9.78 ms per 38 attempts; 80 x 80 x 40 (y 192 for
+// 256): 15.3 -> 12.6; 437 x 291 x 2 energy density 63.3 -> 59.9 us.  Smaller magnets are
+// bound by latency, and in a batch the further launch classes cost more than they
+// save: 24 solves of up to 131,000 cells 18.0 -> 18.2 ms, their first pass 18.6 ->
+// 20.4 ms (larger graphs to instantiate).
+constexpr int64_t THREE_MIN_CELLS = 150000;
+void plan_lengths(const int n[3], bool pow2, int P[3]) {
+  for (int a = 0; a < 3; ++a) P[a] = padded(n[a]);
+  if (pow2 || (int64_t)n[0] * n[1] * n[2] < THREE_MIN_CELLS) return;
+  P[0] = padded3(n[0], 384);
+  const int y = padded3(n[1], 96);
+  if (P[2] <= 16 || split_warp(y, P[2])) P[1] = y;
+}
 int yz_smem(const Magnet* m) { return yz_smem_of(m->dev.n[2], m->nkx, m->P[1], m->P[2]); }
-// y/z class of a magnet: 20 + log2 Pz for the warp-pair pass of y length 2048
+// y/z class of a magnet: 24 + log2 Pz for the y lengths 96, 192 and 384, 29 + log2 Pz
+// for 768, 20 + log2 Pz for the warp-pair pass of y length 2048
 // (z lengths up to 8), 15 + log2 Pz for the warp-column pass of y length 1024,
 // 10 + log2 Pz for y lengths 64 .. 512, else log2 Pz, plus 5 for y transforms
 // longer than 2048 (which need the radix-16 form).  The FFT plan of a magnet
 // depends on its own lengths only, so it computes the same alone and in any
 // batch.
 int yz_class(const Magnet* m) {
+  if (m->P[1] % 3 == 0) return (m->P[1] == 768 ? 29 : 24) + ilog2(m->P[2]);
   if (yz_pair(m->P[1], m->P[2])) return 20 + ilog2(m->P[2]);
   if (m->P[1] == 1024) return 15 + ilog2(m->P[2]);
   if (yz_warp(m->P[1])) return 10 + ilog2(m->P[2]);
@@ -547,6 +574,7 @@ int yz_class(const Magnet* m) {
 constexpr int YZ_THREADS = 384;
 // threads per block of a y/z launch class
 int yz_threads(int cls) {
+  if (cls >= 24) return yzw_threads_of(1 << ((cls - 24) % 5));
   if (cls >= 20) return YZP_THREADS;
   return cls >= 10 ? yzw_threads_of(1 << ((cls - 10) % 5)) : YZ_THREADS;
 }
@@ -563,15 +591,15 @@ int yz_threads(int cls) {
 // same results alone and in any batch).
 int even_rows(int t, int ny) { return ny <= 1 ? 1 : std::max(2, t & ~1); }
 int choose_ty(int ny, int len) {
-  const int t = len == 1024 ? 8 : len == 512 ? 16 : len > 1024 ? 4 : std::min(TY_MAX, std::max(1, 4096 / len));
+  const int t = len == 1024 || len == 768 ? 8 : len == 512 || len == 384 ? 16 : len > 1024 ? 4 : std::min(TY_MAX, std::max(1, 4096 / len));
   return even_rows(std::max(1, std::min(t, ny)), ny);
 }
 int choose_nkx(int nz, int Py, int Pz, int Fh) {
   // warp pairs (y length 2048): up to 12 columns, two per pair of the 6 pairs
   if (yz_pair(Py, Pz)) return std::max(1, std::min(Fh, 12 / (3 * nz)));
   // warp columns (y lengths 64 .. 1024): 32 values per thread, one 1024-value unit per warp
-  const int pts = yz_warp(Py) ? 32 * yzw_threads_of(Pz) : YZ_VPT * YZ_THREADS;
-  return std::max(1, std::min(Fh, pts / (3 * nz * Py)));
+  if (yz_warp(Py)) return std::max(1, std::min(Fh, yzw_threads_of(Pz) / 32 * (1024 / Py) / (3 * nz)));
+  return std::max(1, std::min(Fh, YZ_VPT * YZ_THREADS / (3 * nz * Py)));
 }
 
 // Split path: the warp-column forms at the lengths their transforms cover.  At
@@ -664,7 +692,7 @@ SplitLaunch split_of(const Magnet* m) {
 mpx_status launch_yz(mpx_engine* e, int cls, const Work* work, int n, int smem, bool one, int stage, int gate,
                      cudaStream_t side = nullptr) {
   if (n <= 0) return MPX_OK;
-  const YzFn fn = cls >= 15 ? yz_long_fn(cls) : cls >= 10 ? yz_warp_fn(cls, one) : yz_block_fn(cls);
+  const YzFn fn = cls >= 24 ? yz_three_fn(cls, one) : cls >= 15 ? yz_long_fn(cls) : cls >= 10 ? yz_warp_fn(cls, one) : yz_block_fn(cls);
   if (side)  // beside another class, after the whole x pass
     fn<<<n, yz_threads(cls), smem, side>>>(e->d_mags, e->d_groups, work, stage, gate, e->d_tw);
   else
@@ -689,6 +717,7 @@ int x_threads(const Magnet* m) {
 XForm x_form_of(const Magnet* m, int nt) {
   XForm f;
   f.pair = m->P[0] == 2048;
+  f.three = m->P[0] % 3 == 0;
   f.mask = (m->dev.terms & FLAG_LEAN) && !m->dev.fast;
   f.one = m->P[0] <= 512 && 32 * (m->ty + (m->ty + 1) / 2) <= nt;
   return f;
@@ -833,7 +862,7 @@ mpx_status rebuild_tables(mpx_engine* e) {
   // comes and goes with it would instantiate the attempt graphs anew each time
   // (batches lost 4 %)
   const int ngroups = (int)std::count_if(e->groups.begin(), e->groups.end(), [](const auto& g) { return g != nullptr; });
-  e->x_form = XForm();
+  if (ngroups <= 1) e->x_form = XForm();  // (a form of several groups' launches stays, as the classes below)
   e->x_form.one = ngroups == 1;
   for (int c = 0; c < YZ_CLASSES; ++c) e->yz_one[c] = e->yz_one[c] && ngroups == 1;
   bool any512 = false;
@@ -841,8 +870,9 @@ mpx_status rebuild_tables(mpx_engine* e) {
     const XForm f = x_form_of(pr.first, e->nt_x);
     e->x_form.pair = e->x_form.pair || f.pair;
     e->x_form.mask = e->x_form.mask || f.mask;
+    e->x_form.three = e->x_form.three || f.three;
     e->x_form.one = e->x_form.one && f.one;
-    any512 = any512 || pr.first->P[0] == 512;
+    any512 = any512 || pr.first->P[0] == 512 || pr.first->P[0] == 384;
   }
   e->x_form.one = e->x_form.one && any512;
   // each table: holes for the magnets that left (or whose lists changed), the
@@ -872,6 +902,14 @@ mpx_status rebuild_tables(mpx_engine* e) {
         if (!pr.second->empty() && !T.place.count(pr.first->uid)) T.add(pr.first->uid, pr.first->ver, *pr.second);
     }
     while (!T.items.empty() && T.items.back().mag < 0) T.items.pop_back();  // trailing holes
+    // In an engine of several groups a y/z class stays in the attempt graphs once
+    // it was used (with one hole when empty): solves come and go, and another
+    // set of kernels would instantiate the graphs anew, 1.3 ms each time against
+    // about 2 us per stage for the empty class beside the others.
+    if (t >= mpx_engine::TT_YZ0 && ngroups > 1 && T.items.empty() && T.cap > 0) {
+      T.items.push_back(Work{-1, 0, 0, 0});
+      T.dirty(0, 1);
+    }
     const int used = (int)T.items.size();
     if (used > T.cap) {  // grow: a new device array, everything uploaded
       const int nc = std::max({used, 2 * T.cap, 64});
@@ -931,7 +969,7 @@ mpx_status rebuild_tables(mpx_engine* e) {
   std::vector<long long> sig;
   for (int t = 0; t < NT; ++t) sig.insert(sig.end(), {(long long)(uintptr_t)e->tt[t].dev, (long long)e->tt[t].items.size()});
   for (int c = 0; c < YZ_CLASSES; ++c) sig.insert(sig.end(), {e->smem_yz[c], e->yz_one[c]});
-  sig.insert(sig.end(), {e->smem_x, e->nt_x, e->x_form.pair, e->x_form.mask, e->x_form.one, e->split.smem_y, e->split.smem_z, e->split.max_py,
+  sig.insert(sig.end(), {e->smem_x, e->nt_x, e->x_form.pair, e->x_form.mask, e->x_form.one, e->x_form.three, e->split.smem_y, e->split.smem_z, e->split.max_py,
                          e->split.max_pz, e->split.smem_yw, e->split.smem_zw});
   e->tables_dirty = false;
   if (e->tables_valid && sig == e->tables_sig) return MPX_OK;
@@ -959,7 +997,7 @@ constexpr long long STRAY_FFT_MIN_INTERACTIONS = 1LL << 22;
 // pool that has to grow for a larger one costs more than the launches saved: the
 // first image of a 400 x 400 x 4 film 0.7 -> 2.2 ms), one at a time up to
 // NEWELL_LATTICE_MAX, none (the point-by-point sum) beyond.
-constexpr int64_t NEWELL_LATTICE_ALL = 16LL << 20, NEWELL_LATTICE_MAX = 1LL << 30;
+constexpr int64_t NEWELL_LATTICE_ALL = 64LL << 20, NEWELL_LATTICE_MAX = 1LL << 30;
 int newell_lattice(const KernelGeom& g, const int K[3], const int O[3], int ncomp, NewellLattice* L) {
   int64_t n = 8;
   for (int a = 0; a < 3; ++a) {
@@ -1663,10 +1701,10 @@ mpx_status setup_magnet(mpx_engine* e, Magnet* m, const mpx_magnet_desc* d, bool
   const int N = D.N;
   // demag plan
   m->demag = (D.terms & TERM_DEMAG) != 0;
+  plan_lengths(D.n, e->dft_mode == MPX_DFT_TF32X3, m->P);
   for (int a = 0; a < 3; ++a) {
-    m->P[a] = padded(D.n[a]);
     D.P[a] = m->P[a];
-    D.logP[a] = ilog2(m->P[a]);
+    D.logP[a] = log_length(m->P[a]);
   }
   D.Fh = m->P[0] / 2 + 1;
   D.kcomp = (m->P[2] == 1) ? 4 : 6;
@@ -1698,13 +1736,13 @@ mpx_status setup_magnet(mpx_engine* e, Magnet* m, const mpx_magnet_desc* d, bool
   }
   // field buffers (9 x 3N floats) and spectrum
   size_t fbytes = sizeof(float) * 9 * 3 * (size_t)N;
-  if (!old_fields) {
+  if (!old_fields && !m->probe) {  // (a probe grid has no state)
     MPX_TRY(dalloc(e, nullptr, (void**)&old_fields, fbytes));
     CUDA_TRY(cudaMemsetAsync(old_fields, 0, fbytes, e->stream));
     m->fields_bytes = (int64_t)fbytes;
   }
   m->fields = old_fields;
-  for (int b = 0; b < 9; ++b) D.buf[b] = old_fields + (size_t)b * 3 * N;
+  for (int b = 0; b < 9; ++b) D.buf[b] = old_fields ? old_fields + (size_t)b * 3 * N : nullptr;
   const size_t sbytes = sizeof(float2) * (size_t)D.Fh * 3 * D.n[1] * D.n[2];  // S[kx][c][z][y]
   if (m->demag && !old_spec) {
     MPX_TRY(dalloc(e, nullptr, (void**)&old_spec, sbytes));
@@ -1774,6 +1812,7 @@ mpx_status setup_magnet(mpx_engine* e, Magnet* m, const mpx_magnet_desc* d, bool
 mpx_status upload_tableau(mpx_engine* e, int method) {
   TableauDev t = make_tableau(method);
   CUDA_TRY(upload_tableau_symbol(t, e->stream));
+  if (e->x_form.three) CUDA_TRY(upload_tableau_three(t, e->stream));
   e->tab_method = method;
   return MPX_OK;
 }
@@ -2151,27 +2190,34 @@ mpx_status mpx_engine_create(int device, mpx_engine** out) {
     CUDA_TRY(cudaMemPoolSetAttribute(e->pool, cudaMemPoolAttrReleaseThreshold, &keep));
   }
   // twiddle table exp(-2 pi i k / 4096), computed in FP64
-  std::vector<float2> tw(TW_N);
+  std::vector<float2> tw(TW_N + TW3_N);
   for (int k = 0; k < TW_N; ++k) {
     const double a = -2.0 * M_PI * k / TW_N;
     tw[k] = make_float2((float)std::cos(a), (float)std::sin(a));
   }
-  CUDA_TRY(cudaMalloc(&e->d_tw, sizeof(float2) * TW_N));
-  CUDA_TRY(cudaMemcpy(e->d_tw, tw.data(), sizeof(float2) * TW_N, cudaMemcpyHostToDevice));
+  for (int k = 0; k < TW3_N; ++k) {
+    const double a = -2.0 * M_PI * k / TW3_N;
+    tw[TW_N + k] = make_float2((float)std::cos(a), (float)std::sin(a));
+  }
+  CUDA_TRY(cudaMalloc(&e->d_tw, sizeof(float2) * tw.size()));
+  CUDA_TRY(cudaMemcpy(e->d_tw, tw.data(), sizeof(float2) * tw.size(), cudaMemcpyHostToDevice));
   CUDA_TRY(cudaMalloc(&e->d_red, sizeof(double) * 3 * 1024));
   CUDA_TRY(cudaMalloc(&e->d_redout, sizeof(double) * 4));  // 3 reduction results, or the 4 of k_min_final
   // large dynamic shared memory and the max-shared carveout for the FFT kernels
   std::vector<const void*> fft_kernels;
-  for (int f = 0; f < 6; ++f) {  // the forms of the x passes (warp pairs and one row per warp exclude each other)
+  for (int f = 0; f < 10; ++f) {  // the forms of the x passes
     XForm xf;
     xf.pair = f >> 1 == 1;
-    xf.one = f >> 1 == 2;
+    xf.one = f >> 1 == 2 || f >> 1 == 4;
+    xf.three = f >> 1 >= 3;
     xf.mask = f & 1;
     fft_kernels.push_back((const void*)xfwd_fn(f & 1, xf));
     fft_kernels.push_back((const void*)xinv_fn(xf));
   }
   fft_kernels.push_back((const void*)yz_warp_fn(10, true));
   fft_kernels.push_back((const void*)yz_warp_fn(12, true));
+  fft_kernels.push_back((const void*)yz_three_fn(24, true));
+  fft_kernels.push_back((const void*)yz_three_fn(26, true));
   for (int pair = 0; pair < 2; ++pair) {
     fft_kernels.push_back((const void*)pair_xfwd_fn(pair));
     fft_kernels.push_back((const void*)pair_zmul_fn(pair));
@@ -2180,7 +2226,7 @@ mpx_status mpx_engine_create(int device, mpx_engine** out) {
   fft_kernels.push_back((const void*)pair_xinv_fn());
   for (int l = 0; l < 4; ++l) fft_kernels.push_back((const void*)pair_yz_fn(l));
   for (int c = 0; c < YZ_CLASSES; ++c)
-    fft_kernels.push_back((const void*)(c >= 15 ? yz_long_fn(c) : c >= 10 ? yz_warp_fn(c, false) : yz_block_fn(c)));
+    fft_kernels.push_back((const void*)(c >= 24 ? yz_three_fn(c, false) : c >= 15 ? yz_long_fn(c) : c >= 10 ? yz_warp_fn(c, false) : yz_block_fn(c)));
   fft_kernels.push_back((const void*)ycw_fn(-1));
   fft_kernels.push_back((const void*)ycw_fn(1));
   fft_kernels.push_back((const void*)zcw_fn());
@@ -2618,12 +2664,12 @@ mpx_status mpx_magnet_bytes(const mpx_magnet_desc* d, int64_t* resident, int64_t
   const int64_t L = (int64_t)d->lut_regions * (d->lut_regions - 1) / 2;
   if (L > 0) res += 4 * L * ((d->inter_exchange_lut ? 1 : 0) + (d->scale_exchange_lut ? 1 : 0));
   const bool demag = d->enable_demag && !scalar_zero(d->msat);
-  const int ty = choose_ty(d->size[1], demag ? padded(d->size[0]) : d->size[0]);
+  int P[3];
+  plan_lengths(d->size, false, P);
+  const int ty = choose_ty(d->size[1], demag ? P[0] : d->size[0]);
   res += (int64_t)sizeof(Work) * d->size[2] * ((d->size[1] + ty - 1) / ty);
   int64_t tr = 12 * N;  // initial random state (engine scratch)
   if (demag) {
-    int P[3];
-    for (int a = 0; a < 3; ++a) P[a] = padded(d->size[a]);
     const int64_t Fh = P[0] / 2 + 1;
     const int kc = (P[2] == 1) ? 4 : 6;
     res += 8 * Fh * 3 * d->size[1] * d->size[2];                 // spectrum S[kx][c][z][y]

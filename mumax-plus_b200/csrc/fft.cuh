@@ -23,6 +23,8 @@ namespace mpx {
 
 constexpr int TW_LOG = 12;  // twiddle table covers transforms up to 4096 points
 constexpr int TW_N = 1 << TW_LOG;
+// lengths 3 2^k (96 .. 768): their own table exp(-2 pi i k / 3072) behind it
+constexpr int TW3_N = 3072;
 
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
@@ -104,6 +106,31 @@ __device__ __forceinline__ void bfly(float2 e, float2 o, float2& lo, float2& hi)
     lo = pfma(make_float2(c, c), u, e);
     hi = pfma(make_float2(-c, -c), u, e);
   }
+}
+
+// The same for rotations by M 24ths of a turn (M < 12), of the lengths 3 2^k.
+template <int DIR, int M>
+__device__ __forceinline__ void bfly24(float2 e, float2 o, float2& lo, float2& hi) {
+  if constexpr (M % 3 == 0 && M != 3 && M != 9) {
+    bfly<DIR, M * 4 / 3>(e, o, lo, hi);  // 0 or a quarter turn
+  } else {
+    constexpr bool by_cos = M <= 3 || M >= 9;
+    // distance of the angle from the nearest multiple of a half turn (by_cos) or quarter turn: 1, 2 or 3 24ths
+    constexpr int d = M <= 3 ? M : M >= 9 ? 12 - M : M < 6 ? 6 - M : M - 6;
+    constexpr float tn = d == 1 ? 0.267949192431122706473f : d == 2 ? 0.577350269189625764509f : 1.0f;
+    constexpr float sc = d == 1 ? 0.965925826289068286749f : d == 2 ? 0.866025403784438646764f : 0.707106781186547524401f;
+    constexpr float t = DIR * (M > 6 ? -tn : tn), c = by_cos ? (M >= 9 ? -sc : sc) : DIR * sc;
+    const float2 u = by_cos ? make_float2(__fmaf_rn(-t, o.y, o.x), __fmaf_rn(t, o.x, o.y))
+                            : make_float2(__fmaf_rn(t, o.x, -o.y), __fmaf_rn(t, o.y, o.x));
+    lo = pfma(make_float2(c, c), u, e);
+    hi = pfma(make_float2(-c, -c), u, e);
+  }
+}
+// e +- o exp(DIR 2 pi i K / N), K < N / 2, N a power of two up to 32 or 6, 12, 24
+template <int DIR, int K, int N>
+__device__ __forceinline__ void bfly_of(float2 e, float2 o, float2& lo, float2& hi) {
+  if constexpr (N % 3 == 0) bfly24<DIR, K * (24 / N)>(e, o, lo, hi);
+  else bfly<DIR, K * (32 / N)>(e, o, lo, hi);
 }
 
 // padded shared-memory index and padded column length
@@ -331,7 +358,7 @@ __device__ __forceinline__ void fft_many(float2* buf, int logL, int ncols, int c
 }
 
 // ------------------------------------------------ warp columns (four-step)
-// A transform of length L = 32 Q (Q = 2 .. 32) as Q x 32: with n = j + 32 r and
+// A transform of length L = 32 Q (Q = 2 .. 32, or 3, 6, 12, 24) as Q x 32: with n = j + 32 r and
 // k = s + Q t,  X[s + Q t] = sum_j W32^{j t} W_L^{j s} sum_r x[j + 32 r] W_Q^{r s}.
 // A warp takes W = 32 / Q columns together, 32 values per lane: lane j does the
 // inner Q-point DFTs over r of every column and the twiddles W_L^{j s}; one
@@ -345,8 +372,8 @@ __device__ __forceinline__ void fft_many(float2* buf, int logL, int ncols, int c
 __device__ __forceinline__ int qidx(int i) { return i + (i >> 5); }
 __host__ __device__ constexpr int qlen(int L) { return L + (L >> 5); }
 
-// Radix-2 decimation-in-time DFT of N register values (N = 1 .. 32),
-// unnormalised, natural order.  ZH: inputs N/2 .. N-1 are zero (never read;
+// Radix-2 decimation-in-time DFT of N register values (N = 1 .. 32 a power of two,
+// or 3, 6, 12, 24), unnormalised, natural order.  ZH: inputs N/2 .. N-1 are zero (never read;
 // the zeros stay zeros down the even / odd splits).  LO: only outputs
 // 0 .. N/2-1 are formed.
 template <int N, int DIR, bool ZH, bool LO>
@@ -355,7 +382,7 @@ struct DftZ {
   __device__ __forceinline__ static void combine(float2 (&v)[N], const float2 (&e)[N / 2], const float2 (&o)[N / 2]) {
     if constexpr (K < N / 2) {
       float2 hi;
-      bfly<DIR, K * (32 / N)>(e[K], o[K], v[K], hi);
+      bfly_of<DIR, K, N>(e[K], o[K], v[K], hi);
       if constexpr (!LO) v[K + N / 2] = hi;
       combine<K + 1>(v, e, o);
     }
@@ -385,6 +412,17 @@ struct DftZ<2, DIR, ZH, LO> {
   }
 };
 template <int DIR, bool ZH, bool LO>
+struct DftZ<3, DIR, ZH, LO> {  // the odd factor of 6, 12 and 24
+  __device__ __forceinline__ static void run(float2 (&v)[3]) {
+    constexpr float s = DIR * 0.866025403784438646764f;
+    const float2 t = padd(v[1], v[2]), d = psub(v[1], v[2]);
+    const float2 p = pfma(make_float2(-0.5f, -0.5f), t, v[0]);
+    v[0] = padd(v[0], t);
+    v[1] = make_float2(__fmaf_rn(-s, d.y, p.x), __fmaf_rn(s, d.x, p.y));
+    v[2] = make_float2(__fmaf_rn(s, d.y, p.x), __fmaf_rn(-s, d.x, p.y));
+  }
+};
+template <int DIR, bool ZH, bool LO>
 struct DftZ<1, DIR, ZH, LO> {
   __device__ __forceinline__ static void run(float2 (&)[1]) {}
 };
@@ -407,6 +445,15 @@ __device__ __forceinline__ void load_twq(float2* dst, const float2* __restrict__
 // half the latency of the transform where a small solve leaves the other warps
 // idle.
 //
+// The table of length L = 32 Q with Q = 3 .. 24 a multiple of 3, from tw3 (TW3_N entries).
+__device__ __forceinline__ void load_twq3(float2* dst, const float2* __restrict__ tw3, int Q) {
+  const int qm1 = Q - 1, step = TW3_N / (32 * Q);
+  for (int t = threadIdx.x; t < 32 * qm1; t += blockDim.x) {
+    const int j = t / qm1, s = t - j * qm1 + 1;
+    dst[t] = __ldg(&tw3[j * s * step]);
+  }
+}
+
 // Inner step of lane j for W = 32 / Q columns of length L = 32 Q held together:
 // v[c Q + r] = x_c[j + 32 r] (r < Q; with ZH the values r >= Q/2 are zero and
 // unread).  On return v[c Q + s] holds W_L^{j s} sum_r x_c[j + 32 r] W_Q^{r s}.
@@ -554,7 +601,7 @@ __device__ __forceinline__ void warp_rows(float2* buf, int nrows, int cs, const 
     for (int c = 0; c < W; ++c)
 #pragma unroll
       for (int r = 0; r < Q; ++r)
-        v[c * Q + r] = (c < nc && (!ZIN || r < Q / 2)) ? R[c * cs + lane + 33 * r] : make_float2(0.f, 0.f);
+        v[c * Q + r] = (c < nc && (!ZIN || 2 * r < Q)) ? R[c * cs + lane + 33 * r] : make_float2(0.f, 0.f);
     four_step_inner<Q, DIR, ZIN, W>(v, twq, lane);
     four_step_outer<Q, DIR, LO, W>(v, R, cs, nc, lane);
     if constexpr (Q == 32) {
@@ -580,7 +627,7 @@ __device__ __forceinline__ int xidx(int i, int sh) { return i + (i >> sh); }
 // 16 different 8-byte banks (the outer step of these lengths reads within one
 // row per half-warp).
 __host__ __device__ inline int xrow_stride(int L, int ty) {
-  if (L != 1024 && L != 512 && L != 2048) return xstride(L);
+  if (L != 1024 && L != 512 && L != 2048 && L % 3 != 0) return xstride(L);
   int slots = 1;
   while (slots < ty) slots <<= 1;
   return qlen(L) + (slots >= 16 ? 1 : 16 / slots);

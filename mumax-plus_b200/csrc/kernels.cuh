@@ -228,7 +228,8 @@ __device__ __forceinline__ int tile_log(int ty) { return ty <= 1 ? 0 : 32 - __cl
 // the registers and code of the shorter lengths).
 // ONE: 512-point rows one per warp, for launches of rows up to 512 points whose
 // tiles have no more rows than warps (see k_yzw).
-template <bool COMBINE, bool PAIR = false, bool ONE = false>
+// THREE: rows of 384 and 768 points (lengths 3 2^k) are compiled in.
+template <bool COMBINE, bool PAIR = false, bool ONE = false, bool THREE = false>
 __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups,
                                               const Work* __restrict__ work, int stage, int gate,
                                               const float* __restrict__ msrc_override,
@@ -244,17 +245,20 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __re
   }
   const int z = wk.z, y0 = wk.y0, ty = wk.ty;
   const int nx = M.n[0], ny = M.n[1], nz = M.n[2], N = M.N;
-  const int logL = M.logP[0], L = 1 << logL, cs = xrow_stride(L, ty);
-  if (!PAIR && logL == 11) return;  // 2048-point rows only in the PAIR form (the host never launches them here)
+  const int logL = M.logP[0], L = THREE ? M.P[0] : 1 << logL, cs = xrow_stride(L, ty);
+  // rows of the PAIR and THREE forms (the host never launches them elsewhere)
+  if ((!PAIR && logL == 11) || (!THREE && logL >= LOG_THREE)) return;
+  const bool three = THREE && logL >= LOG_THREE;
   const int nzrows = (ty + 1) >> 1;
   const float* src = msrc_override ? msrc_override : stage_m(M, G, stage);
   float* xs = M.buf[G.map[1]];
   const float* x0 = M.buf[G.map[0]];
   const int rowbase = nx * (y0 + ny * z);
   float2* tws = sm + (ty + nzrows) * cs;  // twiddles of length L
-  const bool wrow = (PAIR && logL == 11) || logL == 10 || logL == 9;  // 2048- / 1024- / 512-point rows: warp (pair) rows
+  const bool wrow = three || (PAIR && logL == 11) || logL == 10 || logL == 9;  // 2048- / 1024- / 512-point rows: warp (pair) rows
   const int sh = wrow ? 5 : 4;
-  if (wrow) load_twq(tws, tw, logL);
+  if (three) load_twq3(tws, tw + TW_N, L >> 5);
+  else if (wrow) load_twq(tws, tw, logL);
   else load_twiddles<3>(tws, tw, logL);
   __shared__ float s_cf[8];
   __shared__ const float* s_kp[8];
@@ -281,10 +285,10 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __re
   if ((nx & 3) == 0 && logLh >= 2 && !M.geom && !M.msat.p && s_al) {
     // four consecutive cells per thread with 16-byte loads and stores (no
     // geometry, uniform Ms; nx and so N a multiple of 4)
-    const int lq = logLh - 2;
-    const float ms = M.msat.u;
-    for (int e = threadIdx.x; e < (ty << lq); e += blockDim.x) {
-      const int yl = e >> lq, x = (e & ((1 << lq) - 1)) << 2;
+    const int lq = logLh - 2, nq = L >> 3;
+    const float ms = M.msat.u, rq = 1.0f / (float)nq;
+    for (int e = threadIdx.x; e < (THREE ? ty * nq : ty << lq); e += blockDim.x) {
+      const int yl = THREE ? tile_row(e, nq, rq) : e >> lq, x = (THREE ? e - yl * nq : e & ((1 << lq) - 1)) << 2;
       float4 r[3];
       const int i = rowbase + yl * nx + x;
       if (x < nx && cell_ok(N, i) && cell_ok(N, i + 3)) {
@@ -312,9 +316,11 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __re
       }
     }
   } else {
+  const int nh = THREE ? max(1, L >> 1) : 0;
+  const float rh = THREE ? 1.0f / (float)nh : 0.f;
 #pragma unroll 2
-  for (int e = threadIdx.x; e < (ty << logLh); e += blockDim.x) {
-    const int yl = e >> logLh, x = e & ((1 << logLh) - 1);
+  for (int e = threadIdx.x; e < (THREE ? ty * nh : ty << logLh); e += blockDim.x) {
+    const int yl = THREE ? tile_row(e, nh, rh) : e >> logLh, x = THREE ? e - yl * nh : e & ((1 << logLh) - 1);
     float3 Mv = f3(0, 0, 0);
     if (x < nx) {
       const int i = rowbase + yl * nx + x;
@@ -340,6 +346,8 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __re
   __syncthreads();
   if (wrow) {
     if (PAIR && logL == 11) pair_rows<-1, true, false>(sm, ty + nzrows, cs, tws);
+    else if (three && L == 384) warp_rows<12, -1, true, false, ONE ? 1 : 2>(sm, ty + nzrows, cs, tws);
+    else if (!ONE && three) warp_rows<24, -1, true, false>(sm, ty + nzrows, cs, tws);
     else if (!ONE && logL == 10) warp_rows<32, -1, true, false>(sm, ty + nzrows, cs, tws);
     else warp_rows<16, -1, true, false, ONE ? 1 : 2>(sm, ty + nzrows, cs, tws);
     __syncthreads();
@@ -361,7 +369,7 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __re
       const int yp = e & ((1 << pl) - 1);
       if (2 * yp >= ty) continue;
       const int kx = e >> pl;
-      const int xk = xidx(kx, sh), xc = xidx((L - kx) & (L - 1), sh);
+      const int xk = xidx(kx, sh), xc = xidx(THREE ? (kx ? L - kx : 0) : (L - kx) & (L - 1), sh);
       const float2* Z0 = sm + (2 * yp) * cs;
       const float2* Z1 = Z0 + cs;
       const float2* Zz = sm + (ty + yp) * cs;
@@ -387,7 +395,7 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __re
     const int yl = e & ((1 << tyl) - 1);
     if (yl >= ty) continue;
     const int kx = e >> tyl;
-    const int xk = xidx(kx, sh), xc = xidx((L - kx) & (L - 1), sh);
+    const int xk = xidx(kx, sh), xc = xidx(THREE ? (kx ? L - kx : 0) : (L - kx) & (L - 1), sh);
     const float2* Z = sm + yl * cs;
     const float2* Zz = sm + (ty + (yl >> 1)) * cs;
     const float2 zk = Z[xk], zc = cconj(Z[xc]), zkz = Zz[xk], zcz = cconj(Zz[xc]);
@@ -641,7 +649,7 @@ __device__ __forceinline__ void prefetch_kslab(const MagnetDev& M, int kx0, int 
   if (threadIdx.x != 0) return;
   const int n = min(nkx, M.Fh - kx0);
   if (n <= 0) return;
-  const size_t slab = (size_t)(Pz / 2 + 1) * M.kcomp * ((1 << M.logP[1]) / 2 + 1);
+  const size_t slab = (size_t)(Pz / 2 + 1) * M.kcomp * (M.P[1] / 2 + 1);
   prefetch_l2(M.kspec + (size_t)kx0 * slab, (size_t)n * slab * sizeof(float));
 }
 
@@ -740,7 +748,7 @@ __device__ __forceinline__ void yzw_forward(const float2* __restrict__ S, int ny
 #pragma unroll
       for (int r = 0; r < Q; ++r) {  // y = lane + 32 r < Py/2; y >= ny is zero padding
         const int y = lane + 32 * r;
-        v[c * Q + r] = (c < nc && r < Q / 2 && y < ny && span_ok((size_t)(col0 + c) * ny + y, sleft))
+        v[c * Q + r] = (c < nc && 2 * r < Q && y < ny && span_ok((size_t)(col0 + c) * ny + y, sleft))
                            ? __ldg(S + (size_t)(col0 + c) * ny + y)
                            : make_float2(0.f, 0.f);
       }
@@ -797,12 +805,13 @@ template <int PZ, int Q, bool ONE = false>
 __device__ __forceinline__ void yzw_body(const MagnetDev& M, int kx0, int nkx, float2* sm,
                                          const float2* __restrict__ tw) {
   constexpr int Py = 32 * Q, cs = qlen(Py);
-  constexpr int LOGPY = Q == 2 ? 6 : Q == 4 ? 7 : Q == 8 ? 8 : Q == 16 ? 9 : 10;
+  constexpr int LOGPY = Q == 2 ? 6 : Q == 4 ? 7 : Q == 8 ? 8 : Q == 16 ? 9 : 10;  // of the powers of two
   const int ny = M.n[1], nz = M.n[2];
   const int ncol = nkx * 3 * nz;
   float2* D = sm;
   float2* twq = sm + ncol * cs;
-  load_twq(twq, tw, LOGPY);
+  if constexpr (Q % 3 == 0) load_twq3(twq, tw + TW_N, Q);
+  else load_twq(twq, tw, LOGPY);
   prefetch_kslab(M, kx0, nkx, PZ);
   __syncthreads();
   pdl_wait();  // the spectrum is written by the x pass
@@ -812,21 +821,21 @@ __device__ __forceinline__ void yzw_body(const MagnetDev& M, int kx0, int nkx, f
   yzw_forward<Q, W>(S, ny, D, ncol, twq, sleft);
   __syncthreads();
   if constexpr (PZ == 1) {
-    for (int t = threadIdx.x; t < nkx << LOGPY; t += blockDim.x) {
-      const int j = t >> LOGPY;
-      zstage_single<true>(D + j * 3 * cs, cs, M, kx0 + j, t & (Py - 1), Py);
+    for (int t = threadIdx.x; t < nkx * Py; t += blockDim.x) {
+      const int j = t / Py;
+      zstage_single<true>(D + j * 3 * cs, cs, M, kx0 + j, t - j * Py, Py);
     }
   } else if constexpr (PZ >= 4) {  // one lane per (kx, ky)
-    for (int t = threadIdx.x; t < nkx << LOGPY; t += blockDim.x) {
-      const int j = t >> LOGPY;
-      zstage_full<PZ, true>(D + j * 3 * nz * cs, cs, M, kx0 + j, t & (Py - 1), nz, Py);
+    for (int t = threadIdx.x; t < nkx * Py; t += blockDim.x) {
+      const int j = t / Py;
+      zstage_full<PZ, true>(D + j * 3 * nz * cs, cs, M, kx0 + j, t - j * Py, nz, Py);
     }
   } else {
     // lanes l and l + 16 of a warp share one (kx, ky): the even and odd kz
     // halves (the item count is a multiple of 32 and so is the block)
-    for (int t = threadIdx.x; t < (2 * nkx) << LOGPY; t += blockDim.x) {
-      const int u = ((t >> 5) << 4) | (t & 15), j = u >> LOGPY;
-      zstage_pair<PZ, true, 16>(D + j * 3 * nz * cs, cs, M, kx0 + j, u & (Py - 1), (t >> 4) & 1, nz, Py);
+    for (int t = threadIdx.x; t < 2 * nkx * Py; t += blockDim.x) {
+      const int u = ((t >> 5) << 4) | (t & 15), j = u / Py;
+      zstage_pair<PZ, true, 16>(D + j * 3 * nz * cs, cs, M, kx0 + j, u - j * Py, (t >> 4) & 1, nz, Py);
     }
   }
   __syncthreads();
@@ -859,6 +868,46 @@ __global__ void __launch_bounds__(yzw_threads<PZ>(), PZ == 16 ? 1 : 2)
     case 8: yzw_body<PZ, 8, ONE>(M, kx0, nkx, sm, tw); break;
     default: yzw_body<PZ, 16, ONE>(M, kx0, nkx, sm, tw); break;
   }
+}
+
+// y lengths 96, 192, 384 (and 768 in a kernel of its own): 3 2^k points where 2 n - 1
+// would be padded to the next power of two.  A column takes Q = 3, 6, 12, 24 inner
+// points per lane and the outer step Q of 32 / W lanes (30, 30, 24 and 24 of the
+// warp's), so a length saves about a quarter of the transforms and the whole quarter
+// of the z stage, the spectrum and the kernel of the power of two above it.
+template <int PZ, bool ONE = false>
+__global__ void __launch_bounds__(yzw_threads<PZ>(), PZ == 16 ? 1 : 2)
+    k_yzw3(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, const Work* __restrict__ work,
+           int stage, int gate, const float2* __restrict__ tw) {
+  extern __shared__ float2 sm[];
+  __shared__ MagnetDev M;
+  __shared__ GroupDev G;
+  pdl_trigger();  // the x-inverse pass may start its prologue during the last wave
+  const Work wk = work[blockIdx.x];
+  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) {
+    pdl_wait();
+    return;
+  }
+  switch (M.P[1]) {
+    case 96: yzw_body<PZ, 3, ONE>(M, wk.z, wk.y0, sm, tw); break;
+    case 192: yzw_body<PZ, 6, ONE>(M, wk.z, wk.y0, sm, tw); break;
+    default: yzw_body<PZ, 12, ONE>(M, wk.z, wk.y0, sm, tw); break;
+  }
+}
+template <int PZ>
+__global__ void __launch_bounds__(yzw_threads<PZ>(), PZ == 16 ? 1 : 2)
+    k_yzw24(const MagnetDev* __restrict__ mags, const GroupDev* __restrict__ groups, const Work* __restrict__ work,
+            int stage, int gate, const float2* __restrict__ tw) {
+  extern __shared__ float2 sm[];
+  __shared__ MagnetDev M;
+  __shared__ GroupDev G;
+  pdl_trigger();  // the x-inverse pass may start its prologue during the last wave
+  const Work wk = work[blockIdx.x];
+  if (!load_descs(M, G, mags, groups, wk.mag, gate, stage)) {
+    pdl_wait();
+    return;
+  }
+  yzw_body<PZ, 24>(M, wk.z, wk.y0, sm, tw);
 }
 
 // y length 1024 in a kernel of its own: the body of one length keeps the hot
@@ -1580,7 +1629,7 @@ __device__ __forceinline__ void stage_quad_lean(const MagnetDev& M, const GroupD
 // by its registers).  A 200 x 200 disc took 21 us of a 45 us stage in the general
 // path (epilogue_cell), whose cells fetch their neighbours one after the other
 // and divide per neighbour: 18 Fehlberg attempts 4.91 -> 3.18 ms.
-template <bool PAIR = false, bool MASK = false, bool ONE = false>
+template <bool PAIR = false, bool MASK = false, bool ONE = false, bool THREE = false>
 __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __restrict__ mags, GroupDev* __restrict__ groups,
                                               const Work* __restrict__ work, EpiArgs ea,
                                               const float2* __restrict__ tw) {
@@ -1595,15 +1644,18 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __re
   }
   const int z = wk.z, y0 = wk.y0, ty = wk.ty;
   const int nx = M.n[0], ny = M.n[1], nz = M.n[2];
-  const int logL = M.logP[0], L = 1 << logL, cs = xrow_stride(L, ty);
-  if (!PAIR && logL == 11) return;  // 2048-point rows only in the PAIR form (the host never launches them here)
+  const int logL = M.logP[0], L = THREE ? M.P[0] : 1 << logL, cs = xrow_stride(L, ty);
+  // rows of the PAIR and THREE forms (the host never launches them elsewhere)
+  if ((!PAIR && logL == 11) || (!THREE && logL >= LOG_THREE)) return;
+  const bool three = THREE && logL >= LOG_THREE;
   const int nzrows = (ty + 1) >> 1;
   const int Fh = M.Fh;
   float2* rows_z = sm + ty * cs;
   float2* tws = sm + (ty + nzrows) * cs;  // twiddles of length L
-  const bool wrow = (PAIR && logL == 11) || logL == 10 || logL == 9;  // 2048- / 1024- / 512-point rows: warp (pair) rows
+  const bool wrow = three || (PAIR && logL == 11) || logL == 10 || logL == 9;  // 2048- / 1024- / 512-point rows: warp (pair) rows
   const int sh = wrow ? 5 : 4;
-  if (wrow) load_twq(tws, tw, logL);
+  if (three) load_twq3(tws, tw + TW_N, L >> 5);
+  else if (wrow) load_twq(tws, tw, logL);
   else load_twiddles<3>(tws, tw, logL);
   __shared__ NbRows T;
   __shared__ float cf[8];  // FSAL error weights dt (b1 - b2) of the stages
@@ -1699,6 +1751,8 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __re
   __syncthreads();
   if (wrow) {  // only x < nx <= L/2 is used
     if (PAIR && logL == 11) pair_rows<1, false, true>(sm, ty + nzrows, cs, tws);
+    else if (three && L == 384) warp_rows<12, 1, false, true, ONE ? 1 : 2>(sm, ty + nzrows, cs, tws);
+    else if (!ONE && three) warp_rows<24, 1, false, true>(sm, ty + nzrows, cs, tws);
     else if (!ONE && logL == 10) warp_rows<32, 1, false, true>(sm, ty + nzrows, cs, tws);
     else warp_rows<16, 1, false, true, ONE ? 1 : 2>(sm, ty + nzrows, cs, tws);
     __syncthreads();

@@ -1,6 +1,6 @@
 // launch.h -- the kernels of the demag passes and of the Runge-Kutta stages, as
 // the engine launches them.  The instantiations are compiled in one file per
-// family (xpass.cu, yz.cu, yzwarp.cu, yzlong.cu, thick.cu, pairs.cu), so that a change of
+// family (xpass.cu, xthree.cu, yz.cu, yzwarp.cu, yzlong.cu, yzthree.cu, thick.cu, pairs.cu), so that a change of
 // one kernel compiles that family only and the families compile in parallel;
 // engine.cu reaches them through these functions.  The index-checked build
 // (-DMPX_BOUNDS_CHECK) keeps everything in one translation unit (checked.cu):
@@ -54,9 +54,10 @@ using ControllerFn = void (*)(GroupDev*, int);
 using YzFn = void (*)(const MagnetDev*, const GroupDev*, const Work*, int, int, const float2*);
 
 // xpass.cu: everything that reads the Butcher tableau
-// Forms of the x passes: warp-pair rows, rows one per warp, masked magnets (kernels.cuh).
+// Forms of the x passes: warp-pair rows, rows one per warp, masked magnets, rows of
+// 384 and 768 points (kernels.cuh).
 struct XForm {
-  bool pair = false, one = false, mask = false;
+  bool pair = false, one = false, mask = false, three = false;
 };
 XfwdFn xfwd_fn(bool combine, XForm f);
 XinvFn xinv_fn(XForm f);
@@ -64,14 +65,19 @@ LocalFn local_fn();
 CombineFn combine_fn();
 ControllerFn controller_fn();
 cudaError_t upload_tableau_symbol(const TableauDev& t, cudaStream_t stream);
+// xthree.cu: the forms of the x passes with `three`
+XfwdFn xfwd_three_fn(bool combine, XForm f);
+XinvFn xinv_three_fn(XForm f);
+cudaError_t upload_tableau_three(const TableauDev& t, cudaStream_t stream);
 
 // Launch classes of the y/z pass (yz_class of engine.cu): 0 .. 9 the block-wide
 // passes (yz.cu), 10 .. 14 the warp columns of y lengths 64 .. 512 (yzwarp.cu),
-// 15 .. 23 y lengths 1024 and 2048 (yzlong.cu).
-constexpr int YZ_CLASSES = 24;
+// 15 .. 23 y lengths 1024 and 2048 (yzlong.cu), 24 .. 33 y lengths 96 .. 768 (yzthree.cu).
+constexpr int YZ_CLASSES = 34;
 YzFn yz_block_fn(int cls);
 YzFn yz_warp_fn(int cls, bool one);
 YzFn yz_long_fn(int cls);
+YzFn yz_three_fn(int cls, bool one);
 
 // thick.cu: the split y/z path
 YzFn ycols_fn(int dir, int maxlr);
@@ -82,7 +88,7 @@ YzFn zcw_fn();
 // Their warp-column forms (k_ycw, k_zcw of yzsplit.cuh): block sizes, columns or ky
 // per block, and dynamic shared memory.
 constexpr int YCW_THREADS = 256;  // 8 warps, 32 / Q columns (1024 values) each
-__host__ __device__ constexpr int ycw_cols(int Py) { return YCW_THREADS * 32 / Py; }
+__host__ __device__ constexpr int ycw_cols(int Py) { return (YCW_THREADS / 32) * (1024 / Py); }
 __host__ __device__ constexpr int ycw_smem(int Py) {
   return ((YCW_THREADS / 32) * (1024 / Py) * qlen(Py) + Py) * (int)sizeof(float2);
 }

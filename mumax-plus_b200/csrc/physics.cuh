@@ -48,6 +48,8 @@ struct DVector {  // uniform value or per-cell SoA array (3*N)
   }
 };
 
+constexpr int LOG_THREE = 16;  // marks the lengths 3 2^k in MagnetDev::logP
+
 // Device description of one magnet (lives in a device array, indexed by slot).
 struct MagnetDev {
   int n[3], N;
@@ -76,7 +78,7 @@ struct MagnetDev {
   unsigned terms;    // TERM_* and FLAG_* bits
   int group;         // solve group slot
   // demag FFT plan: padded sizes P = 2^logP, Fh = Px/2+1
-  int logP[3], P[3], Fh;
+  int logP[3], P[3], Fh;  // logP: log2 P, or LOG_THREE + log2(P / 96) of the lengths 96 .. 768
   int kcomp;         // 6 (3-D kernel) or 4 (Pz == 1)
   float2* spec;      // spectrum S[kx][c][z][y]
   float2* tspec;     // split y/z path: y-transformed spectrum T[kx][c][z][ky] (Py rows), else NULL

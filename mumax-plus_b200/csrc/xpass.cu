@@ -1,17 +1,19 @@
 // xpass.cu -- the x passes, the local-terms kernel, the stage combination and
-// the step controller: every kernel that reads the Butcher tableau in constant
-// memory (one copy per translation unit, so they stay together).
+// the step controller: the kernels that read the Butcher tableau in constant
+// memory (one copy per translation unit; xthree.cu has the other).
 #include "launch.h"
 #include "stages.cuh"
 
 namespace mpx {
 
 XfwdFn xfwd_fn(bool combine, XForm f) {
+  if (f.three) return xfwd_three_fn(combine, f);
   if (f.one) return combine ? k_xfwd<true, false, true> : k_xfwd<false, false, true>;
   if (combine) return f.pair ? k_xfwd<true, true> : k_xfwd<true, false>;
   return f.pair ? k_xfwd<false, true> : k_xfwd<false, false>;
 }
 XinvFn xinv_fn(XForm f) {
+  if (f.three) return xinv_three_fn(f);
   if (f.one) return f.mask ? k_xinv<false, true, true> : k_xinv<false, false, true>;
   if (f.mask) return f.pair ? k_xinv<true, true> : k_xinv<false, true>;
   return f.pair ? k_xinv<true, false> : k_xinv<false, false>;

@@ -175,7 +175,7 @@ __device__ __forceinline__ void ycw_body(const MagnetDev& M, int col0, int ncol,
     for (int r = 0; r < Q; ++r) {
       const int y = lane + 32 * r;
       if constexpr (DIR < 0)  // S: ny rows, zero padding above (y < Py / 2 only)
-        v[c * Q + r] = (c < nc && r < Q / 2 && y < ny && span_ok((size_t)c * ny + y, sleft)) ? S[(size_t)c * ny + y]
+        v[c * Q + r] = (c < nc && 2 * r < Q && y < ny && span_ok((size_t)c * ny + y, sleft)) ? S[(size_t)c * ny + y]
                                                                                               : make_float2(0.f, 0.f);
       else
         v[c * Q + r] = (c < nc && span_ok((size_t)c * Py + y, tleft)) ? T[(size_t)c * Py + y] : make_float2(0.f, 0.f);
@@ -209,9 +209,10 @@ __global__ void __launch_bounds__(YCW_THREADS, 2)
     pdl_wait();
     return;
   }
-  const int logPy = M.logP[1];
-  float2* twq = sm + (YCW_THREADS / 32) * (1024 >> logPy) * qlen(1 << logPy);
-  load_twq(twq, tw, logPy);
+  const int logPy = M.logP[1], Py = M.P[1];
+  float2* twq = sm + (YCW_THREADS / 32) * (1024 / Py) * qlen(Py);
+  if (logPy >= LOG_THREE) load_twq3(twq, tw + TW_N, Py >> 5);
+  else load_twq(twq, tw, logPy);
   __syncthreads();
   pdl_wait();  // the columns are written by the previous pass
   switch (logPy) {
@@ -219,6 +220,10 @@ __global__ void __launch_bounds__(YCW_THREADS, 2)
     case 7: ycw_body<4, DIR>(M, wk.z, wk.y0, sm, twq); break;
     case 8: ycw_body<8, DIR>(M, wk.z, wk.y0, sm, twq); break;
     case 9: ycw_body<16, DIR>(M, wk.z, wk.y0, sm, twq); break;
+    case LOG_THREE: ycw_body<3, DIR>(M, wk.z, wk.y0, sm, twq); break;
+    case LOG_THREE + 1: ycw_body<6, DIR>(M, wk.z, wk.y0, sm, twq); break;
+    case LOG_THREE + 2: ycw_body<12, DIR>(M, wk.z, wk.y0, sm, twq); break;
+    case LOG_THREE + 3: ycw_body<24, DIR>(M, wk.z, wk.y0, sm, twq); break;
     default: ycw_body<32, DIR>(M, wk.z, wk.y0, sm, twq); break;
   }
 }

@@ -5,8 +5,10 @@ damping, the octant construction of the demag kernel, and the stray fields of
 several magnets sharing their launches.
 
 Tolerances as tests/test_gpu_parity.py: fields <= 1e-5 of max|B| (FP32 transforms of
-a few thousand points: about 1e-6), one explicit step of m <= 2e-6 absolute
-(rounding of m, dt k and their sum, 3 x 6e-8 of 1, with a factor of ten)."""
+a few thousand points: about 1e-6), 5e-5 for the demag field alone at 150,000 cells
+and more (the bound of tests/test_gpu_configs.py there; the oracle convolves the
+GPU's kernel values), one explicit step of m <= 2e-6 absolute (rounding of m, dt k and
+their sum, 3 x 6e-8 of 1, with a factor of ten)."""
 import numpy as np
 import pytest
 
@@ -133,3 +135,61 @@ def test_three_magnets_share_launches(mpx):
     world.timesolver.steps(2)
     for q, mag in zip(qs, mags):
         assert np.max(np.abs(mag.magnetization.eval() - ow.get_m(q))) < 2e-6
+
+
+# lengths 3 2^k (magnets of at least 150,000 cells): y lengths 96 .. 768 at z lengths 1, 4, 8, 16 and on the split
+# path, x lengths 384 and 768, sides at the ends of their ranges (2 n - 1 just below the length and just above the
+# power of two below it), odd row counts, one and several columns per warp
+@pytest.mark.parametrize("size", [(1000, 160, 1), (500, 340, 1), (384, 392, 1), (1024, 192, 1), (610, 257, 1),
+                                  (420, 180, 2), (1000, 96, 2), (192, 400, 2), (129, 601, 2), (150, 350, 3),
+                                  (385, 129, 4), (1000, 40, 4), (400, 95, 4), (300, 130, 4), (193, 384, 3),
+                                  (150, 140, 8), (130, 260, 5), (1000, 33, 5), (160, 48, 20), (100, 96, 16),
+                                  (90, 180, 10), (60, 300, 9), (30, 65, 80), (257, 193, 4)])
+def test_lengths_with_a_factor_three(mpx, size):
+    nx, ny, nz = size
+    assert nx * ny * nz >= 150000
+    spec = MagnetSpec(size=size, cellsize=(2e-9, 1.5e-9, 1e-9), msat=8e5)
+    m0 = random_m(spec.shape, seed=3, smooth=2)
+    world, magnet = spec.product(mpx, m0)
+    eng = magnet._engine
+    K = eng.demag_kernel(magnet._id)  # displacement 0 at index K - n
+    octant = np.ascontiguousarray(K[:, K.shape[1] - nz:, K.shape[2] - ny:, K.shape[3] - nx:].astype(np.float64))
+    ow, q = spec.oracle_world(m0)
+    ow.set_kernel_octant(q, octant)  # the same kernel values: the convolution alone is compared
+    got = eng.eval(magnet._id, abi.Q_DEMAG_FIELD, (3, *spec.shape))
+    assert max_rel(got, ow.eval(q, abi.Q_DEMAG_FIELD)) < 5e-5
+
+
+@pytest.mark.parametrize("size", [(150, 350, 3), (301, 167, 3), (1000, 160, 1), (160, 48, 20)])
+def test_stages_with_a_factor_three(mpx, size):
+    """Stage combination, the three passes and the lean epilogue over two Dormand-Prince steps."""
+    s = MagnetSpec(size=size, cellsize=(3e-9, 3e-9, 3e-9), msat=8e5, aex=1.3e-11, alpha=0.1,
+                   world_bias=(0.0, 0.01, 0.0))
+    m0 = random_m(s.shape, seed=8, smooth=3)
+    ow, q = s.oracle_world(m0)
+    ow.set_method("DormandPrince")
+    ow.set_solver(adaptive=0)
+    world, magnet = s.product(mpx, m0)
+    world.timesolver.set_method("DormandPrince")
+    world.timesolver.adaptive_timestep = False
+    dt = 2 * ow.sensible_timestep()
+    ow.timestep = dt
+    world.timesolver.timestep = dt
+    ow.steps(2)
+    world.timesolver.steps(2)
+    assert np.max(np.abs(magnet.magnetization.eval() - ow.get_m(q))) < 2e-6
+
+
+def test_factor_three_solves_in_a_batch(mpx):
+    """Solves with and without these lengths together end as each does alone."""
+    from mumaxplus_b200 import batch, workloads as W
+
+    ws = []
+    for k, (side, nz) in enumerate([(40, 1), (190, 5), (100, 1), (280, 2), (60, 1), (390, 1)]):
+        ws.append(dict(name=f"s{k}", size=(side, side, nz), cellsize=(3e-9, 3e-9, 3e-9), msat=8e5, aex=1.3e-11,
+                       alpha=0.3, world_bias=(0.0, 0.01, 0.0),
+                       m0=lambda s=side, z=nz, k=k: W.smoothed_random_m((z, s, s), 100 + k)))
+    together, _, _ = batch.relax_batch(batch.Batch(), ws, duration=1e-12, torque_stop=0.0, autotune=False)
+    alone, _, _ = batch.run_plain(batch.Batch(), ws, duration=1e-12, torque_stop=0.0)
+    for a, b in zip(together, alone):
+        assert a.steps == b.steps and np.array_equal(a.m, b.m)
