@@ -1092,6 +1092,10 @@ __device__ __forceinline__ void epilogue_cell(const MagnetDev& M, const GroupDev
     }
     return;
   }
+  if (q == 6) {  // the demag field alone needs no local terms (1024 x 1024 x 4 cells: 557 -> 470 us)
+    store3(out, N, i, bdemag);
+    return;
+  }
   const float ms = M.msat.at(i);
   LocalOut lo;
   lo.exch = lo.anis = lo.ext = lo.dmi = f3(0, 0, 0);
