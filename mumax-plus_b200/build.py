@@ -3,9 +3,9 @@
 The kernel families compile in one file each (csrc/*.cu, see csrc/launch.h), in
 parallel, into _build/ and link into one library next to this file, so that it
 travels with the source tree; a file is compiled again when one of the headers
-it includes has changed.  A second build of the same sources in one translation
-unit (csrc/checked.cu) with -DMPX_BOUNDS_CHECK, libmpx_checked.so, verifies the
-index of every per-cell field access (mpx_bounds_check reads the record).
+it includes has changed.  A second build of the same files with
+-DMPX_BOUNDS_CHECK, libmpx_checked.so, verifies the index of every per-cell field
+access (mpx_bounds_check reads the records).
 """
 import concurrent.futures
 import os
@@ -17,6 +17,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 UNITS = ["xthree", "xpass", "yz", "engine", "yzwarp", "yzlong", "yzthree", "thick", "pairs"]
+CHECKED_UNITS = ["checked_" + u for u in UNITS]  # objects of the same files with the check
 OUT = os.path.join(HERE, "libmpx.so")
 OUT_CHECKED = os.path.join(HERE, "libmpx_checked.so")
 
@@ -58,7 +59,7 @@ def _stale(unit):
 
 
 def up_to_date(out=OUT):
-    units = ["checked"] if out == OUT_CHECKED else UNITS
+    units = CHECKED_UNITS if out == OUT_CHECKED else UNITS
     if not os.path.exists(out) or any(_stale(u) for u in units):
         return False
     return all(os.path.getmtime(_obj(u)) <= os.path.getmtime(out) for u in units)
@@ -76,15 +77,14 @@ def _run(cmd, verbose):
 
 def _command(out, extra=(), unit="engine"):
     """The nvcc command of `unit` into `out`; the checked library's adds the check."""
-    defs = ["-DMPX_BOUNDS_CHECK"] if out in (OUT_CHECKED, _obj("checked")) else []
-    return ([nvcc_path()] + NVCC_FLAGS + defs + list(extra) + ["-I", os.path.join(ROOT, "include")]
-            + [os.path.join(CSRC, unit + ".cu"), "-o", out])
+    checked = out == OUT_CHECKED or unit.startswith("checked_")
+    src = os.path.join(CSRC, unit.removeprefix("checked_") + ".cu")
+    return ([nvcc_path()] + NVCC_FLAGS + (["-DMPX_BOUNDS_CHECK"] if checked else []) + list(extra)
+            + ["-I", os.path.join(ROOT, "include"), src, "-o", out])
 
 
 def _compile(unit, extra, verbose):
     extra = list(extra) + ["-c", "-MMD", "-MF", os.path.join(OBJ, unit + ".d")]
-    if unit == "checked":  # one large file: its kernels are optimised in parallel
-        extra.append("--split-compile=0")
     _run(_command(_obj(unit), extra, unit), verbose)
 
 
@@ -93,13 +93,13 @@ def build(force=False, verbose=False, extra=(), checked=True):
     returns the path of libmpx.so."""
     os.makedirs(OBJ, exist_ok=True)
     outs = [o for o in ([OUT, OUT_CHECKED] if checked else [OUT]) if force or not up_to_date(o)]
-    units = [u for o in outs for u in (["checked"] if o == OUT_CHECKED else UNITS) if force or _stale(u)]
-    units.sort(key=lambda u: u != "checked")  # the longest first
+    units = [u for o in outs for u in (CHECKED_UNITS if o == OUT_CHECKED else UNITS) if force or _stale(u)]
+    units.sort(key=lambda u: UNITS.index(u.removeprefix("checked_")))  # the longest first
     with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, os.cpu_count() or 1)) as pool:
         for f in [pool.submit(_compile, u, extra, verbose) for u in units]:
             f.result()
     for out in outs:
-        objs = [_obj(u) for u in (["checked"] if out == OUT_CHECKED else UNITS)]
+        objs = [_obj(u) for u in (CHECKED_UNITS if out == OUT_CHECKED else UNITS)]
         _run([nvcc_path(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", out] + objs, verbose)
     return OUT
 

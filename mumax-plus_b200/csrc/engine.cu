@@ -3630,9 +3630,12 @@ mpx_status mpx_bounds_check(unsigned long long* first_bad) {
   *first_bad = 0;
 #ifdef MPX_BOUNDS_CHECK
   CUDA_TRY(cudaDeviceSynchronize());
-  CUDA_TRY(cudaMemcpyFromSymbol(first_bad, g_bounds_first_bad, sizeof(unsigned long long)));
-  const unsigned long long zero = 0;
-  CUDA_TRY(cudaMemcpyToSymbol(g_bounds_first_bad, &zero, sizeof zero));
+  for (auto take : {bounds_take, bounds_take_xpass, bounds_take_xthree, bounds_take_yz, bounds_take_yzwarp,
+                    bounds_take_yzlong, bounds_take_yzthree, bounds_take_thick, bounds_take_pairs}) {
+    unsigned long long bad = 0;
+    CUDA_TRY(take(&bad));
+    if (!*first_bad) *first_bad = bad;
+  }
   return MPX_OK;
 #else
   return fail(MPX_ERR_UNSUPPORTED, "mpx_bounds_check: library built without MPX_BOUNDS_CHECK (use libmpx_checked.so)");

@@ -2,9 +2,8 @@
 // the engine launches them.  The instantiations are compiled in one file per
 // family (xpass.cu, xthree.cu, yz.cu, yzwarp.cu, yzlong.cu, yzthree.cu, thick.cu, pairs.cu), so that a change of
 // one kernel compiles that family only and the families compile in parallel;
-// engine.cu reaches them through these functions.  The index-checked build
-// (-DMPX_BOUNDS_CHECK) keeps everything in one translation unit (checked.cu):
-// its record of the first bad index is one device variable.
+// engine.cu reaches them through these functions.  In the index-checked build
+// (-DMPX_BOUNDS_CHECK) every file has its own record of the first bad index.
 #pragma once
 #include "../../include/mpx.h"
 #include "kernels.cuh"
@@ -106,5 +105,17 @@ PairFn pair_yfft_fn(int dir);
 PairFn pair_zmul_fn(bool mul);
 PairFn pair_yz_fn(int logPz);
 PairFn pair_xinv_fn();
+
+#ifdef MPX_BOUNDS_CHECK
+// the record of each file: read and cleared
+cudaError_t bounds_take_xpass(unsigned long long* first_bad);
+cudaError_t bounds_take_xthree(unsigned long long* first_bad);
+cudaError_t bounds_take_yz(unsigned long long* first_bad);
+cudaError_t bounds_take_yzwarp(unsigned long long* first_bad);
+cudaError_t bounds_take_yzlong(unsigned long long* first_bad);
+cudaError_t bounds_take_yzthree(unsigned long long* first_bad);
+cudaError_t bounds_take_thick(unsigned long long* first_bad);
+cudaError_t bounds_take_pairs(unsigned long long* first_bad);
+#endif
 
 }  // namespace mpx

@@ -17,4 +17,8 @@ PairFn pair_yz_fn(int logPz) {
 }
 PairFn pair_xinv_fn() { return k_pair_xinv; }
 
+#ifdef MPX_BOUNDS_CHECK
+cudaError_t bounds_take_pairs(unsigned long long* first_bad) { return bounds_take(first_bad); }
+#endif
+
 }  // namespace mpx

@@ -147,6 +147,12 @@ __device__ __forceinline__ bool in_geom(const MagnetDev& M, int i) { return !M.g
 // skipped -- a load gives 0 -- so the kernel runs to its end and the host reads
 // the record with mpx_bounds_check.  Nothing traps.
 static __device__ unsigned long long g_bounds_first_bad;
+// reads and clears this translation unit's record (the device synchronised)
+static inline cudaError_t bounds_take(unsigned long long* first_bad) {
+  const unsigned long long zero = 0;
+  const cudaError_t st = cudaMemcpyFromSymbol(first_bad, g_bounds_first_bad, sizeof(unsigned long long));
+  return st != cudaSuccess ? st : cudaMemcpyToSymbol(g_bounds_first_bad, &zero, sizeof zero);
+}
 __device__ __forceinline__ bool cell_ok(int N, int i) {
   if ((unsigned)i < (unsigned)N) return true;
   atomicCAS(&g_bounds_first_bad, 0ull, (1ull << 63) | ((unsigned long long)(unsigned)N << 32) | (unsigned)i);

@@ -16,4 +16,8 @@ cudaError_t upload_tableau_three(const TableauDev& t, cudaStream_t stream) {
   return cudaMemcpyToSymbolAsync(c_tab, &t, sizeof(t), 0, cudaMemcpyHostToDevice, stream);
 }
 
+#ifdef MPX_BOUNDS_CHECK
+cudaError_t bounds_take_xthree(unsigned long long* first_bad) { return bounds_take(first_bad); }
+#endif
+
 }  // namespace mpx

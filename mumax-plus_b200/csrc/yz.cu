@@ -18,4 +18,8 @@ YzFn yz_block_fn(int cls) {
   }
 }
 
+#ifdef MPX_BOUNDS_CHECK
+cudaError_t bounds_take_yz(unsigned long long* first_bad) { return bounds_take(first_bad); }
+#endif
+
 }  // namespace mpx

@@ -17,4 +17,8 @@ YzFn yz_long_fn(int cls) {
   }
 }
 
+#ifdef MPX_BOUNDS_CHECK
+cudaError_t bounds_take_yzlong(unsigned long long* first_bad) { return bounds_take(first_bad); }
+#endif
+
 }  // namespace mpx

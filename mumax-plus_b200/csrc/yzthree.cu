@@ -20,4 +20,8 @@ YzFn yz_three_fn(int cls, bool one) {
   }
 }
 
+#ifdef MPX_BOUNDS_CHECK
+cudaError_t bounds_take_yzthree(unsigned long long* first_bad) { return bounds_take(first_bad); }
+#endif
+
 }  // namespace mpx

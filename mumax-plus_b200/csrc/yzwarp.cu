@@ -14,4 +14,8 @@ YzFn yz_warp_fn(int cls, bool one) {
   }
 }
 
+#ifdef MPX_BOUNDS_CHECK
+cudaError_t bounds_take_yzwarp(unsigned long long* first_bad) { return bounds_take(first_bad); }
+#endif
+
 }  // namespace mpx
