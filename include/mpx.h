@@ -268,7 +268,8 @@ mpx_status mpx_magnet_add_state(mpx_engine* e, int group, const mpx_magnet_desc*
 /* Device bytes mpx_magnet_add would take for `d`: *resident stays allocated
  * until the magnet is removed (state buffers, spectra, per-cell parameters,
  * work tables); *transient is the extra peak while it is added (the FP64
- * kernel construction buffers).  No engine or device needed; used to admit
+ * kernel construction buffers; up to 4 MB of the engine's own workspace are not
+ * counted).  No engine or device needed; used to admit
  * solves against a memory budget.  No counterpart in the reference, which
  * allocates from its pool as fields are needed (core/gpumemorypool.cu). */
 mpx_status mpx_magnet_bytes(const mpx_magnet_desc* d, int64_t* resident, int64_t* transient);

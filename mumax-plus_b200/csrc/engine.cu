@@ -991,53 +991,103 @@ void release_all(mpx_engine* e, Magnet* m);
 // the FFT form on the pair's kernel grid (periodic images included).
 constexpr long long STRAY_FFT_MIN_INTERACTIONS = 1LL << 22;
 
-// The lattice of the integrals that a table of displacements O + j, j < K per
-// axis, with the images of g, meets (newell.cuh), and how many of its `ncomp`
-// components are held at once: all where they take at most NEWELL_LATTICE_ALL (a
-// pool that has to grow for a larger one costs more than the launches saved: the
-// first image of a 400 x 400 x 4 film 0.7 -> 2.2 ms), one at a time up to
-// NEWELL_LATTICE_MAX, none (the point-by-point sum) beyond.
-constexpr int64_t NEWELL_LATTICE_ALL = 64LL << 20, NEWELL_LATTICE_MAX = 1LL << 30;
-int newell_lattice(const KernelGeom& g, const int K[3], const int O[3], int ncomp, NewellLattice* L) {
-  int64_t n = 8;
+// Lattice (newell.cuh) of the integrals that the displacements O + j, j < K per axis,
+// meet with the images I of the mastergrid mg.  Returns its points per
+// component, or -1 above 2^40.
+int64_t newell_lattice(const int mg[3], const int K[3], const int O[3], const NewellImages& I, NewellLattice* L) {
+  int64_t n = 1;
   for (int a = 0; a < 3; ++a) {
-    const int64_t reach = (int64_t)g.pbc[a] * g.mg[a] + 1, lo = O[a] - reach, hi = O[a] + K[a] - 1 + reach;
-    const int64_t a0 = lo <= 0 && hi >= 0 ? 0 : std::min(std::abs(lo), std::abs(hi));
-    const int64_t len = std::max(std::abs(lo), std::abs(hi)) - a0 + 1;
-    if (len > (1 << 24)) return 0;
-    L->a0[a] = (int)a0;
+    const int64_t from = O[a] + (int64_t)I.lo[a] * mg[a] - 1, to = O[a] + K[a] + (int64_t)I.hi[a] * mg[a];
+    const int64_t near = from <= 0 && to >= 0 ? 0 : std::min(std::abs(from), std::abs(to));
+    const int64_t len = std::max(std::abs(from), std::abs(to)) - near + 1;
+    if (len > (1 << 24) || n * len > (1LL << 40)) return -1;
+    L->a0[a] = (int)near;
     L->len[a] = (int)len;
     n *= len;
-    if (n > NEWELL_LATTICE_MAX) return 0;
   }
-  return n * ncomp <= NEWELL_LATTICE_ALL ? ncomp : 1;
+  return n;
+}
+
+// How a table of the tensor is built: the images of the first `axes` axes one at a
+// time, those of the others together (axes = 4: point by point, without a lattice),
+// `nc` components at a time, with a lattice of at most `points` per component.  The
+// fewest parts whose lattice takes at most `room` bytes are taken, and as many
+// components together as it and NEWELL_LATTICE_ALL allow (a pool that has to grow
+// for more costs more than the launches saved: the first image of a 400 x 400 x 4
+// film 0.7 -> 2.2 ms).  The order of the image sum, and so every bit of the table, is
+// the same in all of them.
+constexpr int64_t NEWELL_LATTICE_ALL = 64LL << 20;
+struct NewellPlan {
+  int axes, nc;
+  int64_t points;
+};
+NewellPlan newell_plan(const KernelGeom& g, const int K[3], const int O[3], int ncomp, int64_t room) {
+  for (int axes = 0; axes < 4; ++axes) {
+    NewellImages I;
+    for (int a = 0; a < 3; ++a) I.hi[a] = a < axes ? 0 : g.pbc[a], I.lo[a] = -I.hi[a];
+    NewellLattice L;
+    int64_t n = newell_lattice(g.mg, K, O, I, &L);
+    if (n < 0) continue;
+    for (int a = 0; a < axes; ++a)  // one image covers up to K + 2 points of an axis
+      if (g.pbc[a] > 0) n = n / L.len[a] * (K[a] + 2);
+    const int64_t nc = std::min(room, NEWELL_LATTICE_ALL) / (8 * n);
+    if (8 * n <= room) return {axes, (int)std::min<int64_t>(ncomp, std::max<int64_t>(1, nc)), n};
+  }
+  return {4, ncomp, 0};
 }
 
 // Components 0 .. ncomp - 1 of the Newell tensor, with the periodic images of g, at
-// the displacements O + j, j < K per axis, into out (layout [c][z][y][x]).
+// the displacements O + j, j < K per axis, into out (layout [c][z][y][x]), with at
+// most `room` bytes of lattice.
 template <typename T>
-mpx_status newell_table(mpx_engine* e, const KernelGeom& g, const int K[3], const int O[3], int ncomp, T* out) {
+mpx_status newell_table(mpx_engine* e, const KernelGeom& g, const int K[3], const int O[3], int ncomp, int64_t room,
+                        T* out) {
   const int grid = 148 * 8;
-  NewellLattice L;
-  const int nc = newell_lattice(g, K, O, ncomp, &L);
-  double* lat = nullptr;
-  if (nc > 0) {
-    const size_t lt = (size_t)L.len[0] * L.len[1] * L.len[2];
-    if (palloc(e, (void**)&lat, sizeof(double) * nc * lt) != MPX_OK) lat = nullptr;  // no room: point by point
+  NewellPlan p = newell_plan(g, K, O, ncomp, room);
+  const size_t Kt = (size_t)K[0] * K[1] * K[2];
+  double *lat = nullptr, *acc = nullptr;  // no room for them: point by point
+  const bool sums = sizeof(T) < sizeof(double) && p.axes > 0;  // FP32 table in parts: FP64 sums of one component
+  if (sums) p.nc = 1;
+  if (p.axes < 4 && palloc(e, (void**)&lat, sizeof(double) * p.nc * (size_t)p.points) == MPX_OK && sums &&
+      palloc(e, (void**)&acc, sizeof(double) * Kt) != MPX_OK) {
+    pfree(e, lat);
+    lat = nullptr;
   }
   if (lat) {
-    for (int c0 = 0; c0 < ncomp; c0 += nc) {
-      k_newell_lattice<<<grid, 128, 0, e->stream>>>(lat, g, L, c0, nc);
-      k_newell_from_lattice<<<grid, 256, 0, e->stream>>>(out, lat, g, L, c0, nc, K[0], K[1], K[2], O[0], O[1], O[2]);
-      e->launches += 2;
-    }
+    int part[3], i[3];  // images per part, first images of a part
+    for (int a = 0; a < 3; ++a) part[a] = a < p.axes ? 1 : 2 * g.pbc[a] + 1;
+    for (int c0 = 0; c0 < ncomp; c0 += p.nc)
+      for (i[0] = -g.pbc[0]; i[0] <= g.pbc[0]; i[0] += part[0])
+        for (i[1] = -g.pbc[1]; i[1] <= g.pbc[1]; i[1] += part[1])
+          for (i[2] = -g.pbc[2]; i[2] <= g.pbc[2]; i[2] += part[2]) {
+            NewellImages I;
+            bool first = true, last = true;
+            for (int a = 0; a < 3; ++a) {
+              I.lo[a] = i[a];
+              I.hi[a] = i[a] + part[a] - 1;
+              first = first && I.lo[a] == -g.pbc[a];
+              last = last && I.hi[a] == g.pbc[a];
+            }
+            NewellLattice L;
+            newell_lattice(g.mg, K, O, I, &L);
+            double* sum = acc;
+            if constexpr (sizeof(T) == sizeof(double)) sum = out;
+            const int nc = std::min(p.nc, ncomp - c0);
+            k_newell_lattice<<<grid, 128, 0, e->stream>>>(lat, g, L, c0, nc);
+            k_newell_from_lattice<<<grid, 256, 0, e->stream>>>(out, sum, sums ? c0 : 0, first, last, lat, g, L, I, c0,
+                                                               nc, K[0], K[1], K[2], O[0], O[1], O[2]);
+            e->launches += 2;
+          }
     pfree(e, lat);
+    pfree(e, acc);
   } else {
     k_newell_direct<<<grid, 128, 0, e->stream>>>(out, g, K[0], K[1], K[2], O[0], O[1], O[2], ncomp);
     e->launches++;
   }
   return check_launch(e, "Newell tensor");
 }
+// Room for the lattice of an FP32 table of 6 components that stays or is copied out.
+int64_t table_room(int64_t entries) { return std::max<int64_t>(NEWELL_LATTICE_ALL, 2 * 24 * entries); }
 
 // The FP32 table of the Newell tensor, with the periodic images of g, at the
 // displacements O + j, j < K per axis (newell_table's layout).  Where a
@@ -1061,11 +1111,11 @@ mpx_status build_pair_table(mpx_engine* e, const KernelGeom& g, const int K[3], 
     kt *= K[a];
   }
   if (2 * lt > kt) {
-    MPX_TRY(newell_table(e, g, K, O, 6, out));
+    MPX_TRY(newell_table(e, g, K, O, 6, table_room(kt), out));
   } else {
     float* abs_tab = nullptr;
     MPX_TRY(palloc(e, (void**)&abs_tab, sizeof(float) * 6 * (size_t)lt));
-    const mpx_status st = newell_table(e, g, L, A, 6, abs_tab);
+    const mpx_status st = newell_table(e, g, L, A, 6, table_room(lt), abs_tab);
     if (st != MPX_OK) {
       pfree(e, abs_tab);
       return st;
@@ -1389,17 +1439,31 @@ mpx_status launch_pairs(mpx_engine* e, int dst, int stage, int gate) {
 int kernel_axis_lines(int P) { return std::max(1, std::min(128, 2048 / P)); }
 int kernel_axis_smem(int P) { return (2 * kernel_axis_lines(P) + 1) * P * (int)sizeof(double2); }
 
-// Device bytes the construction holds beside the spectrum: the octant table with
-// the lattice of its integrals, then with the two transform arrays.
-int64_t kernel_build_bytes(const KernelGeom& g, const int P[3], int kcomp) {
-  const int O[3] = {0, 0, 0};
-  NewellLattice L;
-  const int nc = newell_lattice(g, g.n, O, kcomp, &L);
-  const int64_t lat = nc > 0 ? 8 * (int64_t)nc * L.len[0] * L.len[1] * L.len[2] : 0;
-  const int64_t Fh = P[0] / 2 + 1, hy = P[1] / 2 + 1;
-  return 8 * (int64_t)kcomp * g.n[0] * g.n[1] * g.n[2] +
-         std::max(lat, 8 * (int64_t)kcomp * g.n[2] * Fh * (g.n[1] + hy));
-}
+// Device bytes the construction of a kernel holds beside the spectrum: the octant
+// table, with it first the lattice of its integrals and then the two transform
+// arrays.  The lattice has twice the bytes of the transforms as room, which is below
+// what a padded complex grid per component pair would take, so that a periodic magnet
+// needs no more memory than its size asks for however many images it has (256 x 256 x 1
+// cells with 30 images: one lattice would take 1 GB); its images come in parts then
+// (admitting 256 x 256 x 1 cells with 10 images: 15.7 ms, 6.8 with one lattice of 121 MB).
+// LATTICE_ENGINE is the engine's own, like its reduction buffers, and not counted: it
+// keeps the parts of a small magnet few (32 x 32 x 1 cells with 30 images).
+constexpr int64_t LATTICE_ENGINE = 4LL << 20;
+struct KernelBuild {
+  int64_t octant, transforms, room;
+  KernelBuild(const int n[3], const int P[3], int kcomp) {
+    const int64_t Fh = P[0] / 2 + 1, hy = P[1] / 2 + 1;
+    octant = 8 * (int64_t)kcomp * n[0] * n[1] * n[2];
+    transforms = 8 * (int64_t)kcomp * n[2] * Fh * (n[1] + hy);
+    room = std::max(LATTICE_ENGINE, 2 * transforms);
+  }
+  int64_t bytes(const KernelGeom& g, int kcomp) const {
+    const int O[3] = {0, 0, 0};
+    const NewellPlan p = newell_plan(g, g.n, O, kcomp, room);
+    const int64_t lattice = 8 * (int64_t)p.nc * p.points;
+    return octant + std::max(transforms, lattice > LATTICE_ENGINE ? lattice : 0);
+  }
+};
 
 mpx_status build_kernel_spectrum(mpx_engine* e, Magnet* m) {
   MagnetDev& d = m->dev;
@@ -1417,7 +1481,7 @@ mpx_status build_kernel_spectrum(mpx_engine* e, Magnet* m) {
   double *oct = nullptr, *tx = nullptr, *ty = nullptr;
   mpx_status st = palloc(e, (void**)&oct, sizeof(double) * kcomp * (size_t)d.N);
   const int O[3] = {0, 0, 0};
-  if (st == MPX_OK) st = newell_table(e, g, d.n, O, kcomp, oct);
+  if (st == MPX_OK) st = newell_table(e, g, d.n, O, kcomp, KernelBuild(d.n, m->P, kcomp).room, oct);
   if (st == MPX_OK) st = palloc(e, (void**)&tx, sizeof(double) * kcomp * (size_t)nz * Fh * ny);
   if (st == MPX_OK) st = palloc(e, (void**)&ty, sizeof(double) * kcomp * (size_t)nz * Fh * hy);
   if (st == MPX_OK) {
@@ -2690,7 +2754,7 @@ mpx_status mpx_magnet_bytes(const mpx_magnet_desc* d, int64_t* resident, int64_t
       g.pbc[a] = d->pbc_repetitions[a];
       g.cs[a] = d->cellsize[a];
     }
-    tr += kernel_build_bytes(g, P, kc);  // FP64 construction of the kernel spectrum
+    tr += KernelBuild(d->size, P, kc).bytes(g, kc);  // FP64 construction of the kernel spectrum
   }
   *resident = res;
   *transient = tr;
@@ -3107,7 +3171,7 @@ mpx_status mpx_demag_kernel(mpx_engine* e, int magnet, float* out, int dims[3]) 
   const size_t KK = (size_t)K[0] * K[1] * K[2];
   float* d = nullptr;
   MPX_TRY(palloc(e, (void**)&d, sizeof(float) * 6 * KK));
-  const mpx_status ts = newell_table(e, g, K, O, 6, d);
+  const mpx_status ts = newell_table(e, g, K, O, 6, table_room(KK), d);
   if (ts != MPX_OK) {
     pfree(e, d);
     return ts;

@@ -91,8 +91,8 @@ struct KernelGeom {
 };
 
 // Table of N_c at the displacements O + j, j < K per axis (layout [c][z][y][x]),
-// each with its images, evaluated point by point: for geometries whose lattice
-// (below) would take more memory than the transforms of the kernel do.
+// each with its images, evaluated point by point: where the lattice (below) of even
+// one image does not fit its share of the memory.
 template <typename T>
 __global__ void k_newell_direct(T* __restrict__ out, KernelGeom g, int K0, int K1, int K2, int O0, int O1, int O2,
                                 int ncomp) {
@@ -114,9 +114,13 @@ __global__ void k_newell_direct(T* __restrict__ out, KernelGeom g, int K0, int K
 }
 
 // The lattice points |q| = a0 + p, p < len per axis (q in cells), that a table of
-// displacements meets: every displacement, image included, and its neighbours.
+// displacements meets: every displacement, its images included, and their neighbours.
 struct NewellLattice {
   int a0[3], len[3];
+};
+// Periodic images lo .. hi per axis.
+struct NewellImages {
+  int lo[3], hi[3];
 };
 
 // Axes (u, v, w) of the arguments of component c (newell_comp's permutations).
@@ -149,10 +153,14 @@ static __global__ void k_newell_lattice(double* __restrict__ lat, KernelGeom g, 
 // k_newell_direct's table of components c0 .. c0 + nc - 1 from the lattice.  The
 // integrals of the diagonal components are even in every argument, those of the
 // off-diagonal ones odd in the first two; the 27 terms and the images are added
-// in the order of the direct sum.
+// in the order of the direct sum.  The images may come in several parts of that
+// order: `acc` (components from ca on) holds the sum of the parts before this one
+// unless it is the first, and takes it unless this one is the last.
 template <typename T>
-__global__ void k_newell_from_lattice(T* __restrict__ out, const double* __restrict__ lat, KernelGeom g,
-                                      NewellLattice L, int c0, int nc, int K0, int K1, int K2, int O0, int O1, int O2) {
+__global__ void k_newell_from_lattice(T* out, double* acc, int ca, bool first, bool last,
+                                      const double* __restrict__ lat, KernelGeom g, NewellLattice L, NewellImages I,
+                                      int c0, int nc, int K0, int K1, int K2, int O0, int O1,
+                                      int O2) {
   const long long total = (long long)K0 * K1 * K2, ltot = (long long)L.len[0] * L.len[1] * L.len[2];
   const long long ls[3] = {1, L.len[0], (long long)L.len[0] * L.len[1]};
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total * nc;
@@ -164,10 +172,10 @@ __global__ void k_newell_from_lattice(T* __restrict__ out, const double* __restr
     newell_axes(c, u, v, w);
     const double norm = 4 * M_PI * g.cs[u] * g.cs[v] * g.cs[w];
     const double* __restrict__ F = lat + (c - c0) * ltot;
-    double sum = 0;
-    for (int i = -g.pbc[0]; i <= g.pbc[0]; ++i)
-      for (int j = -g.pbc[1]; j <= g.pbc[1]; ++j)
-        for (int k = -g.pbc[2]; k <= g.pbc[2]; ++k) {
+    double sum = first ? 0 : acc[(c - ca) * total + e];
+    for (int i = I.lo[0]; i <= I.hi[0]; ++i)
+      for (int j = I.lo[1]; j <= I.hi[1]; ++j)
+        for (int k = I.lo[2]; k <= I.hi[2]; ++k) {
           const int q[3] = {d[0] + i * g.mg[0], d[1] + j * g.mg[1], d[2] + k * g.mg[2]};
           const int qu = u == 0 ? q[0] : u == 1 ? q[1] : q[2], qv = v == 0 ? q[0] : v == 1 ? q[1] : q[2];
           const int qw = w == 0 ? q[0] : w == 1 ? q[1] : q[2];
@@ -189,7 +197,8 @@ __global__ void k_newell_from_lattice(T* __restrict__ out, const double* __restr
           }
           sum += r;
         }
-    out[c * total + e] = (T)sum;
+    if (last) out[c * total + e] = (T)sum;
+    else acc[(c - ca) * total + e] = sum;
   }
 }
 

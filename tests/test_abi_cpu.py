@@ -274,3 +274,27 @@ def test_geometry_and_region_masks():
     assert np.array_equal(fm._mask(regions, "regions"), regions)
     with pytest.raises(ValueError):
         fm._mask(-regions - 1, "regions")
+
+
+def _bytes(size, pbc, **kw):
+    from mumaxplus_b200 import batch as B
+
+    mg = tuple(n if r else 0 for n, r in zip(size, pbc))
+    return B.solve_bytes(dict(size=size, cellsize=(2e-9, 2e-9, 2e-9), mastergrid=mg, pbc=pbc, msat=8e5, aex=1e-11,
+                              alpha=0.1), **kw)
+
+
+@pytest.mark.parametrize("size,pbc", [((256, 256, 1), (1, 1, 0)), ((64, 64, 2), (1, 1, 0)), ((512, 512, 8), (1, 1, 0)),
+                                      ((100, 37, 5), (1, 0, 1)), ((700, 16, 1), (0, 1, 0))])
+def test_admission_does_not_grow_with_periodic_images(built_lib, size, pbc):
+    """What a periodic magnet is charged stays within an FP64 octant of 6 components, two padded complex grids and
+    the random initial state, however many images its kernel sums."""
+    padded = 1
+    for n in size:
+        padded *= 1 if n == 1 else 1 << (2 * n - 2).bit_length()
+    cells = size[0] * size[1] * size[2]
+    resident = _bytes(size, (0, 0, 0))[0]
+    for r in (1, 2, 5, 10, 30, 100):
+        res, tr = _bytes(size, tuple(r * p for p in pbc))
+        assert res == resident
+        assert tr <= 12 * cells + 48 * cells + 32 * padded, (r, tr)

@@ -102,6 +102,25 @@ def test_kernel_construction(mpx, size, pbc):
                                   pbc=pbc)) < FIELD_TOL
 
 
+# The demag kernel and the FP32 table of the real-space kernel are built apart, from lattices of different room:
+# the images of the kernel's lattice one at a time along x, along x and y, along all axes, with the table's all
+# together; and the table's one at a time.  The oracle convolves the table's values: with its own the distant images
+# would compare the FP64 cancellation of two tensor codes instead.
+@pytest.mark.parametrize("size,pbc", [((60, 60, 1), (9, 9, 0)), ((24, 60, 4), (0, 8, 9)), ((36, 36, 8), (0, 0, 60)),
+                                      ((200, 2, 3), (4200, 0, 0))])
+def test_kernel_construction_in_parts(mpx, size, pbc):
+    nx, ny, nz = size
+    mg = tuple(n if p else 0 for n, p in zip(size, pbc))
+    spec = MagnetSpec(size=size, cellsize=(1e-9, 2e-9, 1.5e-9), msat=8e5, mastergrid_size=mg, pbc=pbc)
+    m0 = random_m(spec.shape, seed=3, smooth=2)
+    world, magnet = spec.product(mpx, m0)
+    K = magnet._engine.demag_kernel(magnet._id)  # displacement 0 at index K - n
+    ow, q = spec.oracle_world(m0)
+    ow.set_kernel_octant(q, np.ascontiguousarray(K[:, K.shape[1] - nz:, K.shape[2] - ny:, K.shape[3] - nx:]))
+    got = magnet._engine.eval(magnet._id, abi.Q_DEMAG_FIELD, (3, *spec.shape))
+    assert max_rel(got, ow.eval(q, abi.Q_DEMAG_FIELD)) < FIELD_TOL
+
+
 def test_three_magnets_share_launches(mpx):
     """Every destination has two sources; two of the three pairs of sizes share a launch shape, one takes the
     direct sum (below 2^22 interactions)."""
