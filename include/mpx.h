@@ -273,6 +273,9 @@ mpx_status mpx_magnet_add_state(mpx_engine* e, int group, const mpx_magnet_desc*
  * solves against a memory budget.  No counterpart in the reference, which
  * allocates from its pool as fields are needed (core/gpumemorypool.cu). */
 mpx_status mpx_magnet_bytes(const mpx_magnet_desc* d, int64_t* resident, int64_t* transient);
+/* The same for an engine with DFT mode `mode` (mpx_engine_set_dft), whose transform
+ * lengths and paths differ; mpx_magnet_bytes is that of MPX_DFT_FP32, the default. */
+mpx_status mpx_magnet_bytes_dft(const mpx_magnet_desc* d, int mode, int64_t* resident, int64_t* transient);
 /* Re-reads all parameters; rebuilds the demag kernel only when the cell size,
  * geometry-independent grid data, mastergrid or PBC changed. */
 mpx_status mpx_magnet_update(mpx_engine* e, int magnet, const mpx_magnet_desc* d);

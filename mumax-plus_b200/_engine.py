@@ -55,6 +55,7 @@ class Engine:
         check(L.mpx_engine_create(int(device), C.byref(h)))
         self._h = h
         self.device = device
+        self.dft = _abi.MPX_DFT_FP32
 
     def __del__(self):
         h = getattr(self, "_h", None)
@@ -79,6 +80,7 @@ class Engine:
     def set_dft(self, mode):
         """_abi.MPX_DFT_FP32 or _abi.MPX_DFT_TF32X3 (before the first magnet)."""
         check(lib().mpx_engine_set_dft(self._h, int(mode)))
+        self.dft = int(mode)
 
     @staticmethod
     def tc_timeouts():
@@ -294,8 +296,9 @@ class Engine:
         return [done[i] for i in range(nd.value)], nr.value
 
 
-def magnet_bytes(desc):
-    """(resident, transient) device bytes that adding `desc` takes (no GPU needed)."""
+def magnet_bytes(desc, dft=_abi.MPX_DFT_FP32):
+    """(resident, transient) device bytes that adding `desc` to an engine of DFT mode
+    `dft` takes (no GPU needed)."""
     res, tr = C.c_int64(), C.c_int64()
-    check(_abi.load().mpx_magnet_bytes(C.byref(desc), C.byref(res), C.byref(tr)))
+    check(_abi.load().mpx_magnet_bytes_dft(C.byref(desc), int(dft), C.byref(res), C.byref(tr)))
     return res.value, tr.value

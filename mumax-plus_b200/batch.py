@@ -62,9 +62,9 @@ def solve_desc(w, keep):
     return d
 
 
-def solve_bytes(w):
-    """(resident, transient) device bytes of one solve."""
-    return magnet_bytes(solve_desc(w, []))
+def solve_bytes(w, dft=_abi.MPX_DFT_FP32):
+    """(resident, transient) device bytes of one solve on an engine of DFT mode `dft`."""
+    return magnet_bytes(solve_desc(w, []), dft)
 
 
 class Batch:
@@ -92,7 +92,7 @@ class Batch:
             eng.set_solver_params(g, p)
             keep = []
             d = solve_desc(w, keep)
-            s.resident, s.transient = magnet_bytes(d)
+            s.resident, s.transient = magnet_bytes(d, eng.dft)
             # the magnet with its initial state: the group's time step is then
             # the sensible one for that state
             s.magnet = eng.magnet_add_state(g, d, w["m0"]() if m0 is None else m0)
@@ -327,7 +327,7 @@ class Server:
             # admission against the memory budget, in arrival order
             while queue:
                 k, w = queue[0]
-                res, tr = solve_bytes(w)
+                res, tr = solve_bytes(w, b.engine.dft)
                 if b.resident + res + tr > self.budget and b.solves:
                     break
                 if self.max_active is not None and len(b.solves) >= self.max_active:

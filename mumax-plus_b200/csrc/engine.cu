@@ -613,6 +613,11 @@ void split_shapes(int ncols, int Py, int Pz, bool warp, int* ncy, int* nkz) {
   *nkz = std::max(1, std::min(Py, warp ? zcw_kys(Pz) : (YZ_VPT * YZ_THREADS) / (3 * Pz)));
 }
 
+// Tensor-core y transforms (k_ydft_tc): the y lengths that have them, and the columns
+// per 128-sequence tile (4 at Py = 1024, 2 at 2048).
+bool tc_lengths(int mode, const int P[3]) { return mode == MPX_DFT_TF32X3 && (P[1] == 1024 || P[1] == 2048); }
+int tc_columns(int Py) { return 4096 / Py; }
+
 int ycols_smem(const Magnet* m) { return (m->ncy * plen(m->P[1]) + m->P[1]) * (int)sizeof(float2); }
 int zmul_smem(const Magnet* m) { return (3 * m->nkz * plen(m->P[2]) + m->P[2]) * (int)sizeof(float2); }
 
@@ -1784,7 +1789,7 @@ mpx_status setup_magnet(mpx_engine* e, Magnet* m, const mpx_magnet_desc* d, bool
                                        "(grid side above 1024 along x or 2048 along y)");
     // thick magnets (nz > 8) and long y transforms of many columns take the split y/z path;
     // so do y lengths 1024 and 2048 when the engine runs the tensor-core y transforms
-    m->tc = e->dft_mode == MPX_DFT_TF32X3 && (m->P[1] == 1024 || m->P[1] == 2048) && !m->probe;
+    m->tc = tc_lengths(e->dft_mode, m->P) && !m->probe;
     m->split = m->tc || m->P[2] > 16 || yz_smem(m) > SMEM_DYN_MAX;
     if (m->split) {
       if (m->P[2] > MAX_FFT) return fail(MPX_ERR_UNSUPPORTED, "demag: padded FFT length above 4096 along z");
@@ -1852,7 +1857,7 @@ mpx_status setup_magnet(mpx_engine* e, Magnet* m, const mpx_magnet_desc* d, bool
   if (m->demag && m->split) {
     const int ncols = D.Fh * 3 * D.n[2];
     if (m->tc) {
-      const int cpt = 4096 / m->P[1];  // columns per 128-sequence tile: 4 at Py = 1024, 2 at 2048
+      const int cpt = tc_columns(m->P[1]);
       for (int c0 = 0; c0 < ncols; c0 += cpt) m->tcw.push_back(Work{m->slot, c0, std::min(cpt, ncols - c0), 0});
     } else {
       for (int c0 = 0; c0 < ncols; c0 += m->ncy) m->ycw.push_back(Work{m->slot, c0, std::min(m->ncy, ncols - c0), 0});
@@ -2705,6 +2710,11 @@ mpx_status mpx_magnet_update(mpx_engine* e, int magnet, const mpx_magnet_desc* d
 }
 
 mpx_status mpx_magnet_bytes(const mpx_magnet_desc* d, int64_t* resident, int64_t* transient) {
+  return mpx_magnet_bytes_dft(d, MPX_DFT_FP32, resident, transient);
+}
+
+mpx_status mpx_magnet_bytes_dft(const mpx_magnet_desc* d, int mode, int64_t* resident, int64_t* transient) {
+  if (mode != MPX_DFT_FP32 && mode != MPX_DFT_TF32X3) return fail(MPX_ERR_INVALID, "unknown DFT mode");
   if (!resident || !transient) return fail(MPX_ERR_INVALID, "null argument");
   MPX_TRY(validate_desc(d));
   const int64_t N = (int64_t)d->size[0] * d->size[1] * d->size[2];
@@ -2729,7 +2739,7 @@ mpx_status mpx_magnet_bytes(const mpx_magnet_desc* d, int64_t* resident, int64_t
   if (L > 0) res += 4 * L * ((d->inter_exchange_lut ? 1 : 0) + (d->scale_exchange_lut ? 1 : 0));
   const bool demag = d->enable_demag && !scalar_zero(d->msat);
   int P[3];
-  plan_lengths(d->size, false, P);
+  plan_lengths(d->size, mode == MPX_DFT_TF32X3, P);
   const int ty = choose_ty(d->size[1], demag ? P[0] : d->size[0]);
   res += (int64_t)sizeof(Work) * d->size[2] * ((d->size[1] + ty - 1) / ty);
   int64_t tr = 12 * N;  // initial random state (engine scratch)
@@ -2741,10 +2751,12 @@ mpx_status mpx_magnet_bytes(const mpx_magnet_desc* d, int64_t* resident, int64_t
     const int nkx = choose_nkx(d->size[2], P[1], P[2], (int)Fh);
     res += (int64_t)sizeof(Work) * ((Fh + nkx - 1) / nkx);       // y/z work items
     const int yzs = yz_smem_of(d->size[2], nkx, P[1], P[2]);
-    if (P[2] > 16 || yzs > SMEM_DYN_MAX) {  // split y/z path: T and its work items
+    const bool tc = tc_lengths(mode, P);
+    if (tc || P[2] > 16 || yzs > SMEM_DYN_MAX) {  // split y/z path: T and its work items
       res += 8 * Fh * 3 * d->size[2] * P[1];
       int ncy, nkz;
-      split_shapes((int)(Fh * 3 * d->size[2]), P[1], P[2], split_warp(P[1], P[2]), &ncy, &nkz);
+      split_shapes((int)(Fh * 3 * d->size[2]), P[1], P[2], !tc && split_warp(P[1], P[2]), &ncy, &nkz);
+      if (tc) ncy = tc_columns(P[1]);
       res += (int64_t)sizeof(Work) * ((Fh * 3 * d->size[2] + ncy - 1) / ncy + Fh * ((P[1] + nkz - 1) / nkz));
     }
     KernelGeom g;

@@ -298,3 +298,18 @@ def test_admission_does_not_grow_with_periodic_images(built_lib, size, pbc):
         res, tr = _bytes(size, tuple(r * p for p in pbc))
         assert res == resident
         assert tr <= 12 * cells + 48 * cells + 32 * padded, (r, tr)
+
+
+def test_admission_follows_the_dft_mode(built_lib):
+    """300 x 180 x 3 cells are transformed in 768 x 384 points, 1024 x 512 with the TF32x3 transforms: their spectrum
+    (3 components) and kernel (6) differ by that much."""
+    import mumaxplus_b200 as mpx
+
+    modes = [_bytes((300, 180, 3), (0, 0, 0), dft=d) for d in (mpx._abi.MPX_DFT_FP32, mpx._abi.MPX_DFT_TF32X3)]
+    spectra = [8 * (x // 2 + 1) * 3 * 180 * 3 + 4 * 6 * (x // 2 + 1) * (y // 2 + 1) * 5 for x, y in ((768, 384), (1024, 512))]
+    assert abs((modes[1][0] - modes[0][0]) - (spectra[1] - spectra[0])) < 64 * 1024  # the work tables
+    assert modes[1][1] > modes[0][1]
+    small = [_bytes((100, 80, 2), (0, 0, 0), dft=d) for d in (mpx._abi.MPX_DFT_FP32, mpx._abi.MPX_DFT_TF32X3)]
+    assert small[0] == small[1]
+    with pytest.raises(ValueError):
+        _bytes((100, 80, 2), (0, 0, 0), dft=7)

@@ -117,6 +117,20 @@ def test_magnet_bytes_matches_engine_accounting(mpx):
     assert b.engine.memory() == before
 
 
+# 1024 x 512 with the TF32x3 transforms (768 x 384 in FP32), and y lengths of the tensor-core path
+@pytest.mark.parametrize("size", [(300, 180, 3), (40, 300, 14), (20, 600, 2)])
+def test_magnet_bytes_with_tensor_core_transforms(mpx, size):
+    from mumaxplus_b200 import batch as B
+
+    b = B.Batch()
+    b.engine.set_dft(mpx._abi.MPX_DFT_TF32X3)
+    before = b.engine.memory()
+    s = b.add(_solve(0, size, 3e-9, 8e5, 1.3e-11, 0.1, (0.0, 0.0, 0.1)))
+    grown = b.engine.memory() - before
+    assert grown <= s.resident <= grown + 64 * 1024
+    b.finish(s, fetch=False)
+
+
 def test_batch_solve_follows_oracle(mpx):
     """One solve of a batch against the FP64 oracle's Dormand-Prince run."""
     from mumaxplus_b200 import batch as B
