@@ -278,6 +278,27 @@ struct SplitLaunch {
 
 constexpr int N_SIDE = 3;  // side streams of the y/z classes of a batch
 
+// In an engine of several groups a kernel form (or y/z class) that the launched
+// solves no longer need stays in the attempt graphs for KEEP_ATTEMPTS attempts:
+// solves come and go, and another set of kernels instantiates the graphs anew, 1.3 ms
+// each time.  For 13 solves of one layer (334 us per attempt) a visitor's form costs 3 us
+// per attempt (mask, 2048-point rows), an empty class 30 us, both with the rows of 384
+// and 768 points 70 us; 64 attempts of an empty class cost about what the instantiation
+// does, so that neither a form that comes and goes nor one that never returns costs
+// much more than twice the better choice.
+constexpr int64_t KEEP_ATTEMPTS = 64;
+struct Kept {
+  bool on = false;
+  int64_t since = -1;  // attempt count when it was last needed, -1: it is needed
+  bool update(bool needed, bool keep, int64_t attempts) {
+    if (needed) since = -1;
+    else if (since < 0) since = attempts;
+    on = needed || (on && keep && !expired(attempts));
+    return on;
+  }
+  bool expired(int64_t attempts) const { return on && since >= 0 && attempts - since >= KEEP_ATTEMPTS; }
+};
+
 struct mpx_engine {
   int device = 0;
   cudaStream_t own = nullptr, stream = nullptr;
@@ -322,6 +343,8 @@ struct mpx_engine {
   int smem_x = 0, nt_x = 256;
   XForm x_form;                   // of the launched magnets
   bool yz_one[YZ_CLASSES] = {};   // all blocks of the class have no more columns than warps
+  Kept keep_pair, keep_mask, keep_three, keep_class[YZ_CLASSES];  // forms and classes in the attempt graphs
+  int64_t attempts = 0;                                           // replayed so far
   bool any_nodemag = false;
   int64_t bytes = 0;
   int64_t launches = 0;
@@ -867,7 +890,7 @@ mpx_status rebuild_tables(mpx_engine* e) {
   // comes and goes with it would instantiate the attempt graphs anew each time
   // (batches lost 4 %)
   const int ngroups = (int)std::count_if(e->groups.begin(), e->groups.end(), [](const auto& g) { return g != nullptr; });
-  if (ngroups <= 1) e->x_form = XForm();  // (a form of several groups' launches stays, as the classes below)
+  e->x_form = XForm();
   e->x_form.one = ngroups == 1;
   for (int c = 0; c < YZ_CLASSES; ++c) e->yz_one[c] = e->yz_one[c] && ngroups == 1;
   bool any512 = false;
@@ -880,6 +903,10 @@ mpx_status rebuild_tables(mpx_engine* e) {
     any512 = any512 || pr.first->P[0] == 512 || pr.first->P[0] == 384;
   }
   e->x_form.one = e->x_form.one && any512;
+  const bool keep = ngroups > 1;
+  e->x_form.pair = e->keep_pair.update(e->x_form.pair, keep, e->attempts);
+  e->x_form.mask = e->keep_mask.update(e->x_form.mask, keep, e->attempts);
+  e->x_form.three = e->keep_three.update(e->x_form.three, keep, e->attempts);
   // each table: holes for the magnets that left (or whose lists changed), the
   // newcomers appended, compaction when the holes outnumber the live entries,
   // and an upload of the changed entries only
@@ -907,11 +934,9 @@ mpx_status rebuild_tables(mpx_engine* e) {
         if (!pr.second->empty() && !T.place.count(pr.first->uid)) T.add(pr.first->uid, pr.first->ver, *pr.second);
     }
     while (!T.items.empty() && T.items.back().mag < 0) T.items.pop_back();  // trailing holes
-    // In an engine of several groups a y/z class stays in the attempt graphs once
-    // it was used (with one hole when empty): solves come and go, and another
-    // set of kernels would instantiate the graphs anew, 1.3 ms each time against
-    // about 2 us per stage for the empty class beside the others.
-    if (t >= mpx_engine::TT_YZ0 && ngroups > 1 && T.items.empty() && T.cap > 0) {
+    // (an empty y/z class that is kept has one hole)
+    if (t >= mpx_engine::TT_YZ0 &&
+        e->keep_class[t - mpx_engine::TT_YZ0].update(!T.items.empty(), keep, e->attempts) && T.items.empty()) {
       T.items.push_back(Work{-1, 0, 0, 0});
       T.dirty(0, 1);
     }
@@ -2053,6 +2078,8 @@ mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
 
 mpx_status prepare_run(mpx_engine* e, int method) {
   if (e->pairs_dirty) MPX_TRY(rebuild_pairs(e));
+  for (const Kept* k : {&e->keep_pair, &e->keep_mask, &e->keep_three}) e->tables_dirty |= k->expired(e->attempts);
+  for (const Kept& k : e->keep_class) e->tables_dirty |= k.expired(e->attempts);
   if (e->tables_dirty) MPX_TRY(rebuild_tables(e));
   MPX_TRY(ensure_side_streams(e));
   MPX_TRY(upload_tableau(e, method));
@@ -2132,6 +2159,7 @@ mpx_status run_attempts(mpx_engine* e, int method, int n) {
     e->launches += full ? per_full : per_nok0;
     e->need_stage0 = false;
   }
+  e->attempts += n;
   return MPX_OK;
 }
 

@@ -6,6 +6,8 @@ Tolerance: final m of a solve in a mix vs alone <= 1e-6 absolute (the
 batched form's parity bound is 1e-5; the arithmetic is the same per magnet,
 so the results are expected to agree bit for bit).
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -232,3 +234,62 @@ def test_launch_tables_keep_places_through_churn(mpx):
             live.pop(s.group)
     for k, want in alone.items():
         np.testing.assert_array_equal(got[k], want)
+
+
+@pytest.mark.parametrize("guest", [dict(size=(40, 32, 2)), dict(size=(40, 32, 1), mask=True), dict(size=(600, 16, 1)),
+                                   dict(size=(190, 400, 2))])
+def test_forms_leave_with_the_solves_that_needed_them(mpx, monkeypatch, guest):
+    """The kernels that a visiting solve needs (another y/z class, the masked stage epilogue, 2048- and 384-point x
+    rows) stay in the attempt of the others for a while after it has finished, then leave, and the others end as
+    without it."""
+    from mumaxplus_b200 import batch as B
+
+    hosts = [_solve(30 + k, (40, 32, 1), 3e-9, 8e5, 1.3e-11, 0.1, (0.02, 0.0, 0.05)) for k in range(2)]
+
+    def begin():
+        b = B.Batch()
+        ss = [b.add(w, key=i) for i, w in enumerate(hosts)]
+        for s in ss:
+            b.start(s, 1e-6)
+        b.advance(4)
+        b.poll()
+        return b, ss
+
+    def cost(b, n):  # launches and attempt graphs (new or updated) of n attempts
+        l0, g0 = b.engine.launch_count(), sum(b.engine.graph_stats())
+        b.advance(n)
+        b.poll()
+        return b.engine.launch_count() - l0, sum(b.engine.graph_stats()) - g0
+
+    ref, rs = begin()
+    alone = cost(ref, 10)[0]
+    b, ss = begin()
+    w = _solve(40, guest["size"], 3e-9, 8e5, 1.3e-11, 0.3, (0.0, 0.02, 0.05))
+    if guest.get("mask"):
+        disc = np.ascontiguousarray(np.hypot(*(np.mgrid[0:32, 0:40] - np.array([15.5, 19.5])[:, None, None])) < 15,
+                                    dtype=np.uint8)
+
+        def masked(w, keep, plain=B.solve_desc):
+            d = plain(w, keep)
+            d.geometry = disc.ctypes.data_as(C.POINTER(C.c_ubyte))
+            return d
+
+        monkeypatch.setattr(B, "solve_desc", masked)
+    v = b.add(w, key=9)
+    b.start(v, 1e-15)
+    n = 0
+    while v.group in b.solves:
+        b.advance(2)
+        n += 2
+        for s in b.poll()[0]:
+            b.finish(s, fetch=False)
+    launches, graphs = cost(b, 10)  # the solve has left, its kernels stay
+    assert launches >= alone
+    assert cost(b, 20)[1] == 0  # and the attempt does not change
+    launches, graphs = cost(b, 200)
+    launches2, graphs2 = cost(b, 10)
+    assert graphs + graphs2 > 0 and launches2 == alone
+    ref.advance(n + 240 - 10)
+    ref.poll()
+    for r, s in zip(rs, ss):
+        np.testing.assert_array_equal(b.engine.get_m(s.magnet, s.shape), ref.engine.get_m(r.magnet, r.shape))
