@@ -40,14 +40,20 @@ def _obj(unit):
     return os.path.join(OBJ, unit + ".o")
 
 
+def _src(unit):
+    return os.path.join(CSRC, unit.removeprefix("checked_") + ".cu")
+
+
 def _deps(unit):
-    """Files the unit was compiled from (the compiler's dependency file), or None."""
+    """Files of this tree the unit was compiled from (the compiler's dependency file), or None
+    where that file is missing or names another tree's (a copied _build folder)."""
     try:
         with open(os.path.join(OBJ, unit + ".d")) as f:
             words = f.read().replace("\\\n", " ").split()
     except OSError:
         return None
-    return [w for w in words[1:] if w.startswith(ROOT)]
+    deps = [w for w in words[1:] if w.startswith(ROOT + os.sep)]
+    return deps if _src(unit) in deps else None
 
 
 def _stale(unit):
@@ -78,9 +84,8 @@ def _run(cmd, verbose):
 def _command(out, extra=(), unit="engine"):
     """The nvcc command of `unit` into `out`; the checked library's adds the check."""
     checked = out == OUT_CHECKED or unit.startswith("checked_")
-    src = os.path.join(CSRC, unit.removeprefix("checked_") + ".cu")
     return ([nvcc_path()] + NVCC_FLAGS + (["-DMPX_BOUNDS_CHECK"] if checked else []) + list(extra)
-            + ["-I", os.path.join(ROOT, "include"), src, "-o", out])
+            + ["-I", os.path.join(ROOT, "include"), _src(unit), "-o", out])
 
 
 def _compile(unit, extra, verbose):

@@ -313,3 +313,32 @@ def test_admission_follows_the_dft_mode(built_lib):
     assert small[0] == small[1]
     with pytest.raises(ValueError):
         _bytes((100, 80, 2), (0, 0, 0), dft=7)
+
+
+def test_objects_of_another_tree_are_stale(tmp_path, monkeypatch):
+    """A _build folder copied with the tree to another path names the first tree's files: its objects are compiled
+    again there, and a changed file is seen again."""
+    import importlib.util
+
+    spec = importlib.util.spec_from_file_location("_mpx_build", os.path.join(ROOT, "mumax-plus_b200", "build.py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    src, obj = tmp_path / "csrc", tmp_path / "_build"
+    src.mkdir()
+    obj.mkdir()
+    monkeypatch.setattr(mod, "ROOT", str(tmp_path))
+    monkeypatch.setattr(mod, "CSRC", str(src))
+    monkeypatch.setattr(mod, "OBJ", str(obj))
+    (src / "pairs.cu").write_text("")
+    for unit in ("pairs", "checked_pairs"):
+        (obj / f"{unit}.o").write_text("")
+        later = os.path.getmtime(mod.__file__) + 1000
+        os.utime(src / "pairs.cu", (later, later))
+        os.utime(obj / f"{unit}.o", (later + 10, later + 10))
+        (obj / f"{unit}.d").write_text(f"{obj}/{unit}.o: {src}/pairs.cu /usr/include/stdio.h\n")
+        assert not mod._stale(unit)
+        (obj / f"{unit}.d").write_text(f"/other/_build/{unit}.o: /other/csrc/pairs.cu /usr/include/stdio.h\n")
+        assert mod._stale(unit)
+        (obj / f"{unit}.d").write_text(f"{obj}/{unit}.o: {src}/pairs.cu\n")
+        os.utime(src / "pairs.cu", (later + 20, later + 20))
+        assert mod._stale(unit)
