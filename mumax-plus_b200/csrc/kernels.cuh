@@ -247,7 +247,10 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xfwd(const MagnetDev* __re
   const int nx = M.n[0], ny = M.n[1], nz = M.n[2], N = M.N;
   const int logL = M.logP[0], L = THREE ? M.P[0] : 1 << logL, cs = xrow_stride(L, ty);
   // rows of the PAIR and THREE forms (the host never launches them elsewhere)
-  if ((!PAIR && logL == 11) || (!THREE && logL >= LOG_THREE)) return;
+  if ((!PAIR && logL == 11) || (!THREE && logL >= LOG_THREE)) {
+    pdl_wait();
+    return;
+  }
   const bool three = THREE && logL >= LOG_THREE;
   const int nzrows = (ty + 1) >> 1;
   const float* src = msrc_override ? msrc_override : stage_m(M, G, stage);
@@ -446,17 +449,14 @@ __device__ __forceinline__ void apply3(float2* v0, float2* v1, float2* v2, float
 
 // z stage of one ky, half = 0 / 1 computing the even / odd kz of the PZ-point
 // transform of nz <= PZ/2 inputs as a PZ/2-point transform (of x, or of
-// x[n] W_PZ^n); the partner lane (lane ^ PARTNER) holds the other half and the
-// two inverse halves are summed with one shuffle.  Q5: columns in the qidx
-// layout of the warp transforms (else pidx).  PARTNER 16: the two halves of a
-// warp take the even / odd kz of the same 16 ky, so that every store of a
-// half-warp goes to one column at 16 consecutive ky (no bank conflicts).
-template <int PZ, bool Q5 = false, int PARTNER = 1>
+// x[n] W_PZ^n); the partner lane (lane ^ 1) holds the other half and the
+// two inverse halves are summed with one shuffle.
+template <int PZ>
 __device__ __forceinline__ void zstage_pair(float2* D, int cs, const MagnetDev& M, int kx, int ky, int half, int nz,
                                             int Py) {
   constexpr int H = PZ / 2;
   float2 v[3][H];
-  const int pky = Q5 ? qidx(ky) : pidx(ky);
+  const int pky = pidx(ky);
   // kernel spectrum of this lane's kz values, issued before the transforms
   const int hy = Py / 2 + 1;
   const int kyp = min(ky, Py - ky);
@@ -526,8 +526,8 @@ __device__ __forceinline__ void zstage_pair(float2* D, int cs, const MagnetDev& 
       const float2 od = (2 * k + 1 < H) ? v[c][2 * k + 1] : make_float2(0.f, 0.f);
       const float2 send = half ? ev : od;
       const float2 mine = half ? od : ev;
-      const float ox = __shfl_xor_sync(mask, send.x, PARTNER);
-      const float oy = __shfl_xor_sync(mask, send.y, PARTNER);
+      const float ox = __shfl_xor_sync(mask, send.x, 1);
+      const float oy = __shfl_xor_sync(mask, send.y, 1);
       const int n = 2 * k + half;
       if (n < H && n < nz) D[(c * nz + n) * cs + pky] = make_float2(mine.x + ox, mine.y + oy);
     }
@@ -548,7 +548,7 @@ __device__ __forceinline__ float2 rot16_m(float2 v, int m) {
   }
 }
 
-// z stage of one ky in one lane (PZ = 2 .. 16): both halves of zstage_pair<PZ>
+// z stage of one ky in one lane (PZ = 4 .. 16): both halves of zstage_pair<PZ>
 // (the even kz = 2q from the PZ/2-point transform of x, the odd kz = 2q + 1
 // from that of x[n] W_PZ^n), the 3x3 multiply per kz, and the output as the
 // sum of the two PZ/2-point inverses: the same operations on the same values,
@@ -825,17 +825,10 @@ __device__ __forceinline__ void yzw_body(const MagnetDev& M, int kx0, int nkx, f
       const int j = t / Py;
       zstage_single<true>(D + j * 3 * cs, cs, M, kx0 + j, t - j * Py, Py);
     }
-  } else if constexpr (PZ >= 4) {  // one lane per (kx, ky)
+  } else {  // one lane per (kx, ky)
     for (int t = threadIdx.x; t < nkx * Py; t += blockDim.x) {
       const int j = t / Py;
       zstage_full<PZ, true>(D + j * 3 * nz * cs, cs, M, kx0 + j, t - j * Py, nz, Py);
-    }
-  } else {
-    // lanes l and l + 16 of a warp share one (kx, ky): the even and odd kz
-    // halves (the item count is a multiple of 32 and so is the block)
-    for (int t = threadIdx.x; t < 2 * nkx * Py; t += blockDim.x) {
-      const int u = ((t >> 5) << 4) | (t & 15), j = u / Py;
-      zstage_pair<PZ, true, 16>(D + j * 3 * nz * cs, cs, M, kx0 + j, u - j * Py, (t >> 4) & 1, nz, Py);
     }
   }
   __syncthreads();
@@ -983,16 +976,10 @@ __global__ void __launch_bounds__(YZP_THREADS, 1)
       const int j = t >> LOGPY;
       zstage_single<true>(D + j * 3 * cs, cs, M, kx0 + j, t & (Py - 1), Py);
     }
-  } else if constexpr (PZ >= 4) {  // one lane per (kx, ky)
+  } else {  // one lane per (kx, ky)
     for (int t = threadIdx.x; t < nkx << LOGPY; t += blockDim.x) {
       const int j = t >> LOGPY;
       zstage_full<PZ, true>(D + j * 3 * nz * cs, cs, M, kx0 + j, t & (Py - 1), nz, Py);
-    }
-  } else {
-    // lanes l and l + 16 of a warp share one (kx, ky): the even and odd kz halves
-    for (int t = threadIdx.x; t < (2 * nkx) << LOGPY; t += blockDim.x) {
-      const int u = ((t >> 5) << 4) | (t & 15), j = u >> LOGPY;
-      zstage_pair<PZ, true, 16>(D + j * 3 * nz * cs, cs, M, kx0 + j, u & (Py - 1), (t >> 4) & 1, nz, Py);
     }
   }
   __syncthreads();
@@ -1120,7 +1107,6 @@ __device__ __forceinline__ void epilogue_cell(const MagnetDev& M, const GroupDev
     case 3: r = lo.dmi; break;
     case 4: r = lo.anis; break;
     case 5: r = lo.ext; break;
-    case 6: r = bdemag; break;
     case 7:  // total torque: LLG + spin transfer (physics/torque.cu:78-90)
     case 8:
       if (M.frozen.at(i) == 0.0f) {
@@ -1650,7 +1636,10 @@ __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __re
   const int nx = M.n[0], ny = M.n[1], nz = M.n[2];
   const int logL = M.logP[0], L = THREE ? M.P[0] : 1 << logL, cs = xrow_stride(L, ty);
   // rows of the PAIR and THREE forms (the host never launches them elsewhere)
-  if ((!PAIR && logL == 11) || (!THREE && logL >= LOG_THREE)) return;
+  if ((!PAIR && logL == 11) || (!THREE && logL >= LOG_THREE)) {
+    pdl_wait();
+    return;
+  }
   const bool three = THREE && logL >= LOG_THREE;
   const int nzrows = (ty + 1) >> 1;
   const int Fh = M.Fh;

@@ -6,12 +6,10 @@ namespace mpx {
 YzFn yz_long_fn(int cls) {
   switch (cls) {
     case 15: return k_yzw32<1>;
-    case 16: return k_yzw32<2>;
     case 17: return k_yzw32<4>;
     case 18: return k_yzw32<8>;
     case 19: return k_yzw32<16>;
     case 20: return k_yzw64<1>;
-    case 21: return k_yzw64<2>;
     case 22: return k_yzw64<4>;
     default: return k_yzw64<8>;
   }

@@ -6,14 +6,12 @@ namespace mpx {
 YzFn yz_three_fn(int cls, bool one) {
   if (one && cls == 24) return k_yzw3<1, true>;
   if (one && cls == 26) return k_yzw3<4, true>;
-  switch (cls) {  // z length 2 does not occur (2 n - 1 is odd)
+  switch (cls) {
     case 24: return k_yzw3<1>;
-    case 25:
     case 26: return k_yzw3<4>;
     case 27: return k_yzw3<8>;
     case 28: return k_yzw3<16>;
     case 29: return k_yzw24<1>;
-    case 30:
     case 31: return k_yzw24<4>;
     case 32: return k_yzw24<8>;
     default: return k_yzw24<16>;

@@ -7,7 +7,6 @@ YzFn yz_warp_fn(int cls, bool one) {
   if (one) return cls == 10 ? k_yzw<1, true> : k_yzw<4, true>;
   switch (cls) {
     case 10: return k_yzw<1>;
-    case 11: return k_yzw<2>;
     case 12: return k_yzw<4>;
     case 13: return k_yzw<8>;
     default: return k_yzw<16>;
