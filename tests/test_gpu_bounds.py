@@ -1,5 +1,5 @@
-"""Checked build: the parity, random-magnet, stray-field and tensor-core suites
-run again against libmpx_checked.so (the same sources compiled with
+"""Checked build: the parity, random-magnet, stray-field, tensor-core and launch-path
+suites run again against libmpx_checked.so (the same sources compiled with
 -DMPX_BOUNDS_CHECK), where every per-cell access of a field buffer -- stencil
 neighbours under every boundary condition, stage states and derivatives,
 stray-field buffers -- and every spectrum access of the x passes and of the
@@ -26,7 +26,8 @@ CHECKED = os.path.join(ROOT, "mumax-plus_b200", "libmpx_checked.so")
 def test_checked_build_suites_stay_in_bounds():
     assert os.path.exists(CHECKED), "libmpx_checked.so is missing: run __graft_entry__.build()"
     env = dict(os.environ, MPX_LIBRARY=CHECKED, MPX_BOUNDS_CHECK_RUN="1")
-    suites = ["tests/test_gpu_parity.py", "tests/test_gpu_fuzz.py", "tests/test_gpu_stray.py", "tests/test_gpu_tc.py"]
+    suites = ["tests/test_gpu_parity.py", "tests/test_gpu_fuzz.py", "tests/test_gpu_stray.py", "tests/test_gpu_tc.py",
+              "tests/test_gpu_paths.py"]
     res = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider"] + suites,
                          cwd=ROOT, env=env, capture_output=True, text=True, timeout=900)
     assert res.returncode == 0, res.stdout[-4000:] + res.stderr[-2000:]
