@@ -567,10 +567,13 @@ bool split_warp(int Py, int Pz);
 // of powers of two), and 96 .. 768 (y), where they are shorter; all powers of two with
 // the tensor-core y transforms and on the block-wide split path.  300 x 180 x 3 cells
 // (768 x 384 for 1024 x 512): 10.56 -> 9.78 ms per 38 attempts; 80 x 80 x 40 (y 192 for
-// 256): 15.3 -> 12.6; 437 x 291 x 2 energy density 63.3 -> 59.9 us.  Smaller magnets are
-// bound by latency, and in a batch the further launch classes cost more than they
-// save: 24 solves of up to 131,000 cells 18.0 -> 18.2 ms, their first pass 18.6 ->
-// 20.4 ms (larger graphs to instantiate).
+// 256): 15.3 -> 12.6; 437 x 291 x 2 energy density 63.3 -> 59.9 us.  The line is drawn by
+// the batches, whose further launch classes cost more than the lengths save: 24 solves of
+// up to 131,000 cells 17.7 -> 17.95 ms.  Alone, most smaller magnets would gain as well
+// (us per Dormand-Prince attempt: 170 x 60 x 1 125 -> 113, 170 x 170 x 2 151 -> 142,
+// 300 x 300 x 1 200 -> 189, 90 x 90 x 16 309 -> 252; 100 x 300 x 1 and 250 x 250 x 1
+// nothing, 370 x 370 x 1 212 -> 215), but a magnet's lengths must not depend on what
+// else its engine holds.
 constexpr int64_t THREE_MIN_CELLS = 150000;
 void plan_lengths(const int n[3], bool pow2, int P[3]) {
   for (int a = 0; a < 3; ++a) P[a] = padded(n[a]);
@@ -728,10 +731,6 @@ mpx_status launch_yz(mpx_engine* e, int cls, const Work* work, int n, int smem, 
   e->launches++;
   return MPX_OK;
 }
-// The x-pass kernels of a launch: the PAIR forms (2048-point warp-pair rows
-// compiled in) when one of its magnets has 2048-point x rows, else the forms
-// without them (the shorter lengths keep their registers and code).
-
 int x_threads(const Magnet* m) {
   int rows = m->ty + (m->ty + 1) / 2;
   int t = (rows * m->P[0] + 7) / 8;  // 8 values per thread in the x FFTs
@@ -1475,7 +1474,7 @@ int kernel_axis_smem(int P) { return (2 * kernel_axis_lines(P) + 1) * P * (int)s
 // what a padded complex grid per component pair would take, so that a periodic magnet
 // needs no more memory than its size asks for however many images it has (256 x 256 x 1
 // cells with 30 images: one lattice would take 1 GB); its images come in parts then
-// (admitting 256 x 256 x 1 cells with 10 images: 15.7 ms, 6.8 with one lattice of 121 MB).
+// (admitting 256 x 256 x 1 cells with 10 images: 15.7 ms, 6.8 with one lattice of 127 MB).
 // LATTICE_ENGINE is the engine's own, like its reduction buffers, and not counted: it
 // keeps the parts of a small magnet few (32 x 32 x 1 cells with 30 images).
 constexpr int64_t LATTICE_ENGINE = 4LL << 20;
@@ -2015,9 +2014,9 @@ mpx_status launch_attempt(mpx_engine* e, const TableauDev& T, int first_stage) {
     if (e->n_t_demag > 0) {
       // The y/z classes of a batch run beside each other: each is a few waves of
       // blocks, and one after the other every class leaves the SMs idle in its
-      // last wave and in the gap to the next.  The first class follows the x pass
-      // by programmatic launch; the others fork from it into side streams.  The
-      // 24-solve batch (z lengths 1 and 4): 18.38 -> 18.0 ms.
+      // last wave and in the gap to the next.  The last class follows the x pass
+      // by programmatic launch; the earlier ones fork from it into side streams.  The
+      // 24-solve batch (z lengths 1 and 4): 18.4 -> 17.7 ms.
       int last = -1, forked = 0;
       for (int c = 0; c < YZ_CLASSES; ++c)
         if (e->n_kx_demag[c] > 0) last = c;

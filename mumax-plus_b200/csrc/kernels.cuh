@@ -1618,7 +1618,7 @@ __device__ __forceinline__ void stage_quad_lean(const MagnetDev& M, const GroupD
 // among the launch's; in the other forms it would cost the common path 2 - 7 %
 // by its registers).  A 200 x 200 disc took 21 us of a 45 us stage in the general
 // path (epilogue_cell), whose cells fetch their neighbours one after the other
-// and divide per neighbour: 18 Fehlberg attempts 4.91 -> 3.18 ms.
+// and divide per neighbour: 18 Fehlberg attempts 4.95 -> 3.04 ms.
 template <bool PAIR = false, bool MASK = false, bool ONE = false, bool THREE = false>
 __global__ void __launch_bounds__(X_THREADS_MAX, 2) k_xinv(const MagnetDev* __restrict__ mags, GroupDev* __restrict__ groups,
                                               const Work* __restrict__ work, EpiArgs ea,
